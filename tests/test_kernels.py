@@ -155,6 +155,27 @@ def test_gemm_float32_is_not_tf32():
     assert (want - 64.0).abs().min().item() > 1e-2   # TF32 inputs would give exactly 64
 
 
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("m", [1, 2, 3, 8])
+@pytest.mark.parametrize("n, k", [(9216, 1024), (1024, 4608), (70, 36), (1030, 1028), (2, 4)])
+def test_gemm_stream32(m, n, k, swiglu):
+    """The 32-bit weight-streaming product at whole and partial slices of K, rows that end inside a CTA, strided rows of x.
+    A sum of K products in 32-bit, added up by 256 lanes: an error of a few 2^-24 of the sum's size."""
+    from tokenomos_b200 import ops
+    x, w, b = torch.randn(m, k + 8)[:, 4:4 + k], torch.randn(n, k) * k ** -0.5, torch.randn(n)
+    want = x.double() @ w.double().T + b.double()
+    if swiglu:
+        want = torch.nn.functional.silu(want[:, :n // 2]) * want[:, n // 2:]
+    wide = dev(torch.nn.functional.pad(x, (4, 4)))[:, 4:4 + k]
+    assert ops.gemm_stream32_ok(wide, dev(w))
+    got = ops.gemm_stream32(wide, dev(w), dev(b), swiglu).double().cpu()
+    assert (got - want).norm() <= 1e-6 * want.norm()
+    x = dev(x.contiguous())
+    x[0, 0] = float("inf")                       # infinite rows stay infinite, the others' sums are untouched
+    got = ops.gemm_stream32(x, dev(w.abs() + 0.01)).cpu()
+    assert torch.isinf(got[0]).all() and torch.isfinite(got[1:]).all()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_scale_rows_and_logit_options(dtype):
     from tokenomos_b200 import ops

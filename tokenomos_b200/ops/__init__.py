@@ -729,6 +729,33 @@ def gemm(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
     return out
 
 
+STREAM32_MAX_ROWS = 8
+
+
+def gemm_stream32_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether ``gemm_stream32`` takes this product: float32, at most 8 rows of ``x``, K and the row strides multiples of
+    4 elements, 16-byte aligned."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.is_cuda and 0 < x.shape[0] <= STREAM32_MAX_ROWS
+            and x.shape[1] % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and (x.stride(0) % 4 == 0 or x.shape[0] == 1)
+            and w.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_stream32(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, swiglu: bool = False) -> torch.Tensor:
+    """``x @ w.T (+ bias)`` in 32-bit FMA sums for at most 8 rows of ``x``: a weight-streaming kernel (``w`` is a weight: it
+    is read before the kernel before this one has finished). ``swiglu``: ``w`` holds all gate rows, then all up rows, and
+    the result is ``silu(gate) * up`` of width ``N / 2``."""
+    _cuda(x, w, bias)
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K or not gemm_stream32_ok(x, w):
+        raise KernelError(f"gemm_stream32: x {tuple(x.shape)} {x.dtype} against w {tuple(w.shape)} {w.dtype}")
+    width = N // 2 if swiglu else N
+    out = torch.empty(M, width, dtype=torch.float32, device=x.device)
+    _lib.call("tk_gemm_stream32", _ptr(x), x.stride(0) if M > 1 else K, _ptr(w), w.stride(0), _ptr(_f32vec(bias, "bias", N)),
+              _ptr(out), width, M, N, K, int(swiglu), _stream())
+    return out
+
+
 SKINNY_MAX_ROWS = 16
 
 

@@ -2,8 +2,9 @@
 
 Routes, by storage type:
 
-- float32: the CUDA-core kernel with 32-bit FMA accumulation (``ops.gemm``). No tensor-core or
-  reduced-precision mode can reach it, whatever the process-wide torch flags say.
+- float32: 32-bit FMA sums on the CUDA cores: the weight-streaming kernel for up to 8 rows
+  (``ops.gemm_stream32``), else ``ops.gemm``. No reduced-precision mode can reach it, whatever the
+  process-wide torch flags say.
 - bfloat16: by shape (``route``): the hand-written weight-streaming kernel for a few rows
   (``ops.gemm_skinny``), the TMA + tcgen05 kernel for very tall matrices (``ops.gemm_tc``), else
   the library GEMM (cuBLAS through ``torch.nn.functional.linear``), as the reference engine does
@@ -66,10 +67,10 @@ class Linear:
         w = self.weight
         if x.dtype != w.dtype:
             # a 32-bit matrix in a 16-bit model: widen the input, round the result once
-            y = ops.gemm(x.float().contiguous(), w, self.bias, torch.float32)
+            y = self._product32(x.float().contiguous())
             return y if out_dtype == torch.float32 else y.to(x.dtype)
         if w.dtype == torch.float32:
-            return ops.gemm(x, w, self.bias, torch.float32)
+            return self._product32(x)
         if not x.is_cuda:
             raise ops.KernelError("Linear: CUDA tensors only (there is no CPU path)")
         route = self.route(x)
@@ -91,6 +92,12 @@ class Linear:
                 y += self.bias
             return y if out_dtype == torch.float32 else y.to(x.dtype)
         return F.linear(x, w)
+
+    def _product32(self, x: torch.Tensor) -> torch.Tensor:
+        """32-bit operands: the weight-streaming kernel for a few rows, else ``ops.gemm``."""
+        if ops.gemm_stream32_ok(x, self.weight):
+            return ops.gemm_stream32(x, self.weight, self.bias)
+        return ops.gemm(x, self.weight, self.bias, torch.float32)
 
     def route(self, x: torch.Tensor) -> str:
         """Which kernel takes ``x`` [M, in] (thresholds: ``Tuning``): the register-streaming
