@@ -155,6 +155,26 @@ def test_gemm_float32_is_not_tf32():
     assert (want - 64.0).abs().min().item() > 1e-2   # TF32 inputs would give exactly 64
 
 
+@pytest.mark.parametrize("m, n, k", [(9, 128, 128), (33, 257, 1000), (64, 1024, 1024), (100, 1024, 4608), (129, 300, 2048),
+                                     (300, 130, 516), (513, 129, 132)])
+def test_gemm_32_bit_operands_in_parts(m, n, k):
+    """The tensor-core form of the 32-bit product at every width of its token tile, split along K and not, with partial tiles
+    and chunks: no further from 64 bits than a few 2^-24 (tf32 operands would be off by 2^-11); infinities and NaN end up
+    where 32-bit multiply-adds put them, also beside values that round up to infinity in 16 bits."""
+    from tokenomos_b200 import ops
+    x, w, b = torch.randn(m, k + 4)[:, :k], torch.randn(n, k), torch.randn(n)
+    assert ops.gemm_split32_ok(dev(x), dev(w))
+    got = ops.gemm(dev(torch.nn.functional.pad(x, (0, 4)))[:, :k], dev(w), dev(b)).double().cpu()
+    want = x.double() @ w.double().T + b.double()
+    assert (got - want).norm() <= 4e-7 * want.norm()
+    assert (got - want).abs().max() <= 1e-6 * want.abs().max()
+    x, w = x.contiguous(), w.abs() + 0.1
+    x[1, k // 2], x[3, 3], x[5, 5], w[4, 5] = float("inf"), float("nan"), 3.4e38, 0.0
+    got, want = ops.gemm(dev(x), dev(w)).cpu(), x @ w.T
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert ops.gemm_tc_status() == 0
+
+
 @pytest.mark.parametrize("swiglu", [False, True])
 @pytest.mark.parametrize("m", [1, 2, 3, 8])
 @pytest.mark.parametrize("n, k", [(9216, 1024), (1024, 4608), (70, 36), (1030, 1028), (2, 4)])

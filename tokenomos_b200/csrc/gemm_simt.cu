@@ -1,6 +1,6 @@
 // C[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) on the CUDA cores with 32-bit FMA accumulation.
-// This is the matrix product of the true 32-bit path (no tensor cores, no reduced-precision
-// mode can reach it), and the any-shape fallback of the 16-bit path (16-bit operands widen
+// This is the any-shape matrix product of the true 32-bit path (gemm_stream32.cu takes a few rows,
+// gemm_split32.cu larger sizes in 16-byte rows), and the any-shape fallback of the 16-bit path (16-bit operands widen
 // exactly, the sum stays 32-bit, the result is float or rounded once to 16-bit).
 #include "common.cuh"
 

@@ -713,10 +713,21 @@ def gemm_skinny_conv(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None
     return out
 
 
+SPLIT32_MIN_ROWS, SPLIT32_MIN_SIDE = 9, 128
+
+
+def gemm_split32_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether a 32-bit product goes to the tensor cores in parts that keep all of its 32 bits (csrc/gemm_split32.cu): 16-byte
+    rows, and sizes at which that is the faster way (below 128 rows of ``w`` or columns its 128-row tiles are mostly empty)."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] >= SPLIT32_MIN_ROWS
+            and w.shape[0] >= SPLIT32_MIN_SIDE and x.shape[1] >= SPLIT32_MIN_SIDE and x.shape[1] % 4 == 0
+            and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
 def gemm(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
          out_dtype: torch.dtype | None = None) -> torch.Tensor:
-    """``x @ w.T (+ bias)`` on the CUDA cores with 32-bit accumulation, any shape.
-    ``x`` [M, K] (row stride free), ``w`` [N, K]; ``bias`` float32 [N]."""
+    """``x @ w.T (+ bias)`` with 32-bit accumulation, any shape: on the CUDA cores, or, for 32-bit operands of some size, on
+    the tensor cores in parts that lose nothing of them. ``x`` [M, K] (row stride free), ``w`` [N, K]; ``bias`` float32 [N]."""
     _cuda(x, w, bias)
     M, K = x.shape
     N = w.shape[0]
@@ -724,6 +735,10 @@ def gemm(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
         raise KernelError(f"gemm: x {tuple(x.shape)} {x.dtype} against w {tuple(w.shape)} {w.dtype}")
     out_dtype = out_dtype or x.dtype
     out = torch.empty(M, N, dtype=out_dtype, device=x.device)
+    if out_dtype == torch.float32 and gemm_split32_ok(x, w):
+        _lib.call("tk_gemm_split32", _ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(_f32vec(bias, "bias", N)),
+                  _ptr(out), N, M, N, K, _stream())
+        return out
     _lib.call("tk_gemm_simt", _ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(_f32vec(bias, "bias", N)),
               _ptr(out), N, M, N, K, _dtype_code(x), _dtype_code(out), _stream())
     return out
@@ -831,7 +846,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
 def gemm_tc_status() -> int:
     """0, or where a tensor-core GEMM gave up waiting on a barrier since the last call (the
     kernels bound every wait instead of hanging)."""
-    return _lib.call("tk_gemm_tc_status")
+    return _lib.call("tk_gemm_tc_status") or _lib.call("tk_gemm_split32_status")
 
 
 def sample_status() -> int:

@@ -61,6 +61,8 @@ _SIGNATURES = {
     "tk_conv_gated": [P, L, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P],
     "tk_gemm_skinny_conv": [P, L, P, L, P, P, L, I, I, I, P, P, P, P, P, I, F, P],
     "tk_gemm_simt": [P, L, P, L, P, P, L, I, I, I, I, I, P],
+    "tk_gemm_split32": [P, L, P, L, P, P, L, I, I, I, P],
+    "tk_gemm_split32_status": [],
     "tk_gemm_stream32_max_rows": [],
     "tk_gemm_stream32": [P, L, P, L, P, P, L, I, I, I, I, P],
     "tk_gemm_skinny": [P, L, P, L, P, P, L, I, I, I, I, I, F, P, L, P],
@@ -173,7 +175,8 @@ _QUERIES = {"tk_check_device", "tk_built_for", "tk_set_pdl", "tk_checks_enabled"
             "tk_attn_latent_rows", "tk_attn_latent_max_rank", "tk_gemm_grouped_tile", "tk_attn_latent_mma_rows",
             "tk_attn_latent_mma_supported", "tk_attn_pointwise_rows", "tk_attn_pointwise_mma_supported",
             "tk_attn_pointwise_mma_tokens", "tk_ssd_max_state", "tk_ssd_split", "tk_linmem_max_dim", "tk_linmem_scratch",
-            "tk_attn_biased_mma_supported", "tk_attn_biased_mma_tokens", "tk_gemm_stream32_max_rows"}
+            "tk_attn_biased_mma_supported", "tk_attn_biased_mma_tokens", "tk_gemm_stream32_max_rows",
+            "tk_gemm_split32_status"}
 
 
 _fns: dict = {}

@@ -2,9 +2,9 @@
 
 Routes, by storage type:
 
-- float32: 32-bit FMA sums on the CUDA cores: the weight-streaming kernel for up to 8 rows
-  (``ops.gemm_stream32``), else ``ops.gemm``. No reduced-precision mode can reach it, whatever the
-  process-wide torch flags say.
+- float32: the weight-streaming kernel for up to 8 rows (``ops.gemm_stream32``), else ``ops.gemm``: 32-bit
+  multiply-adds on the CUDA cores, or tensor-core products of operands taken apart so that none of their 32
+  bits is lost. No reduced-precision mode can reach it, whatever the process-wide torch flags say.
 - bfloat16: by shape (``route``): the hand-written weight-streaming kernel for a few rows
   (``ops.gemm_skinny``), the TMA + tcgen05 kernel for very tall matrices (``ops.gemm_tc``), else
   the library GEMM (cuBLAS through ``torch.nn.functional.linear``), as the reference engine does
