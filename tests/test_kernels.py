@@ -371,6 +371,47 @@ def test_attention_far_key_and_window_edge(dtype):
         assert (got.double().cpu().mean().item() > 2.0) == seen
 
 
+@pytest.mark.parametrize("nsplit", [1, 3])
+@pytest.mark.parametrize("window", [None, 1, 33, 100, -48])
+@pytest.mark.parametrize("H, Hkv, P", [(4, 4, 16), (16, 8, 16), (8, 2, 7), (8, 1, 64)])
+def test_attention_f32_equals_the_general_kernel(monkeypatch, H, Hkv, P, window, nsplit):
+    """Prompt tiles and single tokens of the 32-bit kernels for heads of 64, on pools whose other rows are NaN: partial tiles
+    of rows and of keys, windows that begin inside a tile, chunks, splits with more blocks than keys."""
+    from tokenomos_b200 import ops
+    general, seen = ops.attention, {}
+
+    def parts(q, pool, positions, tok_seq, table, tok0, ntok, per_tile, win, scale):
+        win = window                                     # (attention_case's own mask knows no chunks: given as None)
+        seen["want"] = general(q, pool, positions, tok_seq, table, tok0, ntok, per_tile, win, scale)
+        out, per = torch.full_like(q, float("nan")), ops.attention_f32_tokens(H, Hkv)
+        firsts, counts, singles, start = [], [], [], 0
+        for n in torch.bincount(tok_seq.cpu().long()).tolist():
+            if n == 1:
+                singles.append(start)
+            else:
+                for o in range(0, n, per):
+                    firsts.append(start + o)
+                    counts.append(min(per, n - o))
+            start += n
+        ops.attention_f32_prefill(q, pool, out, positions, tok_seq, table, i32(firsts + [0]), i32(counts + [0]), win, scale)
+        ops.attention_f32_decode(q, pool, out, positions, tok_seq, table, i32(singles + [-1]), win, scale, nsplit)
+        return out
+
+    monkeypatch.setattr(ops, "attention", parts)
+    got, _ = attention_case(torch.float32, H, Hkv, 64, P, [(0, 1), (17, 3), (0, 40), (40, 150), (333, 1), (5, 2)])
+    assert torch.isfinite(got).all()
+    assert (got - seen["want"]).norm() <= 2e-6 * seen["want"].norm()
+
+
+def test_swiglu32_vectorised_equals_the_scalar_kernel():
+    """Whole and partial blocks of a row; rows that do not begin on 16 bytes go the scalar way, with the same bits."""
+    from tokenomos_b200 import ops
+    for rows, inter in ((3, 8), (2, 2048), (5, 2052), (1, 4608)):
+        gu = torch.randn(rows, 2 * inter, device="cuda") * 4
+        odd = torch.empty(rows * 2 * inter + 1, device="cuda")[1:].view(rows, 2 * inter).copy_(gu)
+        assert odd.data_ptr() % 16 and torch.equal(ops.swiglu(gu), ops.swiglu(odd))
+
+
 def test_attention_poison_is_a_real_control():
     """If the kernel read a row it must not, the NaN would surface: reading one position too
     many (a table that claims one more token) does surface it."""

@@ -282,6 +282,55 @@ def attention(q: torch.Tensor, kv_pool: torch.Tensor, positions: torch.Tensor,
     return out
 
 
+def attention_f32_supported(heads: int, kv_heads: int, head_dim: int, v_dim: int, row: int, dtype: torch.dtype) -> bool:
+    """Whether ``attention_f32_prefill`` and ``attention_f32_decode`` take a layer: 32-bit storage, keys, values and cache
+    rows of 64, 1, 2, 4 or 8 query heads a KV head."""
+    return (dtype == torch.float32 and head_dim == v_dim == row
+            and bool(_lib.call("tk_attn_f32_supported", heads, kv_heads, head_dim)))
+
+
+def attention_f32_tokens(heads: int, kv_heads: int) -> int:
+    """Tokens of one sequence a tile of ``attention_f32_prefill`` takes."""
+    return _lib.call("tk_attn_f32_tokens", heads, kv_heads)
+
+
+def _check_attention_f32(q, kv_pool, out, name):
+    T, H, D = q.shape
+    _, two, Hkv, P, Dp = kv_pool.shape
+    if (two != 2 or not attention_f32_supported(H, Hkv, D, D, Dp, q.dtype) or kv_pool.dtype != q.dtype or out.shape != q.shape
+            or out.dtype != q.dtype or not (q.is_contiguous() and kv_pool.is_contiguous() and out.is_contiguous())):
+        raise KernelError(f"{name}: q / cache / out layouts do not match")
+    return T, H, D, Hkv, P
+
+
+def attention_f32_prefill(q: torch.Tensor, kv_pool: torch.Tensor, out: torch.Tensor, positions: torch.Tensor,
+                          tok_seq: torch.Tensor, block_table: torch.Tensor, tile_tok0: torch.Tensor,
+                          tile_ntok: torch.Tensor, window: int | None, scale: float) -> None:
+    """``attention`` for the tiles of prompt portions (at most ``attention_f32_tokens`` tokens each) of a 32-bit model with
+    heads of 64; writes those rows of ``out`` [T, H, 64]."""
+    _cuda(q, kv_pool, out, positions, tok_seq, block_table, tile_tok0, tile_ntok)
+    T, H, D, Hkv, P = _check_attention_f32(q, kv_pool, out, "attention_f32_prefill")
+    _lib.call("tk_attn_f32_prefill", _ptr(q), _ptr(kv_pool), _ptr(out), _ptr(_i32(positions, "positions")),
+              _ptr(_i32(tok_seq, "tok_seq")), _ptr(_i32(block_table, "block_table")), block_table.stride(0),
+              _ptr(_i32(tile_tok0, "tile_tok0")), _ptr(_i32(tile_ntok, "tile_ntok")), tile_tok0.numel(), H, Hkv, P,
+              int(window or 0), float(scale), _stream())
+
+
+def attention_f32_decode(q: torch.Tensor, kv_pool: torch.Tensor, out: torch.Tensor, positions: torch.Tensor,
+                         tok_seq: torch.Tensor, block_table: torch.Tensor, tok_index: torch.Tensor | None,
+                         window: int | None, scale: float, nsplit: int) -> None:
+    """The same for sequences that bring one token (``tok_index``: their rows; None: every row of ``q``), each split
+    ``nsplit`` ways over its keys (partial results through scratch memory and a merge kernel)."""
+    _cuda(q, kv_pool, out, positions, tok_seq, block_table, tok_index)
+    T, H, D, Hkv, P = _check_attention_f32(q, kv_pool, out, "attention_f32_decode")
+    n = tok_index.numel() if tok_index is not None else T
+    scratch = torch.empty(n * H * nsplit * (D + 2), dtype=torch.float32, device=q.device) if nsplit > 1 else None
+    _lib.call("tk_attn_f32_decode", _ptr(q), _ptr(kv_pool), _ptr(out), _ptr(_i32(positions, "positions")),
+              _ptr(_i32(tok_seq, "tok_seq")), _ptr(_i32(block_table, "block_table")), block_table.stride(0),
+              _ptr(_i32(tok_index, "tok_index") if tok_index is not None else None), n, H, Hkv, P, int(window or 0),
+              float(scale), int(nsplit), _ptr(scratch), _stream())
+
+
 def _bias_table(bias: torch.Tensor | None, heads: int):
     """(pointer, columns) of a bias by distance [heads, L], or (None, 0)."""
     if bias is None:

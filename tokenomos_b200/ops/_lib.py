@@ -36,6 +36,10 @@ _SIGNATURES = {
     "tk_qk_norm_rope_write": [P, L, P, P, P, P, F, P, P, P, P, I, I, I, I, I, I, I, I, P],
     "tk_attn_generic_rows": [],
     "tk_attn_generic": [P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, I, I, I, F, F, P, I, I, P],
+    "tk_attn_f32_supported": [I, I, I],
+    "tk_attn_f32_tokens": [I, I],
+    "tk_attn_f32_prefill": [P, P, P, P, P, P, I, P, P, I, I, I, I, I, F, P],
+    "tk_attn_f32_decode": [P, P, P, P, P, P, I, P, I, I, I, I, I, F, I, P, P],
     "tk_rotary_write": [P, L, P, P, P, F, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P],
     "tk_stream32_add_norm": [P, P, L, P, P, P, F, P, P, P, I, I, I, P],
     "tk_glu_clamped": [P, P, I, I, I, F, F, F, I, P],
@@ -176,7 +180,7 @@ _QUERIES = {"tk_check_device", "tk_built_for", "tk_set_pdl", "tk_checks_enabled"
             "tk_attn_latent_mma_supported", "tk_attn_pointwise_rows", "tk_attn_pointwise_mma_supported",
             "tk_attn_pointwise_mma_tokens", "tk_ssd_max_state", "tk_ssd_split", "tk_linmem_max_dim", "tk_linmem_scratch",
             "tk_attn_biased_mma_supported", "tk_attn_biased_mma_tokens", "tk_gemm_stream32_max_rows",
-            "tk_gemm_split32_status"}
+            "tk_gemm_split32_status", "tk_attn_f32_supported", "tk_attn_f32_tokens"}
 
 
 _fns: dict = {}

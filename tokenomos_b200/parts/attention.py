@@ -360,17 +360,36 @@ class Attention:
             elif gate is not None:
                 ops.sigmoid_gate(out, gate)
             return out
-        rows = ops.attention_rows()
-        group = self.heads // self.kv_heads
-        per_tile = max(1, rows // group)
-        _, tok0, _, ntok = ctx.tiles(per_tile)
-        out = ops.attention(q, pool, ctx.positions, ctx.tok_seq, table, tok0, ntok, per_tile,
-                            self.reach, self.scale, self.keep_first, self.sink, self.v_dim,
-                            round_p=not self.exact)
+        if not (self.sink or self.keep_first) and ops.attention_f32_supported(
+                self.heads, self.kv_heads, self.head_dim, self.v_dim, pool.shape[-1], q.dtype):
+            out = self._attend_f32(q, pool, table, ctx)
+        else:
+            rows = ops.attention_rows()
+            group = self.heads // self.kv_heads
+            per_tile = max(1, rows // group)
+            _, tok0, _, ntok = ctx.tiles(per_tile)
+            out = ops.attention(q, pool, ctx.positions, ctx.tok_seq, table, tok0, ntok, per_tile,
+                                self.reach, self.scale, self.keep_first, self.sink, self.v_dim,
+                                round_p=not self.exact)
         if gate is not None and self.gate_kind == "head":
             ops.head_gate(out, gate, self.heads, self.v_dim)
         elif gate is not None:
             ops.sigmoid_gate(out, gate)
+        return out
+
+    def _attend_f32(self, q, pool, table, ctx: StepContext) -> torch.Tensor:
+        """32-bit models with heads of 64: prompt portions in tiles of 64 rows, single tokens shared out over their keys."""
+        out = torch.empty_like(q)
+        if not ctx.host.decode_only:
+            _, tok0, _, ntok = ctx.tiles(ops.attention_f32_tokens(self.heads, self.kv_heads), "multi")
+            if tok0.numel():
+                ops.attention_f32_prefill(q, pool, out, ctx.positions, ctx.tok_seq, table, tok0, ntok, self.reach, self.scale)
+        singles = None if ctx.host.decode_only else ctx.singles()
+        rows = ctx.n_tokens if singles is None else singles.numel()
+        if rows:
+            longest = min(ctx.host.longest, self.span) if self.span is not None else ctx.host.longest
+            nsplit = self.decode_splits(rows, self.kv_heads, longest, self.tuning)
+            ops.attention_f32_decode(q, pool, out, ctx.positions, ctx.tok_seq, table, singles, self.reach, self.scale, nsplit)
         return out
 
     def _value_rows(self, qkv: torch.Tensor, ctx: StepContext, call: int) -> ValueRows | None:
