@@ -922,3 +922,57 @@ def test_trace_program_and_command_line(folders, tmp_path):
     lines = [json.loads(ln) for ln in proc.stdout.splitlines() if ln.startswith("{")]
     assert len(lines) == 1 and len(lines[0]["token_ids"]) == 5
     teacher_forced_ok(CASES[name]["config"], folders[name][1], [1, 2, 3, 4], lines[0]["token_ids"], 1e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H, V, N, G, lens, ctx", [(4, 64, 128, 2, (2000, 1, 65, 64, 877), (0, 5, 9, 0, 3)), (2, 128, 64, 1, (321,), (7,)),
+                                                   (3, 64, 64, 3, (0, 996, 0, 1130), (0, 0, 0, 2))])
+def test_scan_by_chunks(H, V, N, G, lens, ctx, dtype):
+    """The chunked form of the scan over portions that end inside a chunk and on its edge, behind states and from nothing,
+    beside empty sequences: against the recurrence in 64-bit, decays from 1 to e^-40 a token among them. In 32-bit the sums of
+    up to 128 + 64 products are off by a few 2^-24; a token that is not finite reaches no token before it."""
+    from tokenomos_b200 import ops
+    dt_ = getattr(torch, dtype)
+    g = torch.Generator().manual_seed(5)
+    T, S = sum(lens), len(lens)
+    xbc = torch.randn(T, H * V + 2 * G * N + 12, generator=g).to(dt_)
+    raw = torch.randn(T, H + 4, generator=g) * 2
+    raw[::17] += 8.0
+    bias, a_log, skip = (torch.randn(H, generator=g) for _ in range(3))
+    a_log[0] = 1.5
+    state = torch.randn(S + 1, H, N, V, generator=g)
+    assert ops._lib.call("tk_ssd_chunked_scratch", T, S, H, V, N, G) > 0
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    slots = list(range(S, 0, -1))
+    run = lambda rows, st: ops.ssd_scan(rows, raw.cuda(), bias.cuda(), a_log.cuda(), skip.cuda(), st, i32(cu), i32(list(ctx)),  # noqa: E731
+                                        i32(slots), S, H, V, N, G)
+    st = state.cuda()
+    wide = torch.nn.functional.pad(xbc, (0, 4)).cuda()[:, :xbc.shape[1]]
+    got = run(wide, st)
+    assert tuple(got.shape) == (1, T, H * V)
+    want, after = torch.empty(T, H, V, dtype=torch.float64), state.double()
+    x = xbc[:, :H * V].double().view(T, H, V)
+    B = xbc[:, H * V:H * V + G * N].double().view(T, G, N).repeat_interleave(H // G, 1)
+    C = xbc[:, H * V + G * N:H * V + 2 * G * N].double().view(T, G, N).repeat_interleave(H // G, 1)
+    step = torch.nn.functional.softplus(raw[:, :H].double() + bias.double())
+    decay = torch.exp(-torch.exp(a_log.double()) * step)
+    for s in range(S):
+        M = after[slots[s]] if ctx[s] else torch.zeros(H, N, V, dtype=torch.float64)
+        for t in range(cu[s], cu[s + 1]):
+            M = decay[t, :, None, None] * M + step[t, :, None, None] * B[t][:, :, None] * x[t][:, None, :]
+            want[t] = torch.einsum("hn,hnv->hv", C[t], M) + skip.double()[:, None] * x[t]
+        if lens[s]:
+            after[slots[s]] = M
+    err = (got[0].double().cpu().view(T, H, V) - want).norm() / want.norm()
+    assert err <= 1e-6, err
+    assert (st.double().cpu() - after).norm() <= 1e-6 * after.norm()
+    last = max(range(S), key=lambda s: lens[s])
+    t = cu[last] + lens[last] // 2
+    wide[t, 0] = float("nan")                    # a value of x, and of B, at one token
+    wide[t, H * V] = float("inf")
+    again = run(wide, state.cuda())[0].view(T, H * V)
+    assert torch.equal(again[:t], got[0][:t]) and torch.isnan(again[t]).any()

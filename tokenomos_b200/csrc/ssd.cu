@@ -20,7 +20,7 @@
 // step continues from the stored S exactly where the step before left it.
 #include <math.h>
 
-#include "common.cuh"
+#include "chunked.cuh"
 
 namespace {
 enum : int { TK_K_SSD = 11 };
@@ -303,6 +303,41 @@ TK_API int tk_ssd_scan(const void* xbc, int64_t xbc_stride, const float* dt_raw,
 #undef TK_SSD
     TK_CHECK_LAUNCH("ssd_scan");
     return 0;
+}
+
+// The same recurrence chunk by chunk (chunked.cuh): float32 words of scratch it needs, 0 where it does not take the sizes or
+// the walk is the better way. The walk's time is its longest sequence's (0.19 us a token) until the sequences fill the GPU,
+// the chunks' that of all tokens together. 32 heads of 64 x 128, chunks against walk: one sequence of 200 tokens 50 us
+// against 44, of 700 72 against 139, of 2,048 142 against 396; four of 256 94 against 74, of 512 about equal; sixteen of 128
+// 200 against 132. So the line lies at 256 tokens a sequence and 64 more for every one; and at 512 MB of scratch.
+TK_API int tk_ssd_chunked_scratch(int tokens, int n_seqs, int H, int V, int N, int G) {
+    if (!chunked_takes(V, N) || n_seqs <= 0 || n_seqs > 1024 || tokens < n_seqs * (256 + 64 * n_seqs) || G <= 0 || H % G) return 0;
+    const int64_t words = chunked_scratch(tokens, n_seqs, H, V, N, G);
+    return words <= (int64_t)128 << 20 ? (int)words : 0;
+}
+
+// As tk_ssd_scan, with y [T, H V] (one part); xbc's rows and bases in whole groups of four elements.
+TK_API int tk_ssd_chunked(const void* xbc, int64_t xbc_stride, const float* dt_raw, int64_t dt_stride, const float* dt_bias,
+                          const float* A_log, const float* D_skip, float* state, const int* cu_seqlens, const int* seq_ctx,
+                          const int* seq_slot, int n_seqs, int tokens, float* y, int H, int V, int N, int G, float* scratch,
+                          int dtype, cudaStream_t stream) {
+    TK_CHECK_ARG(chunked_takes(V, N) && n_seqs > 0 && tokens > 0 && H > 0 && G > 0 && H % G == 0, "state-space chunks: %d tokens of %d sequences, heads of %d x %d",
+                 tokens, n_seqs, N, V);
+    const int es = dtype == TK_F32 ? 4 : 2;
+    TK_CHECK_ARG(xbc_stride % 4 == 0 && (uintptr_t)xbc % (4 * es) == 0 && (uintptr_t)scratch % 16 == 0,
+                 "state-space chunks: rows in whole groups of four elements");
+    TK_CHECK_ARG(dtype == TK_F32 || dtype == TK_BF16, "state-space chunks: unknown dtype %d", dtype);
+    Chunked m = {};
+    const char* base = (const char*)xbc;
+    m.x = {base, V, xbc_stride};
+    m.b = {base + (int64_t)H * V * es, N, xbc_stride};
+    m.c = {base + ((int64_t)H * V + (int64_t)G * N) * es, N, xbc_stride};
+    m.cu_seqlens = cu_seqlens, m.seq_ctx = seq_ctx, m.seq_slot = seq_slot;
+    m.n_seqs = n_seqs, m.H = H, m.V = V, m.N = N, m.groups = G;
+    m.y = y, m.state = state, m.state_vn = 0, m.check = TK_K_SSD;
+    const SsdDecay d = {dt_raw, dt_stride, dt_bias, A_log, D_skip};
+    return dtype == TK_F32 ? launch_chunked<float, float>(m, d, scratch, tokens, stream)
+                           : launch_chunked<__nv_bfloat16, __nv_bfloat16>(m, d, scratch, tokens, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1538,7 +1538,8 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
     n_state] (rows may be strided): x, then B, then C; ``dt_raw`` float32 [T, >= heads]; ``state`` float32 [slots,
     heads, n_state, v_dim]. Returns ``y`` float32 [parts, T, heads v_dim]: a step of few, long portions is walked
     by several blocks a head, each over a part of the state's rows, and their sums are still to be added
-    (``gated_group_norm`` does; ``y.sum(0)`` is the result)."""
+    (``gated_group_norm`` does; ``y.sum(0)`` is the result). Few, long portions of states the chunked kernels take are formed
+    chunk by chunk instead (one part)."""
     _cuda(xbc, dt_raw, dt_bias, a_log, d_skip, state)
     T = xbc.shape[0]
     if xbc.stride(1) != 1 or xbc.shape[1] < heads * v_dim + 2 * groups * n_state:
@@ -1547,6 +1548,17 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
         raise KernelError(f"ssd_scan: dt is float32 [{T}, >= {heads}]")
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, n_state, v_dim) or not state.is_contiguous():
         raise KernelError(f"ssd_scan: the state is float32 [slots, {heads}, {n_state}, {v_dim}]")
+    words = _lib.call("tk_ssd_chunked_scratch", T, int(n_seqs), heads, v_dim, n_state, groups)
+    if words and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0:
+        # portions of some length: chunk by chunk, all side by side
+        scratch = torch.empty(words, dtype=torch.float32, device=xbc.device)
+        y = torch.empty(1, T, heads * v_dim, dtype=torch.float32, device=xbc.device)
+        _lib.call("tk_ssd_chunked", _ptr(xbc), xbc.stride(0), _ptr(dt_raw), dt_raw.stride(0),
+                  _ptr(_f32vec(dt_bias, "dt_bias", heads)), _ptr(_f32vec(a_log, "A_log", heads)),
+                  _ptr(_f32vec(d_skip, "D", heads)), _ptr(state), _ptr(_i32(cu_seqlens, "cu_seqlens")),
+                  _ptr(_i32(seq_ctx, "seq_ctx")), _ptr(_i32(seq_slot, "seq_slot")), int(n_seqs), T, _ptr(y), heads, v_dim,
+                  n_state, groups, _ptr(scratch), _dtype_code(xbc), _stream())
+        return y
     split = _lib.call("tk_ssd_split", T, int(n_seqs), heads, v_dim, n_state, int(sm_count))
     y = torch.empty(split, T, heads * v_dim, dtype=torch.float32, device=xbc.device)
     _lib.call("tk_ssd_scan", _ptr(xbc), xbc.stride(0), _ptr(dt_raw), dt_raw.stride(0), _ptr(_f32vec(dt_bias, "dt_bias", heads)),

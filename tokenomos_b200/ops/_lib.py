@@ -109,6 +109,8 @@ _SIGNATURES = {
     "tk_mlstm_norm_gate": [P, P, P, P, P, L, P, P, P, P, I, I, I, F, I, P],
     "tk_ssd_max_state": [],
     "tk_ssd_scan": [P, L, P, L, P, P, P, P, P, P, P, I, I, P, I, I, I, I, I, I, P],
+    "tk_ssd_chunked_scratch": [I, I, I, I, I, I],
+    "tk_ssd_chunked": [P, L, P, L, P, P, P, P, P, P, P, I, I, P, I, I, I, I, P, I, P],
     "tk_ssd_split": [I, I, I, I, I, I],
     "tk_gated_group_norm": [P, I, P, L, P, F, P, I, I, I, I, P],
     "tk_qkv_maps_write": [P, L, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, P],
@@ -180,7 +182,7 @@ _QUERIES = {"tk_check_device", "tk_built_for", "tk_set_pdl", "tk_checks_enabled"
             "tk_attn_latent_mma_supported", "tk_attn_pointwise_rows", "tk_attn_pointwise_mma_supported",
             "tk_attn_pointwise_mma_tokens", "tk_ssd_max_state", "tk_ssd_split", "tk_linmem_max_dim", "tk_linmem_scratch",
             "tk_attn_biased_mma_supported", "tk_attn_biased_mma_tokens", "tk_gemm_stream32_max_rows",
-            "tk_gemm_split32_status", "tk_attn_f32_supported", "tk_attn_f32_tokens"}
+            "tk_gemm_split32_status", "tk_attn_f32_supported", "tk_attn_f32_tokens", "tk_ssd_chunked_scratch"}
 
 
 _fns: dict = {}
