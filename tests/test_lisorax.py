@@ -779,6 +779,32 @@ def test_gated_activation_in_the_grouped_products_epilogue(E, ff, width, T, top)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("act", [False, True, "swiglu8", "clamped8"])
+@pytest.mark.parametrize("tile", [8, 16])
+@pytest.mark.parametrize("E, N, K, T, top", [(5, 48, 40, 37, 2), (3, 272, 1032, 50, 3), (9, 16, 8, 3, 4)])
+def test_streamed_product_of_a_few_rows_an_expert(E, N, K, T, top, tile, act):
+    """Tiles of 8 and 16 rows of the sorted layout, partial slices of K, columns that end inside a CTA, gathered rows and rows
+    where they are, padding left alone: the bits of the general grouped product but for the order of its sums."""
+    from tokenomos_b200 import ops
+
+    g = torch.Generator().manual_seed(E * 100 + N)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(E, N, K, generator=g) * K ** -0.5).to(torch.bfloat16).cuda()
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32).cuda()
+    clamp = (1.5, 1.7, 1.0)
+    row_token, pair_row, tile_expert = ops.moe_sort(idx, E, tile)
+    got = ops.moe_stream(x, w, tile_expert, row_token, True, tile, act, clamp)[pair_row.long()]
+    rows = torch.where((row_token >= 0)[:, None], x[row_token.clamp(min=0).long()], torch.full_like(x[:1], float("nan")))
+    again = ops.moe_stream(rows, w, tile_expert, row_token, False, tile, act, clamp)[pair_row.long()]
+    t64, p64, e64 = ops.moe_sort(idx, E, 64)
+    want = ops.gemm_grouped(x, w, e64, t64, t64.numel(), act=act, clamp=clamp)[p64.long()]
+    assert torch.equal(got, again)
+    # one rounding to 16 bits where sums differ in their last places (gate and up are rounded before the activation too)
+    assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
+    assert (got.float() - want.float()).norm() <= 2e-3 * want.float().norm()
+
+
+@pytest.mark.gpu
 def test_router_takes_the_lowest_index_of_equal_logits(tmp_path):
     width = 32
     layer = dict(mlstm(1, 8, 8, 5.0), mlp=moe(6, 2, 16))

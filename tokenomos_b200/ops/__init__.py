@@ -1245,6 +1245,40 @@ def gemm_grouped(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, row
     return out
 
 
+def moe_stream_tile(x: torch.Tensor, up: torch.Tensor, down: torch.Tensor, pairs: int) -> int:
+    """Rows of a tile of ``moe_stream`` for ``pairs`` (token, expert) rows, 0 where the tiles of ``gemm_grouped`` are the better
+    way: 8 up to five rows an expert on average, 16 up to sixteen; bfloat16 rows in whole 16-byte chunks. (A mixture of 32
+    experts of 2,048 x 1,536, us with tiles of 8, of 16, with ``gemm_grouped``: two rows an expert 134, 141, 215; six 151, 155,
+    222; eight 165, 159, 223; sixteen 235, 207, 225; twenty-four 304, 253, 227. 16 of 1,024 x 1,536: four 62, 62, 105; eight
+    71, 66, 104; sixteen 85, 81, 106; twenty-four 106, 94, 108.)"""
+    experts = up.shape[0]
+    if not (_grouped_mma_ok(x, up, up.shape[1], up.shape[2]) and _grouped_mma_ok(x, down, down.shape[1], down.shape[2])
+            and x.stride(1) == 1 and up.is_contiguous() and down.is_contiguous()):
+        return 0
+    return 8 if pairs <= 5 * experts else 16 if pairs <= 16 * experts else 0
+
+
+def moe_stream(a: torch.Tensor, w: torch.Tensor, tile_group: torch.Tensor, row_token: torch.Tensor, gather: bool, tile: int,
+               act: bool | str = False, clamp: tuple | None = None) -> torch.Tensor:
+    """``gemm_grouped`` for steps of a few rows an expert: a weight-streaming kernel over tiles of 8 or 16 rows of the sorted
+    layout (``moe_stream_tile``). ``row_token`` [rows]: -1 marks padding, whose rows are not written; ``gather``: row m reads
+    ``a[row_token[m]]``, else ``a[m]``. ``act`` and ``clamp`` as there."""
+    _cuda(a, w, tile_group, row_token)
+    _, N, K = w.shape
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or a.stride(1) != 1 or not w.is_contiguous() or a.shape[1] != K:
+        raise KernelError(f"moe_stream: a {tuple(a.shape)} {a.dtype} against w {tuple(w.shape)} {w.dtype}")
+    rows, gated = row_token.numel(), act in ("swiglu8", "clamped8")
+    if tile_group.numel() * tile != rows or (not gather and a.shape[0] < rows):
+        raise KernelError(f"moe_stream: {rows} rows in {tile_group.numel()} tiles of {tile}")
+    limit, alpha, shift = clamp if act == "clamped8" else (None, 1.0, 0.0)
+    out = torch.empty(rows, N // 2 if gated else N, dtype=a.dtype, device=a.device)
+    _lib.call("tk_moe_stream", _ptr(a), a.stride(0), _ptr(_i32(row_token, "row_token")), int(bool(gather)), _ptr(w),
+              _ptr(_i32(tile_group, "tile_group")), _ptr(out), out.shape[1], rows, N, K,
+              {"clamped8": 3, "swiglu8": 2}.get(act, int(bool(act))), int(tile), float(limit or 0.0), float(alpha), float(shift),
+              _stream())
+    return out
+
+
 def gemm_grouped_fuses_swiglu(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether ``gemm_grouped(a, w, ..., act="swiglu8")`` is built for these operands."""
     N, K = w.shape[-2:]

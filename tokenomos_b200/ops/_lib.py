@@ -95,6 +95,7 @@ _SIGNATURES = {
     "tk_gemm_grouped_tile": [],
     "tk_gemm_grouped_simt": [P, L, L, P, P, L, L, P, P, L, L, I, I, I, I, I, I, P],
     "tk_gemm_grouped_mma": [P, L, L, P, P, L, L, P, P, L, L, I, I, I, I, I, I, P, L, F, F, F, P],
+    "tk_moe_stream": [P, L, P, I, P, P, P, L, I, I, I, I, I, F, F, F, P],
     "tk_moe_combine": [P, P, P, P, P, P, I, I, I, I, P],
     "tk_relu2": [P, L, I, P],
     "tk_scale_rows_f32": [P, L, P, F, I, I, I, P],

@@ -96,6 +96,14 @@ class RoutedExperts:
         if self.library and x.shape[0] * self.top >= self.library_rows:
             y, pair_row = self._experts_library(x, idx)
             return ops.moe_combine(y, pair_row, w, self._shared(x), gate)
+        tile = ops.moe_stream_tile(x, self.up, self.down, x.shape[0] * self.top)
+        if tile and (not self.gated or self.gate_run):
+            # a few rows an expert: the chosen experts' weights streamed past tiles of as few rows
+            row_token, pair_row, tile_expert = ops.moe_sort(idx, self.experts, tile)
+            kind = True if not self.gated else "swiglu8" if self.activation == "swiglu" else "clamped8"
+            act = ops.moe_stream(x, self.up, tile_expert, row_token, True, tile, kind, self.clamp)
+            y = ops.moe_stream(act, self.down, tile_expert, row_token, False, tile)
+            return ops.moe_combine(y, pair_row, w, self._shared(x), gate)
         # (both products, [ff, width] and [width, ff], must take the tile: the common divisor stands for both sizes)
         tile = ops.gemm_grouped_tiles(x.dtype, math.gcd(self._tile_n, self.ff), math.gcd(self._tile_n, self.ff),
                                       x.shape[0] * self.top)
