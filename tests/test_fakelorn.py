@@ -976,3 +976,83 @@ def test_scan_by_chunks(H, V, N, G, lens, ctx, dtype):
     wide[t, H * V] = float("inf")
     again = run(wide, state.cuda())[0].view(T, H * V)
     assert torch.equal(again[:t], got[0][:t]) and torch.isnan(again[t]).any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [2, 3, 4])
+@pytest.mark.parametrize("C, tile", [(4, 4), (516, 16), (1028, 5)])
+def test_four_channels_a_thread_give_the_scalar_convolutions_bits(C, tile, K):
+    """Portions shorter than the taps, tiles that end inside the loads in flight, states and their absence, a bias, a residual
+    and the activation; rows that do not begin on 8 bytes go the scalar way."""
+    from tokenomos_b200 import ops
+    g = torch.Generator().manual_seed(C + K)
+    lens, ctx, slots = (1, 37, 2, 70, 0, 16), (5, 0, 1, 9, 3, 0), (3, 1, 6, 2, 5, 4)
+    T = sum(lens)
+    wide = torch.randn(T, C + 5, generator=g).to(torch.bfloat16).cuda()
+    taps, bias, state = (torch.randn(*shape, generator=g).cuda() for shape in ((C, K), (C,), (7, K - 1, C)))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    cu, tiles = [0], ([], [], [], [])
+    for s, n in enumerate(lens):
+        for o in range(0, n, tile):
+            for col, v in zip(tiles, (s, cu[-1] + o, o, min(tile, n - o))):
+                col.append(v)
+        cu.append(cu[-1] + n)
+    odd = wide[:, 1:1 + C]
+    even = torch.empty(T, C + 4, dtype=torch.bfloat16, device="cuda")[:, :C].copy_(odd)
+    assert odd.data_ptr() % 8 and not even.data_ptr() % 8
+    for residual, act, b in ((False, True, bias), (True, False, None)):
+        s1, s2 = state.clone(), state.clone()
+        args = (i32(cu), i32(list(ctx)), i32(list(slots)), tuple(i32(t) for t in tiles), torch.bfloat16)
+        want = ops.seq_conv(odd, taps, b, s1, *args, residual=residual, act=act)
+        got = ops.seq_conv(even, taps, b, s2, *args, residual=residual, act=act)
+        assert torch.equal(got, want) and torch.equal(s1, s2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("groups, part", [(3, 4), (2, 128), (5, 132), (2, 512), (2, 516), (3, 30)])
+def test_norms_with_a_gate_at_the_edges_of_their_forms(groups, part, dtype):
+    """Parts of one to sixteen steps of four elements a lane, longer ones and ones that are no whole steps, with the sums of a
+    scan left in two parts."""
+    from tokenomos_b200 import ops
+    g = torch.Generator().manual_seed(part)
+    rows, width = 19, groups * part
+    y = torch.randn(2, rows, width, generator=g)
+    z = torch.randn(rows, width + 4, generator=g).to(dtype)
+    w = torch.randn(width, generator=g)
+    zz = z[:, :width].double()
+    silu = zz * torch.sigmoid(zz)
+    want = plain.group_norm(y.double().sum(0) * silu, w.double(), groups, 1e-6)
+    got = ops.gated_group_norm(y.cuda(), z.cuda()[:, :width], w.cuda(), 1e-6, groups).double().cpu()
+    tol = 2e-6 if dtype == torch.float32 else 2.0 ** -8           # one rounding to the storage type
+    assert (got - want).abs().max() <= tol * want.abs().max()
+    want = plain.group_norm(y[0].double(), w.double(), groups, 1e-6) * silu
+    got = ops.norm_gate(y[0].cuda(), z.cuda()[:, :width], w.cuda(), 1e-6, groups, "silu").double().cpu()
+    assert (got - want).abs().max() <= (4 * tol) * want.abs().max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("E, T, top, tile, width", [(1, 3, 1, 8, 64), (40, 700, 3, 8, 2048), (1030, 900, 2, 64, 1032), (33, 5, 5, 16, 30)])
+def test_rows_sorted_by_expert_and_combined(E, T, top, tile, width):
+    """Every pair has a row of its own in a tile of its expert, padding and unused tiles are marked, the experts' blocks end where
+    they say; the combination adds a token's rows by their weights."""
+    from tokenomos_b200 import ops
+    g = torch.Generator().manual_seed(E)
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32)
+    row_token, pair_row, tile_expert, ends = (t.cpu() for t in ops.moe_sort(idx.cuda(), E, tile, ends=True))
+    assert len(set(pair_row.tolist())) == T * top
+    for p, r in enumerate(pair_row.tolist()):
+        assert row_token[r] == p // top and tile_expert[r // tile] == idx.reshape(-1)[p]
+    assert int((row_token >= 0).sum()) == T * top
+    tiles = [-(-int(c) // tile) for c in torch.bincount(idx.reshape(-1).long(), minlength=E)]
+    assert ends.tolist() == [tile * sum(tiles[:e + 1]) for e in range(E)]
+    assert (tile_expert[sum(tiles):] == -1).all() and (tile_expert[:sum(tiles)] >= 0).all()
+    Y = torch.randn(row_token.numel(), width, generator=g).to(torch.bfloat16)
+    w, shared, gate = torch.rand(T, top, generator=g), torch.randn(T, width, generator=g).to(torch.bfloat16), torch.rand(T, generator=g)
+    for sh, gt in ((shared, gate), (shared, None), (None, None)):
+        got = ops.moe_combine(Y.cuda(), pair_row.cuda(), w.cuda(), sh.cuda() if sh is not None else None,
+                              gt.cuda() if gt is not None else None).double().cpu()
+        want = (Y.double()[pair_row.long()].view(T, top, width) * w.double()[:, :, None]).sum(1)
+        if sh is not None:
+            want = want + sh.double() * (gt.double()[:, None] if gt is not None else 1.0)
+        assert (got - want).abs().max() <= 2.0 ** -8 * want.abs().max()

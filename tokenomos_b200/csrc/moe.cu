@@ -136,17 +136,34 @@ moe_sort_kernel(const int* idx, int pairs, int top, int E, int tile, int cap_row
     for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&count[idx[p]], 1);
     for (int r = threadIdx.x; r < cap_rows; r += blockDim.x) row_token[r] = -1;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0;
-        for (int e = 0; e < E; ++e) {
-            start[e] = at;
-            const int tiles = (count[e] + tile - 1) / tile;
-            for (int k = 0; k < tiles; ++k) tile_expert[at / tile + k] = e;
-            at += tiles * tile;
-            if (expert_end != nullptr) expert_end[e] = at;      // where the expert's padded block ends
+    // where every expert's whole tiles begin: a scan of their counts, 1,024 experts at a time (8,192 pairs
+    // in tiles of 8: 9.2 us; 18.8 with one thread walking experts and tiles)
+    __shared__ int warp_total[32], base_s;
+    if (threadIdx.x == 0) base_s = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int e0 = 0; e0 < E; e0 += blockDim.x) {
+        const int e = e0 + threadIdx.x, tiles = e < E ? (count[e] + tile - 1) / tile : 0;
+        int sum = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += up;
         }
-        for (int k = at / tile; k < cap_rows / tile; ++k) tile_expert[k] = -1;
+        if (lane == 31) warp_total[warp] = sum;
+        __syncthreads();
+        int before = base_s;
+        for (int w = 0; w < warp; ++w) before += warp_total[w];
+        const int at = before + sum - tiles;                     // in tiles
+        if (e < E) {
+            start[e] = at * tile;
+            for (int k = 0; k < tiles; ++k) tile_expert[at + k] = e;
+            if (expert_end != nullptr) expert_end[e] = (at + tiles) * tile;      // where the expert's padded block ends
+        }
+        __syncthreads();
+        if (threadIdx.x == blockDim.x - 1) base_s = at + tiles;
+        __syncthreads();
     }
+    for (int k = base_s + threadIdx.x; k < cap_rows / tile; k += blockDim.x) tile_expert[k] = -1;
     __syncthreads();
     for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
         const int e = idx[p];
@@ -296,6 +313,56 @@ moe_combine_kernel(const T* Y, const int* pair_row, const float* w, const T* sha
     }
 }
 
+// The same 16 bytes a thread and row (rows in whole 16-byte chunks): all of a token's rows in flight together, the sums in the
+// same order (2,048 tokens of 4 rows of 2,048, 50 MB: 10.1 us, one element at a time 21.4).
+__global__ void __launch_bounds__(256)
+moe_combine_vec_kernel(const __nv_bfloat16* Y, const int* pair_row, const float* w, const __nv_bfloat16* shared, const float* gate,
+                       __nv_bfloat16* out, int top, int width) {
+    constexpr int TOGETHER = 4;
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t t = blockIdx.x;
+    const float g = shared != nullptr ? (gate != nullptr ? gate[t] : 1.f) : 0.f;
+    auto add = [](float (&v)[8], const uint4& raw, float f) {
+        const uint32_t* p = &raw.x;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + e));
+            v[2 * e] = fmaf(f, x.x, v[2 * e]);
+            v[2 * e + 1] = fmaf(f, x.y, v[2 * e + 1]);
+        }
+    };
+    for (int i = threadIdx.x * 8; i < width; i += blockDim.x * 8) {
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+        uint4 sh = make_uint4(0u, 0u, 0u, 0u);
+        if (shared != nullptr) sh = *reinterpret_cast<const uint4*>(shared + t * width + i);
+        for (int k0 = 0; k0 < top; k0 += TOGETHER) {
+            uint4 raw[TOGETHER];
+            float f[TOGETHER];
+#pragma unroll
+            for (int k = 0; k < TOGETHER; ++k)
+                if (k0 + k < top) {
+                    raw[k] = *reinterpret_cast<const uint4*>(Y + (size_t)pair_row[t * top + k0 + k] * width + i);
+                    f[k] = w[t * top + k0 + k];
+                }
+#pragma unroll
+            for (int k = 0; k < TOGETHER; ++k)
+                if (k0 + k < top) add(v, raw[k], f[k]);
+        }
+        if (shared != nullptr) add(v, sh, g);
+        uint4 packed;
+        uint32_t* o = &packed.x;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+            o[e] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+        *reinterpret_cast<uint4*>(out + t * width + i) = packed;
+    }
+}
+
 TK_API int tk_moe_combine(const void* Y, const int* pair_row, const float* w, const void* shared,
                           const float* gate, void* out, int tokens, int top, int width, int dtype,
                           cudaStream_t stream) {
@@ -304,6 +371,9 @@ TK_API int tk_moe_combine(const void* Y, const int* pair_row, const float* w, co
     if (dtype == TK_F32)
         tk_launch(moe_combine_kernel<float>, dim3(tokens), dim3(256), 0, stream, (const float*)Y, pair_row, w,
                   (const float*)shared, gate, (float*)out, top, width);
+    else if (dtype == TK_BF16 && width % 8 == 0 && ((uintptr_t)Y | (uintptr_t)shared | (uintptr_t)out) % 16 == 0)
+        tk_launch(moe_combine_vec_kernel, dim3(tokens), dim3(width >= 2048 ? 256 : width >= 1024 ? 128 : 64), 0, stream,
+                  (const __nv_bfloat16*)Y, pair_row, w, (const __nv_bfloat16*)shared, gate, (__nv_bfloat16*)out, top, width);
     else if (dtype == TK_BF16)
         tk_launch(moe_combine_kernel<__nv_bfloat16>, dim3(tokens), dim3(256), 0, stream, (const __nv_bfloat16*)Y,
                   pair_row, w, (const __nv_bfloat16*)shared, gate, (__nv_bfloat16*)out, top, width);

@@ -384,6 +384,55 @@ gated_group_norm_kernel(const float* y, int parts, const T* z, int64_t z_stride,
     }
 }
 
+// The same four neighbouring elements a lane and step (16 bytes of y, 8 or 16 of z), QUADS of them in registers: rows of 2,048 in
+// four groups, 2,048 tokens (34 MB): 11.2 us, one element at a time 20.8.
+template <typename T, int QUADS>
+__global__ void __launch_bounds__(128)
+gated_group_norm_quad_kernel(const float* y, int parts, const T* z, int64_t z_stride, const float* __restrict__ w, float eps,
+                             T* out, int rows, int width, int groups) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (warp >= rows * groups) return;
+    const int r = warp / groups, gw = width / groups, c0 = (warp % groups) * gw;
+    float4 keep[QUADS], zv[QUADS];
+#pragma unroll
+    for (int k = 0; k < QUADS; ++k) {
+        const int i = (lane + 32 * k) * 4;
+        keep[k] = zv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < gw) {
+            keep[k] = *reinterpret_cast<const float4*>(y + (size_t)r * width + c0 + i);
+            zv[k] = Quad<T>::load(z + (size_t)r * z_stride + c0 + i);
+            for (int p = 1; p < parts; ++p) {
+                const float4 more = *reinterpret_cast<const float4*>(y + ((size_t)p * rows + r) * width + c0 + i);
+                keep[k].x += more.x, keep[k].y += more.y, keep[k].z += more.z, keep[k].w += more.w;
+            }
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < QUADS; ++k) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float& v = (&keep[k].x)[e];
+            const float g = (&zv[k].x)[e];
+            v *= g / (1.0f + expf(-g));
+            ss += v * v;
+        }
+    }
+    const float rstd = 1.0f / sqrtf(warp_sum(ss) / (float)gw + eps);
+#pragma unroll
+    for (int k = 0; k < QUADS; ++k) {
+        const int i = (lane + 32 * k) * 4;
+        if (i < gw) {
+            const float4 wv = *reinterpret_cast<const float4*>(w + c0 + i);
+            Quad<T>::store(out + (size_t)r * width + c0 + i,
+                           make_float4(keep[k].x * rstd * wv.x, keep[k].y * rstd * wv.y, keep[k].z * rstd * wv.z,
+                                       keep[k].w * rstd * wv.w));
+        }
+    }
+}
+
 // y: float32 [parts, rows, width], the parts to be added up; z: [rows, width] (type dtype) rows `z_stride` apart; w: float32 [width];
 // out: [rows, width] (type dtype).
 TK_API int tk_gated_group_norm(const float* y, int parts, const void* z, int64_t z_stride, const float* w, float eps, void* out,
@@ -394,6 +443,23 @@ TK_API int tk_gated_group_norm(const float* y, int parts, const void* z, int64_t
     const int gw = width / groups;
     const int warps = rows * groups;
     dim3 grid((warps + 3) / 4), block(128);
+    const size_t es = dtype == TK_F32 ? 4 : 2;
+    if (gw % 4 == 0 && gw <= 32 * 16 && z_stride % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)w % 16 == 0 &&
+        (uintptr_t)z % (4 * es) == 0 && (uintptr_t)out % (4 * es) == 0 && (dtype == TK_F32 || dtype == TK_BF16)) {
+#define TK_GGQ(TT, QUADS)                                                                                               \
+    tk_launch(gated_group_norm_quad_kernel<TT, QUADS>, grid, block, 0, stream, y, parts, (const TT*)z, z_stride, w, eps, \
+              (TT*)out, rows, width, groups)
+        if (dtype == TK_F32) {
+            if (gw <= 128) TK_GGQ(float, 1);
+            else TK_GGQ(float, 4);
+        } else {
+            if (gw <= 128) TK_GGQ(__nv_bfloat16, 1);
+            else TK_GGQ(__nv_bfloat16, 4);
+        }
+#undef TK_GGQ
+        TK_CHECK_LAUNCH("gated_group_norm_quad");
+        return 0;
+    }
 #define TK_GGN(TT)                                                                                               \
     do {                                                                                                         \
         if (gw <= 32 * 4)                                                                                        \

@@ -1351,13 +1351,14 @@ SEQ_CONV_MAX_TAPS = 8
 _SEQ_CONV_RESIDENT = 148 * 4      # blocks of the sequence convolution that run at once
 
 
-def seq_conv_tile(base: int, tokens: int, channels: int) -> int:
+def seq_conv_tile(base: int, tokens: int, channels: int, quad: bool = False) -> int:
     """The tile length for ``seq_conv`` on a step of ``tokens`` tokens: ``base``, doubled (up to 128)
     while the tiles of all channel blocks would not run at once. A thread walks its tile in order,
-    so short tiles are quick, but a second wave of blocks costs more than a longer walk."""
+    so short tiles are quick, but a second wave of blocks costs more than a longer walk. ``quad``: for bfloat16 rows that
+    the four-channel form takes (blocks of 512 channels in 128 threads, ten an SM)."""
     tile = max(int(base), 1)
-    blocks = -(-int(channels) // 256)
-    while tile < 128 and -(-int(tokens) // tile) * blocks > _SEQ_CONV_RESIDENT:
+    blocks, resident = (-(-int(channels) // 512), 148 * 10) if quad else (-(-int(channels) // 256), _SEQ_CONV_RESIDENT)
+    while tile < 128 and -(-int(tokens) // tile) * blocks > resident:
         tile *= 2
     return tile
 

@@ -92,7 +92,7 @@ class GatedDelta:
         proj = self.in_proj(x)
         z = self.gate_proj(x, out_dtype=torch.float32)
         u = ops.seq_conv(proj[:, :C], self.taps, None, ctx.states.get((call, "conv")), ctx.cu_seqlens, ctx.seq_ctx,
-                         ctx.seq_slot, ctx.tiles(ops.seq_conv_tile(self.tile, T, C)), proj.dtype, act=True)
+                         ctx.seq_slot, ctx.tiles(ops.seq_conv_tile(self.tile, T, C, proj.dtype == torch.bfloat16)), proj.dtype, act=True)
         if self.decay == "channel":
             n = C + self.decay_up.in_features
             decay = self.decay_up(proj[:, C:n], out_dtype=torch.float32)

@@ -72,7 +72,8 @@ class StateSpaceDuality:
         dt = self.dt_proj(x, out_dtype=torch.float32)
         xbc = ops.seq_conv(proj[:, self.inner:], self.conv, self.conv_bias, ctx.states.get((call, "conv")),
                            ctx.cu_seqlens, ctx.seq_ctx, ctx.seq_slot,
-                           ctx.tiles(ops.seq_conv_tile(self.tile, T, self.channels)), proj.dtype, act=True)
+                           ctx.tiles(ops.seq_conv_tile(self.tile, T, self.channels, proj.dtype == torch.bfloat16)),
+                           proj.dtype, act=True)
         y = ops.ssd_scan(xbc, dt, self.dt_bias, self.a_log, self.d_skip, ctx.states[(call, "S")], ctx.cu_seqlens,
                          ctx.seq_ctx, ctx.seq_slot, ctx.n_seqs, self.heads, self.v_dim, self.state, self.groups,
                          self.sm_count)
