@@ -1068,6 +1068,27 @@ def test_gemm_skinny(m, n, k, out_dtype):
     close(got, wide[:, 8:8 + k].double() @ w.double().T, out_dtype, "skinny strided")
 
 
+@pytest.mark.parametrize("m", [1, 5, 8])
+@pytest.mark.parametrize("n, k", [(7120, 1032), (9504, 2048), (7136, 1992)])
+def test_gemm_skinny_tall_matrices(m, n, k):
+    """Tall matrices of one to two thousand columns, whose blocks a CTA takes one after the other: a last round and a last block
+    that are not full, slices of K that end inside a warp's second one; with a bias and 32-bit rows, the activation and the
+    norm of the stream in front."""
+    from tokenomos_b200 import ops
+    x, w, b = torch.randn(m, k).to(torch.bfloat16), (torch.randn(n, k) * k ** -0.5).to(torch.bfloat16), torch.randn(n)
+    want = x.double() @ w.double().T
+    got = ops.gemm_skinny(dev(x), dev(w), dev(b), torch.float32).double().cpu()
+    assert (got - want - b.double()).norm() <= 1e-6 * want.norm()
+    view, rows = dev(x)[:, 8:], dev(w)[:-3, 8:]
+    close(ops.gemm_skinny(view, rows, None), x[:, 8:].double() @ w[:-3, 8:].double().T, torch.bfloat16, "tall skinny, strided")
+    rstd = 1.0 / torch.sqrt(x.double().pow(2).mean(1, keepdim=True) + 1e-5)
+    close(ops.gemm_skinny(dev(x), dev(w), None, norm_eps=1e-5), want * rstd, torch.bfloat16, "tall skinny with the norm")
+    runs = want.view(m, n // 16, 2, 8)
+    for scale, eps in ((torch.ones(m, 1, 1).double(), 0.0), (rstd[:, :, None], 1e-5)):
+        act = (torch.nn.functional.silu(runs[:, :, 0] * scale) * runs[:, :, 1] * scale).reshape(m, n // 2)
+        close(ops.gemm_skinny(dev(x), dev(w), None, swiglu=True, norm_eps=eps), act, torch.bfloat16, "tall skinny swiglu")
+
+
 def test_gemm_skinny_refuses_what_it_cannot_take():
     from tokenomos_b200 import ops
     x = torch.zeros(17, 64, dtype=torch.bfloat16, device="cuda")

@@ -92,6 +92,129 @@ __device__ __forceinline__ float sum_squares(const uint4& v) {
     return acc;
 }
 
+// From the warps' partial sums red[warp][row][token] of the weight rows n0 .. n0 + cta_rows - 1 (block `block` of them) to the
+// result. `pf`, `pf_res_ok`: what this thread needs of the conv state or the residual was asked for ahead.
+template <int MT, typename TO, int EPI, bool NORM, bool ADD>
+__device__ __forceinline__ void skinny_epilogue(const float* red, int warps, const float* rstd_s, int block, int n0, int cta_rows,
+                                                const float* __restrict__ bias, TO* out, int64_t ldo, int M, int N,
+                                                const ConvTail& tail, const Fuse& fuse, bool pf, int pf_ctx,
+                                                const float (&pf_state)[3], bool pf_res_ok, float pf_res) {
+    constexpr bool SWIGLU = EPI == EPI_SWIGLU, CONV = EPI == EPI_CONV;
+    constexpr int RED_ROWS = CONV ? 24 : ROWS;
+    if constexpr (CONV) {
+        // one thread per (token, channel): B, C, X of the channel as the unfused path stores them,
+        // u = B X, the taps over the state row and u, the state moved on by one
+        const int W = tail.W, d = tail.d;
+        for (int idx = threadIdx.x; idx < 8 * MT; idx += blockDim.x) {
+            const int tok = idx / 8, j = idx % 8;
+            const int c = block * 8 + j;
+            if (tok >= M || c >= d) continue;
+            float bv = 0.f, cv = 0.f, xv = 0.f;
+            for (int wv = 0; wv < warps; ++wv) {
+                const float* src = red + (size_t)wv * RED_ROWS * MT + tok;
+                bv += src[j * MT];
+                cv += src[(j + 8) * MT];
+                xv += src[(j + 16) * MT];
+            }
+            if constexpr (NORM) {
+                const float rs = rstd_s[tok];
+                bv *= rs;
+                cv *= rs;
+                xv *= rs;
+            }
+            if (bias != nullptr) {
+                bv += bias[n0 + j];
+                cv += bias[n0 + 8 + j];
+                xv += bias[n0 + 16 + j];
+            }
+            bv = round_as<TO>(bv);
+            cv = round_as<TO>(cv);
+            xv = round_as<TO>(xv);
+            const float u = round_as<TO>(bv * xv);
+            const bool have = pf && idx == (int)threadIdx.x;          // fetched at the start
+            const int ctx = have ? pf_ctx : tail.seq_ctx[tok];
+            __nv_bfloat16* st = tail.state + (size_t)TK_SLOT(TK_K_SKINNY_CONV, tail.seq_slot[tok]) * (W - 1) * d + c;
+            const float* taps = tail.taps + (size_t)c * W;
+            // state row k holds u of position ctx - (W - 1) + k; before position 0 it reads as 0
+            float acc_c = 0.f;
+            if (have) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    if (k < W - 1) {
+                        const float hv = ctx - (W - 1) + k < 0 ? 0.f : pf_state[k];
+                        acc_c += hv * taps[k];
+                        if (k > 0) st[(size_t)(k - 1) * d] = __float2bfloat16_rn(hv);
+                    }
+                }
+            } else {
+                for (int k = 0; k < W - 1; ++k) {
+                    const float hv = ctx - (W - 1) + k < 0 ? 0.f : __bfloat162float(st[(size_t)k * d]);
+                    acc_c += hv * taps[k];
+                    // row k - 1 takes what row k held (it was read in the pass before this one)
+                    if (k > 0) st[(size_t)(k - 1) * d] = __float2bfloat16_rn(hv);
+                }
+            }
+            st[(size_t)(W - 2) * d] = __float2bfloat16_rn(u);
+            acc_c += u * taps[W - 1];
+            if (tail.bias != nullptr) acc_c += tail.bias[c];
+            const float y = round_as<TO>(acc_c);
+            out[(size_t)tok * ldo + c] = from_f<TO>(cv * y);
+        }
+    } else if constexpr (SWIGLU) {
+        for (int idx = threadIdx.x; idx < 8 * MT; idx += blockDim.x) {
+            const int tok = idx / 8, j = idx % 8;
+            if (tok >= M || n0 + 8 + j >= N) continue;
+            float gate = 0.f, up = 0.f;
+            for (int wv = 0; wv < warps; ++wv) {
+                gate += red[(size_t)wv * ROWS * MT + j * MT + tok];
+                up += red[(size_t)wv * ROWS * MT + (j + 8) * MT + tok];
+            }
+            if constexpr (NORM) {
+                gate *= rstd_s[tok];
+                up *= rstd_s[tok];
+            }
+            if (bias != nullptr) {
+                gate += bias[n0 + j];
+                up += bias[n0 + 8 + j];
+            }
+            if (fuse.glu == 2) {
+                out[(size_t)tok * ldo + n0 / 2 + j] = from_f<TO>(gelu_tanh_as<TO>(gate) * up);
+                continue;
+            }
+            if (fuse.glu) {
+                if (fuse.glu_limit > 0.f) {
+                    gate = fminf(gate, fuse.glu_limit);
+                    up = fminf(fmaxf(up, -fuse.glu_limit), fuse.glu_limit);
+                }
+                out[(size_t)tok * ldo + n0 / 2 + j] =
+                    from_f<TO>(gate / (1.0f + __expf(-fuse.glu_alpha * gate)) * (up + fuse.glu_shift));
+                continue;
+            }
+            // the unfused path stores gate and up in the output type, then rounds silu(gate)
+            gate = round_as<TO>(gate);
+            up = round_as<TO>(up);
+            const float act = silu_as<TO>(gate);
+            out[(size_t)tok * ldo + n0 / 2 + j] = from_f<TO>(act * up);
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < cta_rows * MT; idx += blockDim.x) {
+            const int tok = idx / cta_rows, r = idx % cta_rows;   // rows fastest: neighbours in memory
+            if (tok >= M || n0 + r >= N) continue;
+            float v = 0.f;
+            for (int wv = 0; wv < warps; ++wv) v += red[(size_t)wv * ROWS * MT + r * MT + tok];
+            if constexpr (NORM) v *= rstd_s[tok];
+            if (bias != nullptr) v += bias[n0 + r];
+            if constexpr (ADD) {
+                const float res = (pf_res_ok && idx == (int)threadIdx.x)
+                                      ? pf_res
+                                      : __bfloat162float(fuse.residual[(size_t)tok * fuse.ldr + n0 + r]);
+                v = res + round_as<TO>(v);
+            }
+            out[(size_t)tok * ldo + n0 + r] = from_f<TO>(v);
+        }
+    }
+}
+
 // MT: 8 or 16 tokens (one or two n8 tiles). R8: the CTA owns 8 weight rows instead of 16 (the
 // upper half of the mma tile stays zero): twice as many CTAs for matrices with few rows.
 // EPI_SWIGLU: the weight rows come in blocks of 16, 8 gate rows then the 8 up rows of the same
@@ -108,7 +231,7 @@ gemm_skinny_kernel(const __nv_bfloat16* x, int64_t ldx,
                    TO* out, int64_t ldo, int M, int N, int K, ConvTail tail, Fuse fuse) {
     extern __shared__ float red[];                 // [warps][RED_ROWS][MT], NORM: + [warps][MT] + [MT]
     pdl_launch_dependents();
-    constexpr bool SWIGLU = EPI == EPI_SWIGLU, CONV = EPI == EPI_CONV;
+    constexpr bool CONV = EPI == EPI_CONV;
     constexpr int RED_ROWS = CONV ? 24 : ROWS;
     const int warps = blockDim.x >> 5;
     float* ssq_s = red + (size_t)warps * RED_ROWS * MT;      // NORM: each warp's sums of squares
@@ -251,118 +374,143 @@ gemm_skinny_kernel(const __nv_bfloat16* x, int64_t ldx,
         }
         __syncthreads();
     }
-    if constexpr (CONV) {
-        // one thread per (token, channel): B, C, X of the channel as the unfused path stores them,
-        // u = B X, the taps over the state row and u, the state moved on by one
-        const int W = tail.W, d = tail.d;
-        for (int idx = threadIdx.x; idx < 8 * MT; idx += blockDim.x) {
-            const int tok = idx / 8, j = idx % 8;
-            const int c = blockIdx.x * 8 + j;
-            if (tok >= M || c >= d) continue;
-            float bv = 0.f, cv = 0.f, xv = 0.f;
-            for (int wv = 0; wv < warps; ++wv) {
-                const float* src = red + (size_t)wv * RED_ROWS * MT + tok;
-                bv += src[j * MT];
-                cv += src[(j + 8) * MT];
-                xv += src[(j + 16) * MT];
-            }
-            if constexpr (NORM) {
-                const float rs = rstd_s[tok];
-                bv *= rs;
-                cv *= rs;
-                xv *= rs;
-            }
-            if (bias != nullptr) {
-                bv += bias[n0 + j];
-                cv += bias[n0 + 8 + j];
-                xv += bias[n0 + 16 + j];
-            }
-            bv = round_as<TO>(bv);
-            cv = round_as<TO>(cv);
-            xv = round_as<TO>(xv);
-            const float u = round_as<TO>(bv * xv);
-            const bool have = pf && idx == (int)threadIdx.x;          // fetched at the start
-            const int ctx = have ? pf_ctx : tail.seq_ctx[tok];
-            __nv_bfloat16* st = tail.state + (size_t)TK_SLOT(TK_K_SKINNY_CONV, tail.seq_slot[tok]) * (W - 1) * d + c;
-            const float* taps = tail.taps + (size_t)c * W;
-            // state row k holds u of position ctx - (W - 1) + k; before position 0 it reads as 0
-            float acc_c = 0.f;
-            if (have) {
+    skinny_epilogue<MT, TO, EPI, NORM, ADD>(red, warps, rstd_s, blockIdx.x, n0, CTA_ROWS, bias, out, ldo, M, N, tail, fuse, pf, pf_ctx,
+                                            pf_state, pf_res_ok, pf_res);
+}
+
+
+// The same products for at most 8 tokens and tall matrices as one stream of weights an SM: a CTA of 16 warps takes blocks of 16
+// weight rows, one after the other, and every thread asks for its 16-byte shares of them RING_DEPTH slices of K ahead by
+// cp.async into shared memory of its own (no other thread reads them: waiting for its own copies is all the synchronisation
+// they need), across the ends of blocks. The form above asks for two slices a warp, adds up, and begins again with the next
+// CTA: 1,024 blocks ran in 2.3 waves of CTAs, each with its own ramp, where a seventh round of 148 is nearly full. What a
+// thread needs of x, two slices of K at most, stays in its registers for all blocks. Measured in a chain of itself, 8 rows:
+// 16,384 x 2,048 with norm and SwiGLU 11.5 us (5.8 TB/s), the form above 14.7; 21,504 x 2,048 14.9 and 19.7; the head of
+// 65,536 x 2,048 41.2 and 43.1. With one slice a warp (K up to 1,024) a barrier every 32 KB undoes it (9,216 x 1,024: 5.3
+// against 4.9), and so does reading x again for every slice beyond 2,048 (2,048 x 8,192: 9.8 against 8.3).
+constexpr int RING_WARPS = 16, RING_THREADS = 32 * RING_WARPS, RING_DEPTH = 3, RING_SX = 2;
+
+__device__ __forceinline__ void ring_copy(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+template <typename TO, int EPI, bool NORM>
+__global__ void __launch_bounds__(RING_THREADS)
+gemm_skinny_ring_kernel(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* __restrict__ w, int64_t ldw,
+                        const float* __restrict__ bias, TO* out, int64_t ldo, int M, int N, int K, int n_blocks, Fuse fuse) {
+    constexpr int MT = 8, PARTS = 4;              // PARTS: 16-byte loads of a thread and slice
+    extern __shared__ __align__(16) unsigned char ring_smem[];
+    float* red = reinterpret_cast<float*>(ring_smem + (size_t)RING_DEPTH * PARTS * RING_THREADS * 16);      // [2][warps][ROWS][MT]
+    float* ssq_s = red + 2 * RING_WARPS * ROWS * MT;
+    float* rstd_s = ssq_s + RING_WARPS * MT;
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int total = (n_blocks - blockIdx.x + gridDim.x - 1) / gridDim.x * RING_SX;
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(ring_smem) + threadIdx.x * 16;
+    int in_block = blockIdx.x, in_e = 0, in_slot = 0, asked = 0;                  // the copies' place
+    auto ask = [&]() {
+        if (asked < total) {
+            const int n0 = in_block * ROWS;
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    if (k < W - 1) {
-                        const float hv = ctx - (W - 1) + k < 0 ? 0.f : pf_state[k];
-                        acc_c += hv * taps[k];
-                        if (k > 0) st[(size_t)(k - 1) * d] = __float2bfloat16_rn(hv);
-                    }
-                }
-            } else {
-                for (int k = 0; k < W - 1; ++k) {
-                    const float hv = ctx - (W - 1) + k < 0 ? 0.f : __bfloat162float(st[(size_t)k * d]);
-                    acc_c += hv * taps[k];
-                    // row k - 1 takes what row k held (it was read in the pass before this one)
-                    if (k > 0) st[(size_t)(k - 1) * d] = __float2bfloat16_rn(hv);
-                }
+            for (int part = 0; part < PARTS; ++part) {
+                const int r = n0 + g + (part >> 1) * 8, k = (warp + in_e * RING_WARPS) * KSLICE + (part & 1) * 32 + 8 * t;
+                const bool ok = k < K && r < N;
+                ring_copy(mine + (uint32_t)((in_slot * PARTS + part) * RING_THREADS * 16), ok ? w + (size_t)r * ldw + k : w, ok);
             }
-            st[(size_t)(W - 2) * d] = __float2bfloat16_rn(u);
-            acc_c += u * taps[W - 1];
-            if (tail.bias != nullptr) acc_c += tail.bias[c];
-            const float y = round_as<TO>(acc_c);
-            out[(size_t)tok * ldo + c] = from_f<TO>(cv * y);
+            if (++in_e == RING_SX) in_e = 0, in_block += gridDim.x;
+            if (++in_slot == RING_DEPTH) in_slot = 0;
+            ++asked;
         }
-    } else if constexpr (SWIGLU) {
-        for (int idx = threadIdx.x; idx < 8 * MT; idx += blockDim.x) {
-            const int tok = idx / 8, j = idx % 8;
-            if (tok >= M || n0 + 8 + j >= N) continue;
-            float gate = 0.f, up = 0.f;
-            for (int wv = 0; wv < warps; ++wv) {
-                gate += red[(size_t)wv * ROWS * MT + j * MT + tok];
-                up += red[(size_t)wv * ROWS * MT + (j + 8) * MT + tok];
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < RING_DEPTH; ++i) ask();   // weights are no kernel's output: they stream while the kernel before finishes
+    pdl_wait();
+    uint4 xs[RING_SX][2];
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < RING_SX; ++e)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = (warp + e * RING_WARPS) * KSLICE + h * 32 + 8 * t;
+            xs[e][h] = g < M && k < K ? ld_activation(x + (size_t)g * ldx + k) : make_uint4(0u, 0u, 0u, 0u);
+            if constexpr (NORM) ss += sum_squares(xs[e][h]);
+        }
+    const float no_state[3] = {0.f, 0.f, 0.f};
+    int slot = 0, buf = 0;
+    for (int block = blockIdx.x; block < n_blocks; block += gridDim.x) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < RING_SX; ++e) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(RING_DEPTH - 1) : "memory");
+            uint4 v[PARTS];
+#pragma unroll
+            for (int part = 0; part < PARTS; ++part)
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(v[part].x), "=r"(v[part].y), "=r"(v[part].z), "=r"(v[part].w)
+                             : "r"(mine + (uint32_t)((slot * PARTS + part) * RING_THREADS * 16))
+                             : "memory");
+            if (++slot == RING_DEPTH) slot = 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                // elements 0..3 of the 16 bytes are one mma step, 4..7 the next
+                mma16816(acc, v[h].x, v[2 + h].x, v[h].y, v[2 + h].y, xs[e][h].x, xs[e][h].y);
+                mma16816(acc, v[h].z, v[2 + h].z, v[h].w, v[2 + h].w, xs[e][h].z, xs[e][h].w);
             }
-            if constexpr (NORM) {
-                gate *= rstd_s[tok];
-                up *= rstd_s[tok];
+            ask();
+        }
+        // acc: rows g / g + 8, tokens 2 t, + 1
+        float* part_s = red + (size_t)buf * RING_WARPS * ROWS * MT;
+        float* dst = part_s + (size_t)warp * ROWS * MT;
+        *reinterpret_cast<float2*>(dst + g * MT + 2 * t) = make_float2(acc[0], acc[1]);
+        *reinterpret_cast<float2*>(dst + (g + 8) * MT + 2 * t) = make_float2(acc[2], acc[3]);
+        const bool first = block == (int)blockIdx.x;
+        if constexpr (NORM) {
+            if (first) {
+                // lanes t = 0..3 of a quad hold parts of token g's sum; the CTA's warps cover all of K
+                float v = ss;
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if (t == 0) ssq_s[warp * MT + g] = v;
             }
-            if (bias != nullptr) {
-                gate += bias[n0 + j];
-                up += bias[n0 + 8 + j];
-            }
-            if (fuse.glu == 2) {
-                out[(size_t)tok * ldo + n0 / 2 + j] = from_f<TO>(gelu_tanh_as<TO>(gate) * up);
-                continue;
-            }
-            if (fuse.glu) {
-                if (fuse.glu_limit > 0.f) {
-                    gate = fminf(gate, fuse.glu_limit);
-                    up = fminf(fmaxf(up, -fuse.glu_limit), fuse.glu_limit);
+        }
+        __syncthreads();          // (the other buffer of partial sums is written next: one barrier a block is enough)
+        if constexpr (NORM) {
+            if (first) {
+                if ((int)threadIdx.x < MT) {
+                    float v = 0.f;
+                    for (int wv = 0; wv < RING_WARPS; ++wv) v += ssq_s[wv * MT + threadIdx.x];
+                    rstd_s[threadIdx.x] = rsqrtf(v / (float)K + fuse.eps);
                 }
-                out[(size_t)tok * ldo + n0 / 2 + j] =
-                    from_f<TO>(gate / (1.0f + __expf(-fuse.glu_alpha * gate)) * (up + fuse.glu_shift));
-                continue;
+                __syncthreads();
             }
-            // the unfused path stores gate and up in the output type, then rounds silu(gate)
-            gate = round_as<TO>(gate);
-            up = round_as<TO>(up);
-            const float act = silu_as<TO>(gate);
-            out[(size_t)tok * ldo + n0 / 2 + j] = from_f<TO>(act * up);
         }
-    } else {
-        for (int idx = threadIdx.x; idx < CTA_ROWS * MT; idx += blockDim.x) {
-            const int tok = idx / CTA_ROWS, r = idx % CTA_ROWS;   // rows fastest: neighbours in memory
-            if (tok >= M || n0 + r >= N) continue;
-            float v = 0.f;
-            for (int wv = 0; wv < warps; ++wv) v += red[(size_t)wv * ROWS * MT + r * MT + tok];
-            if constexpr (NORM) v *= rstd_s[tok];
-            if (bias != nullptr) v += bias[n0 + r];
-            if constexpr (ADD) {
-                const float res = (pf_res_ok && idx == (int)threadIdx.x)
-                                      ? pf_res
-                                      : __bfloat162float(fuse.residual[(size_t)tok * fuse.ldr + n0 + r]);
-                v = res + round_as<TO>(v);
-            }
-            out[(size_t)tok * ldo + n0 + r] = from_f<TO>(v);
-        }
+        skinny_epilogue<MT, TO, EPI, NORM, false>(part_s, RING_WARPS, rstd_s, block, block * ROWS, ROWS, bias, out, ldo, M, N,
+                                                  ConvTail{}, fuse, false, 0, no_state, false, 0.f);
+        buf ^= 1;
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Three rounds of blocks at least, two slices of K a warp.
+bool ring_takes(int N, int K) {
+    return N > 3 * 148 * ROWS && K > RING_WARPS * KSLICE && K <= RING_SX * RING_WARPS * KSLICE;
+}
+
+template <typename TO, int EPI, bool NORM>
+cudaError_t launch_ring(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* w, int64_t ldw, const float* bias, TO* out,
+                        int64_t ldo, int M, int N, int K, const Fuse& fuse, cudaStream_t stream) {
+    auto kernel = gemm_skinny_ring_kernel<TO, EPI, NORM>;
+    const int smem = RING_DEPTH * 4 * RING_THREADS * 16 + (2 * RING_WARPS * ROWS + RING_WARPS + 1) * 8 * 4;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // One CTA an SM, and the split between shared memory and L1 that the decode attention asks for: an SM changes its split
+    // only when it is empty, so a kernel that asks for another one starts behind its neighbours instead of under them (a
+    // decode step of 8 rows: 326 us; with all of the SM as shared memory, two CTAs or one, 405 and 462; 350 without this kernel)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 62);
+    if (e != cudaSuccess) return e;
+    const int n_blocks = (N + ROWS - 1) / ROWS;
+    return tk_launch(kernel, dim3(n_blocks < 148 ? n_blocks : 148), dim3(RING_THREADS), smem, stream, x, ldx, w, ldw, bias, out, ldo,
+                     M, N, K, n_blocks, fuse);
 }
 
 }  // namespace
@@ -413,6 +561,25 @@ static int skinny_launch(const void* x, int64_t ldx, const void* w, int64_t ldw,
     auto x_ = (const __nv_bfloat16*)x;
     auto w_ = (const __nv_bfloat16*)w;
     const Fuse fuse{norm_eps, (const __nv_bfloat16*)residual, ldr, glu, glu_limit, glu_alpha, glu_shift};
+    if (M <= 8 && !add && ring_takes(N, K)) {
+        cudaError_t e = cudaSuccess;
+#define TK_RING_AS(TO_, EPI_, NORM_) \
+    e = launch_ring<TO_, EPI_, NORM_>(x_, ldx, w_, ldw, bias, (TO_*)out, ldo, M, N, K, fuse, stream)
+        if (norm && swiglu) TK_RING_AS(__nv_bfloat16, EPI_SWIGLU, true);
+        else if (norm) TK_RING_AS(__nv_bfloat16, EPI_NONE, true);
+        else if (out_dtype == TK_BF16 && swiglu) TK_RING_AS(__nv_bfloat16, EPI_SWIGLU, false);
+        else if (out_dtype == TK_BF16) TK_RING_AS(__nv_bfloat16, EPI_NONE, false);
+        else if (out_dtype == TK_F32 && swiglu) TK_RING_AS(float, EPI_SWIGLU, false);
+        else if (out_dtype == TK_F32) TK_RING_AS(float, EPI_NONE, false);
+        else TK_CHECK_ARG(false, "gemm_skinny: output dtype %d", out_dtype);
+#undef TK_RING_AS
+        if (e != cudaSuccess) {
+            tk_set_error("gemm_skinny: launch failed: %s", cudaGetErrorString(e));
+            cudaGetLastError();
+            return -2;
+        }
+        return 0;
+    }
 #define TK_SKINNY_F(MT_, TO_, R8_, SW_, NORM_, ADD_)                                               \
     do {                                                                                           \
         if (unroll == 2)                                                                           \
