@@ -887,3 +887,59 @@ def test_trace_program_and_command_line(folders, tmp_path):
     lines = [json.loads(ln) for ln in proc.stdout.splitlines() if ln.startswith("{")]
     assert len(lines) == 1 and len(lines[0]["token_ids"]) == 5
     teacher_forced_ok(CASES[name]["config"], folders[name][1], [1, 2, 3, 4], lines[0]["token_ids"], 1e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H, K, D, V, lens, ctx", [(4, 2, 128, 128, (300, 1, 33, 16, 177), (0, 5, 9, 0, 3)), (2, 1, 64, 40, (121,), (7,)),
+                                                   (2, 2, 200, 24, (0, 96, 0, 130), (0, 0, 0, 2)), (3, 3, 24, 24, (47, 18), (0, 4))])
+def test_delta_rule_two_tokens_a_step(H, K, D, V, lens, ctx, dtype):
+    """The delta rule with a decay per head over portions that begin on odd rows and end inside a stage of 16 tokens and on its
+    edge, at every register form of a column: against the recurrence in 64-bit from the same rows, decays from 1 to e^-40 a
+    token among them, sums of up to 200 products in 32-bit; a token that is not finite reaches none before it."""
+    from tokenomos_b200 import ops
+    g = torch.Generator().manual_seed(7)
+    T, S = sum(lens), len(lens)
+    nk, nv = K * D, H * V
+    u = torch.randn(T, 2 * nk + nv + 4, generator=g).to(getattr(torch, dtype))
+    zb, za = torch.randn(T, H + 4, generator=g), torch.randn(T, H + 4, generator=g) - 1.0
+    za[::19] += 6.0
+    A, bias = torch.rand(H, generator=g) * 3, torch.randn(H, generator=g)
+    state = torch.randn(S + 1, H, V, D, generator=g) * 0.3
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    slots = list(range(S, 0, -1))
+
+    def run(rows, st):
+        return ops.linmem_scan(rows, (0, nk, 2 * nk), "delta", "head", A.cuda(), st, i32(cu), i32(list(ctx)), i32(slots), S, H, K,
+                               D, V, D ** -0.5, unit=True, beta=zb.cuda(), gates=za.cuda(), bias=bias.cuda())
+
+    st, rows = state.cuda(), u.cuda()
+    got = run(rows, st)
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+    q = (unit(u[:, :nk].double().view(T, K, D)) * D ** -0.5).repeat_interleave(H // K, 1)
+    k = unit(u[:, nk:2 * nk].double().view(T, K, D)).repeat_interleave(H // K, 1)
+    v = u[:, 2 * nk:2 * nk + nv].double().view(T, H, V)
+    beta = torch.sigmoid(zb[:, :H].double())
+    decay = torch.exp(-A.double() * torch.nn.functional.softplus(za[:, :H].double() + bias.double()))
+    want, after = torch.empty(T, H, V, dtype=torch.float64), state.double()
+    for s in range(S):
+        M = after[slots[s]] if ctx[s] else torch.zeros(H, V, D, dtype=torch.float64)          # [head, value, key]
+        for t in range(cu[s], cu[s + 1]):
+            M = decay[t, :, None, None] * M
+            w = beta[t, :, None] * (v[t] - torch.einsum("hvk,hk->hv", M, k[t]))
+            M = M + w[:, :, None] * k[t][:, None, :]
+            want[t] = torch.einsum("hvk,hk->hv", M, q[t])
+        if lens[s]:
+            after[slots[s]] = M
+    err = (got.double().cpu().view(T, H, V) - want).norm() / want.norm()
+    print(f"pairs {dtype} {D}x{V}: {err:.2e}")
+    assert err <= 1e-6, err
+    assert (st.double().cpu() - after).norm() <= 1e-6 * after.norm()
+    last = max(range(S), key=lambda s: lens[s])
+    t = cu[last] + lens[last] // 2 + 1 - lens[last] // 2 % 2             # the second token of a pair
+    rows[t, nk] = float("nan")
+    again = run(rows, state.cuda())
+    assert torch.equal(again[:t], got[:t]) and torch.isnan(again[t]).any()

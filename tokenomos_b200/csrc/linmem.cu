@@ -36,6 +36,16 @@ constexpr int LM_SEG = 256;      // tokens of a segment (whole stages)
 
 enum : int { LM_ADD = 0, LM_DELTA = 1 };
 enum : int { LM_FIXED = 0, LM_HEAD = 1, LM_CHANNEL = 2 };
+// Whether the walk may take two tokens a step (lm_pair), and whether it does: up to eight sequences of keys up to 64, where the
+// path from token to token bounds it (16 heads of 64 x 64, one sequence of 2,048 tokens: 282 us, 353 token by token; more
+// sequences hide the path from each other, 16 of 128: 64 us against 62). Keys up to 128 are bound by the multiply-adds of a
+// block (16 heads of 128 x 128: 406 and 410), until one column a thread spreads them over twice the SMs: while those blocks
+// are no more than the SMs (one sequence of 2,048 tokens 319 us; two of 1,024 243 against 219).
+constexpr bool LM_PAIRS(int rule, int decay) { return rule == LM_DELTA && decay == LM_HEAD; }
+inline bool lm_pairs(int decay, int n_seqs, int H, int D, int V, int sm_count) {
+    if (decay != LM_HEAD || D > 128) return false;
+    return D <= 64 ? n_seqs <= 8 : (V + 15) / 16 * H * n_seqs <= sm_count;
+}
 
 struct LinMem {
     const void* qkv;
@@ -161,6 +171,52 @@ __device__ __forceinline__ float lm_step(float2 (&S)[R / 2], const float* k, con
     return fmaf(kq, u, DECAY == LM_CHANNEL ? o : a * o);
 }
 
+// Two tokens of the delta rule with a decay per head for CPT columns: what both read of the state is formed from the state before
+// the first, so that the sums over the rows of both, and the exchange between lanes that follows, run side by side and the
+// path from pair to pair is as long as that from token to token:
+//     u_1 = beta_1 (v_1 - a_1 S.k_1)            u_2 = beta_2 (v_2 - a_2 (a_1 S.k_2 + (k_1.k_2) u_1))
+//     o_1 = a_1 S.q_1 + (k_1.q_1) u_1           o_2 = a_2 (a_1 S.q_2 + (k_1.q_2) u_1) + (k_2.q_2) u_2
+//     S <- a_2 a_1 S + a_2 u_1 k_1 + u_2 k_2
+// kq: this lane's first row of token 1's k, with its q, token 2's k and q each DP further; c1, c2: (a, beta, k . q, -);
+// near: token 2's products with k_1.
+template <int R, int CPT>
+__device__ __forceinline__ void lm_pair(float2 (&S)[CPT][R / 2], const float* kq, const float (&v1)[CPT], const float (&v2)[CPT],
+                                        const float4& c1, const float4& c2, const float2& near, float (&o1)[CPT], float (&o2)[CPT]) {
+    constexpr int DP = 8 * R;
+    float2 k1[R / 2], k2[R / 2], s[CPT][4];
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[c][e] = two(0.f);
+#pragma unroll
+    for (int i = 0; i < R / 4; ++i) {
+        const float4 ka = *reinterpret_cast<const float4*>(kq + 32 * i), qa = *reinterpret_cast<const float4*>(kq + DP + 32 * i);
+        const float4 kb = *reinterpret_cast<const float4*>(kq + 2 * DP + 32 * i), qb = *reinterpret_cast<const float4*>(kq + 3 * DP + 32 * i);
+        k1[2 * i] = make_float2(ka.x, ka.y), k1[2 * i + 1] = make_float2(ka.z, ka.w);
+        k2[2 * i] = make_float2(kb.x, kb.y), k2[2 * i + 1] = make_float2(kb.z, kb.w);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+            const float2 x = S[c][2 * i], y = S[c][2 * i + 1];
+            s[c][0] = fma2(y, k1[2 * i + 1], fma2(x, k1[2 * i], s[c][0]));
+            s[c][1] = fma2(y, k2[2 * i + 1], fma2(x, k2[2 * i], s[c][1]));
+            s[c][2] = fma2(y, make_float2(qa.z, qa.w), fma2(x, make_float2(qa.x, qa.y), s[c][2]));
+            s[c][3] = fma2(y, make_float2(qb.z, qb.w), fma2(x, make_float2(qb.x, qb.y), s[c][3]));
+        }
+    }
+    const float a12 = c1.x * c2.x;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+        const float p1 = sum8(s[c][0].x + s[c][0].y), p2 = sum8(s[c][1].x + s[c][1].y);
+        const float u1 = c1.y * fmaf(-c1.x, p1, v1[c]);
+        const float u2 = c2.y * fmaf(-c2.x, fmaf(c1.x, p2, near.x * u1), v2[c]);
+        const float2 w1 = two(c2.x * u1), w2 = two(u2), a = two(a12);
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) S[c][i] = fma2(k2[i], w2, fma2(k1[i], w1, mul2(a, S[c][i])));
+        o1[c] = fmaf(c1.z, u1, c1.x * sum8(s[c][2].x + s[c][2].y));
+        o2[c] = fmaf(c2.z, u2, c2.x * fmaf(c1.x, sum8(s[c][3].x + s[c][3].y), near.y * u1));
+    }
+}
+
 // A warp stages one token's k and q (silu, rotation, unit length, q_scale), k . q and the decay per channel. A lane holds
 // the elements lane + 32 j.
 template <typename T, int DPL>
@@ -240,11 +296,13 @@ __device__ __forceinline__ void lm_shape(const LinMem& m, int lane, float (&kv)[
 
 // Portions, first kernel: everything a token brings to the walk that does not depend on the state, formed once and laid
 // out as the walk reads it (32-bit, zeros past D and V): kq [K][T'][k | q][DP], decays [H][T'][DP] (per channel),
-// values [H][T'][VP], and per head and token (a, beta, k . q, -). T' = T + LM_TOK rows, so that a stage may read past the
+// values [H][T'][VP], and per head and token (a, beta, k . q, -); for the pairs of the delta rule with a decay per head also, per q/k head
+// and token, (k . k of the token before, q . k of the token before). T' = T + LM_TOK rows, so that a stage may read past the
 // last token. One block per token.
 struct LinMemPrep {
     float *kq, *g, *v;
     float4* sc;
+    float2* near;            // [K][T'] or null
     int rows, VP;            // T', the values' padded size
     float* seg;              // [slots][H][V][D]: what each segment adds to the state, or null: no segments
     int n_seqs;
@@ -298,6 +356,25 @@ linmem_prepare_kernel(const LinMem m, const LinMemPrep p) {
             lm_fetch_partners<T, DPL>(m, t, kh * (m.H / m.K), lane, kp, qp);
             lm_rotate<DPL>(m, lane, cs, kv, qv, kp, qp);
         }
+        if (LM_PAIRS(RULE, DECAY) && p.near != nullptr) {
+            // (the first token of the step has none before it, and no pair reaches across a sequence's start)
+            float kb[DPL], unused[DPL], skb = 0.f, kk = 0.f, qk = 0.f, sk = 0.f, sq = 0.f;
+            lm_fetch<T, DPL>(m, max(t - 1, 0), kh * (m.H / m.K), lane, kb, unused);
+#pragma unroll
+            for (int j = 0; j < DPL; ++j) {
+                const float k0 = m.act ? lm_silu(kv[j]) : kv[j], q0 = m.act ? lm_silu(qv[j]) : qv[j];
+                const float b = m.act ? lm_silu(kb[j]) : kb[j];
+                skb = fmaf(b, b, skb);
+                sk = fmaf(k0, k0, sk);
+                sq = fmaf(q0, q0, sq);
+                kk = fmaf(b, k0, kk);
+                qk = fmaf(b, q0, qk);
+            }
+            skb = warp_sum(skb), sk = warp_sum(sk), sq = warp_sum(sq), kk = warp_sum(kk), qk = warp_sum(qk);
+            const float mb = m.unit ? 1.0f / sqrtf(skb + 1e-6f) : 1.0f, mk = m.unit ? 1.0f / sqrtf(sk + 1e-6f) : 1.0f;
+            const float mq = (m.unit ? 1.0f / sqrtf(sq + 1e-6f) : 1.0f) * m.q_scale;
+            if (lane == 0) p.near[(size_t)kh * p.rows + t] = make_float2(kk * mb * mk, qk * mb * mq);
+        }
         lm_shape<DPL>(m, lane, kv, qv, dst, dst + DP, kq_s + kh);
     }
     const T* v = (const T*)m.qkv + (size_t)t * m.stride + m.v_off;
@@ -322,6 +399,9 @@ linmem_prepare_kernel(const LinMem m, const LinMemPrep p) {
     }
 }
 
+__device__ __forceinline__ void lm_copy8(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
+}
 __device__ __forceinline__ void lm_copy16(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
 }
@@ -411,7 +491,7 @@ linmem_segment_kernel(const LinMem m, const LinMemPrep p) {
 
 // Portions, second kernel: a block owns LM_COLS * CPT columns a warp of a head of a sequence and walks the sequence's
 // tokens; stages of LM_TOK tokens are copied LM_STAGES - 1 ahead. SEG: it walks one segment of the sequence.
-template <int R, int RULE, int DECAY, int CPT, bool SEG>
+template <int R, int RULE, int DECAY, int CPT, bool SEG, bool PAIRS = false>
 __global__ void __launch_bounds__(256)
 linmem_scan_kernel(const LinMem m, const LinMemPrep p) {
     constexpr int DP = 8 * R;                            // the key size, padded
@@ -430,7 +510,8 @@ linmem_scan_kernel(const LinMem m, const LinMemPrep p) {
     const int len = SEG ? min(rest, LM_SEG) : rest;
     if (len <= 0) return;
     const int r = lane & 7, wc = warp * LM_COLS * CPT + (lane >> 3);        // this thread's first column of the block
-    const int stage_floats = LM_TOK * (VEC * DP + cols + 4);
+    const int stage_floats = LM_TOK * (VEC * DP + cols + 4 + (PAIRS ? 2 : 0));
+    const float* near = reinterpret_cast<const float*>(p.near + (size_t)(h / (m.H / m.K)) * p.rows + first);      // (pairs)
     const float* kq = p.kq + ((size_t)(h / (m.H / m.K)) * p.rows + first) * 2 * DP;
     const float* g = DECAY == LM_CHANNEL ? p.g + ((size_t)h * p.rows + first) * DP : nullptr;
     const float* v = p.v + ((size_t)h * p.rows + first) * p.VP + c0;
@@ -451,6 +532,11 @@ linmem_scan_kernel(const LinMem m, const LinMemPrep p) {
             }
             dst += LM_TOK * cols;
             for (int i = threadIdx.x; i < LM_TOK; i += blockDim.x) lm_copy16(dst + 4 * i, sc + 4 * (size_t)(t0 + i));
+            if constexpr (PAIRS) {
+                // (8 bytes a copy: a sequence may begin on any token)
+                dst += LM_TOK * 4;
+                for (int i = threadIdx.x; i < LM_TOK; i += blockDim.x) lm_copy8(dst + 2 * i, near + 2 * (size_t)(t0 + i));
+            }
         }
         asm volatile("cp.async.commit_group;\n" ::);
     };
@@ -508,7 +594,23 @@ linmem_scan_kernel(const LinMem m, const LinMemPrep p) {
                                                vt[t * cols + LM_COLS * c], c4.y, c4.z);
         };
         const int nt = min(LM_TOK, len - t0);
-        if (nt == LM_TOK) {
+        if (PAIRS && nt == LM_TOK) {
+            const float2* nears = reinterpret_cast<const float2*>(base + LM_TOK * (VEC * DP + cols + 4));
+            float keep[CPT];
+#pragma unroll 4
+            for (int t = 0; t < LM_TOK; t += 2) {
+                float v1[CPT], v2[CPT], o1[CPT], o2[CPT];
+#pragma unroll
+                for (int c = 0; c < CPT; ++c) v1[c] = vt[t * cols + LM_COLS * c], v2[c] = vt[(t + 1) * cols + LM_COLS * c];
+                lm_pair<R, CPT>(S, ks + t * 2 * DP, v1, v2, scs[t], scs[t + 1], nears[t + 1], o1, o2);
+#pragma unroll
+                for (int c = 0; c < CPT; ++c) {
+                    if (r == (t & 7)) keep[c] = o1[c];
+                    if (r == (t & 7) + 1) keep[c] = o2[c];
+                    if ((t & 7) == 6 && c0 + wc + LM_COLS * c < m.V) y[(size_t)(t0 + t - 6 + r) * HV + LM_COLS * c] = keep[c];
+                }
+            }
+        } else if (nt == LM_TOK) {
             float keep[CPT];
 #pragma unroll 8
             for (int t = 0; t < LM_TOK; ++t) {
@@ -648,6 +750,7 @@ void lm_launch(const LinMem& m, int n_seqs, int tokens, float* scratch, int sm_c
     p.v = p.kq + (size_t)m.K * p.rows * 2 * DP;
     p.sc = reinterpret_cast<float4*>(p.v + (size_t)m.H * p.rows * p.VP);
     p.g = reinterpret_cast<float*>(p.sc + (size_t)m.H * p.rows);
+    p.near = LM_PAIRS(RULE, DECAY) && lm_pairs(DECAY, n_seqs, m.H, m.D, m.V, sm_count) ? reinterpret_cast<float2*>(p.g) : nullptr;      // (a decay per head stages none per channel)
     p.seg = nullptr;
     p.n_seqs = n_seqs;
     tk_launch(linmem_prepare_kernel<T, R / 4, RULE, DECAY>, dim3(tokens), dim3(256),
@@ -684,6 +787,19 @@ void lm_launch(const LinMem& m, int n_seqs, int tokens, float* scratch, int sm_c
             return;
         }
     }
+    if constexpr (LM_PAIRS(RULE, DECAY) && R <= 16) {
+        if (p.near != nullptr) {
+            constexpr int PC = R == 16 ? 1 : CPT;
+            int pw = R == 16 ? 4 : warps;
+            while (pw > 1 && m.V <= LM_COLS * PC * pw / 2) pw /= 2;
+            const int pc = LM_COLS * PC * pw;
+            const size_t ps = (size_t)LM_STAGES * LM_TOK * (VEC * DP + pc + 4 + 2) * sizeof(float);
+            auto kernel = linmem_scan_kernel<R, RULE, DECAY, PC, false, true>;
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps);
+            tk_launch_after(kernel, dim3((m.V + pc - 1) / pc, m.H, n_seqs), dim3(32 * pw), ps, stream, m, p);
+            return;
+        }
+    }
     static size_t raised = 48 * 1024;
     if (smem > raised) {
         cudaFuncSetAttribute(linmem_scan_kernel<R, RULE, DECAY, CPT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -709,7 +825,8 @@ TK_API int tk_linmem_max_dim() { return 256; }
 TK_API int tk_linmem_scratch(int tokens, int n_seqs, int H, int K, int D, int V, int decay, int sm_count) {
     if (tokens < 4 * n_seqs || n_seqs == 0) return 0;
     const int64_t DP = D <= 32 ? 32 : D <= 64 ? 64 : D <= 128 ? 128 : 256, VP = (V + 3) / 4 * 4;
-    const int64_t floats = (int64_t)(tokens + LM_TOK) * (2 * K * DP + H * (VP + 4) + (decay == LM_CHANNEL ? H * DP : 0)) +
+    const int64_t floats = (int64_t)(tokens + LM_TOK) * (2 * K * DP + H * (VP + 4) + (decay == LM_CHANNEL ? H * DP : 0) +
+                                                      (lm_pairs(decay, n_seqs, H, D, V, sm_count) ? 2 * K : 0)) +
                            (int64_t)lm_slots(tokens, n_seqs, H, D, V, decay, sm_count) * H * V * D;
     return (int)((floats + 31) / 32);
 }
