@@ -155,8 +155,8 @@ def test_gemm_float32_is_not_tf32():
     assert (want - 64.0).abs().min().item() > 1e-2   # TF32 inputs would give exactly 64
 
 
-@pytest.mark.parametrize("m, n, k", [(9, 128, 128), (33, 257, 1000), (64, 1024, 1024), (100, 1024, 4608), (129, 300, 2048),
-                                     (300, 130, 516), (513, 129, 132)])
+@pytest.mark.parametrize("m, n, k", [(9, 256, 256), (33, 257, 1000), (64, 1024, 1024), (100, 1024, 4608), (129, 300, 2048),
+                                     (300, 260, 516), (513, 257, 260)])
 def test_gemm_32_bit_operands_in_parts(m, n, k):
     """The tensor-core form of the 32-bit product at every width of its token tile, split along K and not, with partial tiles
     and chunks: no further from 64 bits than a few 2^-24 (tf32 operands would be off by 2^-11); infinities and NaN end up

@@ -14,9 +14,9 @@
 //
 // Bound by the tensor pipe: six bfloat16 products, i.e. a sixth of its rate, against which the CUDA cores' multiply-adds
 // have a twentieth: 2,048 x 16,384 x 2,048 in 717 us (192 TFLOP/s; gemm_simt.cu 5,414), 16 x 2,048 x 2,048 in 17 us (119),
-// never slower than it from 9 rows and 128 x 128 weights on (14.2 us against 14.5). A CTA owns 128 rows of W (the MMA's M) and BN tokens; 16 warps read 32 columns of both operands
-// from memory into registers a chunk ahead, take them apart and store the three parts as K-major tiles in the 128-byte
-// swizzle (h and m side by side in one row, l in a tile that the two buffers share by halves), one thread issues the
+// never slower than it from 9 rows and 128 x 128 weights on (14.2 us against 14.5; taken from 256 x 256 on). A CTA owns
+// 128 rows of W (the MMA's M) and BN tokens; 16 warps read 32 columns of both operands from memory into registers a chunk
+// ahead, take them apart and store the three parts as K-major tiles in the 128-byte swizzle (h and m side by side in one row, l in a tile that the two buffers share by halves), one thread issues the
 // twelve MMAs of a chunk, and all warps work on the next chunk meanwhile. BN = 256 keeps shared memory (96 bytes a cycle
 // of operand reads) below what the MMAs would need at 128 columns (128). The tokens' tiles are the grid's fast axis, so
 // that neighbouring CTAs read the same rows of W from L2. A product with few tiles is split along K over a cluster whose

@@ -762,12 +762,13 @@ def gemm_skinny_conv(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None
     return out
 
 
-SPLIT32_MIN_ROWS, SPLIT32_MIN_SIDE = 9, 128
+SPLIT32_MIN_ROWS, SPLIT32_MIN_SIDE = 9, 256
 
 
 def gemm_split32_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether a 32-bit product goes to the tensor cores in parts that keep all of its 32 bits (csrc/gemm_split32.cu): 16-byte
-    rows, and sizes at which that is the faster way (below 128 rows of ``w`` or columns its 128-row tiles are mostly empty)."""
+    rows, and sizes at which that is the faster way (below 256 rows of ``w`` or columns either takes as long as a launch, and
+    the sums keep the one order they have in steps of any size)."""
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] >= SPLIT32_MIN_ROWS
             and w.shape[0] >= SPLIT32_MIN_SIDE and x.shape[1] >= SPLIT32_MIN_SIDE and x.shape[1] % 4 == 0
             and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
@@ -793,7 +794,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
     return out
 
 
-STREAM32_MAX_ROWS = 8
+STREAM32_MAX_ROWS, STREAM32_MIN_SIDE = 8, 256
 
 
 def gemm_stream32_ok(x: torch.Tensor, w: torch.Tensor) -> bool:

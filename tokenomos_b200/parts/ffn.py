@@ -33,7 +33,8 @@ class SwiGLU:
         if (self.run == RUN and x.shape[0] <= self.gate_up.tuning.swiglu_fused_rows
                 and ops.gemm_skinny_ok(x, w)):
             act = ops.gemm_skinny(x, w, self.gate_up.bias, swiglu=True)
-        elif self.run == 0 and w.dtype == torch.float32 and ops.gemm_stream32_ok(x, w):
+        elif (self.run == 0 and w.dtype == torch.float32 and min(w.shape) >= ops.STREAM32_MIN_SIDE
+              and ops.gemm_stream32_ok(x, w)):
             act = ops.gemm_stream32(x, w, self.gate_up.bias, swiglu=True)
         else:
             act = ops.swiglu(self.gate_up(x), self.run)

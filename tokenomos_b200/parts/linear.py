@@ -94,8 +94,9 @@ class Linear:
         return F.linear(x, w)
 
     def _product32(self, x: torch.Tensor) -> torch.Tensor:
-        """32-bit operands: the weight-streaming kernel for a few rows, else ``ops.gemm``."""
-        if ops.gemm_stream32_ok(x, self.weight):
+        """32-bit operands: the weight-streaming kernel for a few rows of a matrix of some size, else ``ops.gemm`` (small ones take as
+        long as a launch either way, and keep one order of their sums in steps of any size)."""
+        if min(self.out_features, self.in_features) >= ops.STREAM32_MIN_SIDE and ops.gemm_stream32_ok(x, self.weight):
             return ops.gemm_stream32(x, self.weight, self.bias)
         return ops.gemm(x, self.weight, self.bias, torch.float32)
 
