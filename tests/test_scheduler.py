@@ -345,3 +345,20 @@ def test_prefill_attention_split_rule():
                 n = f(tokens, entries, 32, kv)
                 assert 1 <= n <= 16
                 assert n == 1 or entries * kv * n * 128 * 66 * 4 <= 64 << 20
+
+
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 200])
+@pytest.mark.parametrize("which", ["all", "prompt"])
+def test_tiles_of_one_prompt_are_those_it_has_beside_others(n, which):
+    """The form for one sequence against the general one, whose first sequence it is; the four lists keep their places when they
+    come from one device array."""
+    import numpy as np
+
+    from tokenomos_b200.engine.step import _Tiles
+    one, many = _Tiles.cut([n], 64, which), _Tiles.cut([n, 70], 64, which)
+    k = len(one[0])
+    assert k == int((many[0] == 0).sum())
+    tiles = _Tiles([n], "cpu", None)
+    tiles.put((64, which), torch.from_numpy(np.concatenate(one)))
+    for a, b, c in zip(one, many, tiles.cache[(64, which)]):
+        assert a.dtype == b.dtype and np.array_equal(a, b[:k]) and np.array_equal(c.numpy(), a)

@@ -66,11 +66,16 @@ class _Tiles:
         self.seq_lens, self.device, self.upload = seq_lens, device, upload
         self.cache: dict[int, tuple] = {}
         self.asked = asked          # every (size, which) any step's parts have asked for
+        self.used: set = set()      # what this step's parts have asked for
 
     @staticmethod
     def cut(seq_lens: list[int], size: int, which: str):
         """Host arrays (sequence, first token, offset in the portion, tokens) of the tiles, in
         the order of the sequences; ``which`` other than "all" leaves single-token sequences out."""
+        if len(seq_lens) == 1:               # one prompt: its runs, without the bookkeeping of several
+            n = seq_lens[0] if which == "all" or seq_lens[0] > 1 else 0
+            off = np.arange(0, n, size, dtype=np.int32)
+            return np.zeros(len(off), dtype=np.int32), off, off, np.minimum(size, n - off).astype(np.int32)
         lens = np.asarray(seq_lens, dtype=np.int64)
         starts = np.cumsum(lens) - lens
         counts = -(-lens // size)
@@ -87,16 +92,16 @@ class _Tiles:
         key = (size, which)
         if self.asked is not None:
             self.asked.add(key)
+        self.used.add(key)
         if key not in self.cache:
-            seq, tok0, off, n = self.cut(self.seq_lens, size, which)
-            k = len(seq)
-            if k == 0:
-                empty = torch.empty(0, dtype=torch.int32, device=self.device)
-                self.cache[key] = (empty, empty, empty, empty)
-            else:
-                flat = self.upload(np.concatenate((seq, tok0, off, n)))
-                self.cache[key] = (flat[:k], flat[k:2 * k], flat[2 * k:3 * k], flat[3 * k:])
+            flat = np.concatenate(self.cut(self.seq_lens, size, which))
+            self.put(key, self.upload(flat) if len(flat) else torch.empty(0, dtype=torch.int32, device=self.device))
         return self.cache[key]
+
+    def put(self, key: tuple, flat: torch.Tensor) -> None:
+        """The tiles of ``key`` from one device array (the four of ``cut`` end to end)."""
+        k = flat.numel() // 4
+        self.cache[key] = (flat[:k], flat[k:2 * k], flat[2 * k:3 * k], flat[3 * k:])
 
     def singles(self):
         if self.asked is not None:
@@ -428,6 +433,7 @@ class StepFunction:
         self._step_graph_uses: dict[tuple, int] = {}
         self._graph_pool = None
         self._tile_keys: set = set()     # what the model's parts ask the tile source for
+        self._last_tiles: set = set()    # what the parts of the last step with a prompt portion asked for
         self._tiles_known = False        # an eager step with a prompt portion has run: the set is complete
         # a mixed step's bucket is captured once this many steps have fallen into it
         self.capture_after = 2
@@ -527,10 +533,14 @@ class StepFunction:
             for si, e in enumerate(entries):
                 row = cache.block_table(e.rid, g)
                 tables[gi, si, :min(width, len(row))] = row[:width]
+        # the tile lists that the last step with a prompt portion asked for ride in the same copy (a copy and its event cost the
+        # host as much as two launches)
+        decode_only = all(n == 1 for n in seq_lens)
+        cuts = {} if decode_only else {key: np.concatenate(_Tiles.cut(seq_lens, *key)) for key in sorted(self._last_tiles)}
         flat = self._upload(np.concatenate((
             positions, tok_seq, np.asarray(cu, dtype=np.int32), np.asarray(seq_ctx, dtype=np.int32),
             np.asarray(seq_slot, dtype=np.int32), ids, np.asarray(want, dtype=np.int32),
-            tables.reshape(-1))))
+            tables.reshape(-1), *cuts.values())))
         o = 0
 
         def take(n):
@@ -542,13 +552,18 @@ class StepFunction:
         d_pos, d_tok_seq, d_cu = take(T), take(T), take(S + 1)
         d_ctx, d_slot, d_ids, d_want = take(S), take(S), take(T), take(len(want))
         block_tables = {g: take(S * width).view(S, width) for g in groups}
-        host = HostLayout(seq_lens, seq_ctx, seq_slot, all(n == 1 for n in seq_lens),
+        tiles = _Tiles(seq_lens, self.device, self._upload, self._tile_keys)
+        for key, cut in cuts.items():
+            tiles.put(key, take(len(cut)))
+        if not decode_only:
+            self._last_tiles = tiles.used        # (filled as the parts ask)
+        host = HostLayout(seq_lens, seq_ctx, seq_slot, decode_only,
                           max(c + n for c, n in zip(seq_ctx, seq_lens)))
         ctx = StepContext(
             n_tokens=T, n_seqs=S, positions=d_pos, tok_seq=d_tok_seq, cu_seqlens=d_cu,
             seq_ctx=d_ctx, seq_slot=d_slot, block_tables=block_tables, states=cache.states,
             state_groups=cache.state_groups, page_size=cache.page_size, host=host,
-            tile_source=_Tiles(seq_lens, self.device, self._upload, self._tile_keys))
+            tile_source=tiles)
         return ctx, d_ids, d_want
 
     @torch.no_grad()
