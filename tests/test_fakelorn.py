@@ -905,6 +905,28 @@ def test_greedy_generation_through_llm(name, work, graphs, folders):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("work", ["fp32", "bf16"])
+def test_recorded_steps_whose_convolution_is_cut_otherwise_than_an_eager_ones(work, tmp_path):
+    """6,144 channels: prompts of 1,500 and 1,900 tokens are cut into other tiles than the 2,048-token step that is recorded
+    for them, at the third prompt or ahead of time; it gives the replies of steps that are never recorded."""
+    from tokenomos_b200 import LLM, SamplingParams
+
+    config = {"architecture": "Fakelorn", "vocab": 64, "width": 64, "norm": {"eps": 1e-5, "groups": 1},
+              "layers": [dict(mamba(64, 64, 128, 8, 4, 8), mlp=dense(64))]}
+    write_folder(tmp_path / "wide", config, make_tensors(config, 9))
+    g = torch.Generator().manual_seed(2)
+    prompts = [torch.randint(0, 64, (n,), generator=g).tolist() for n in (1500, 1900, 1500, 1700)]
+    replies = {}
+    for graphs, warmup in ((False, False), (True, False), (True, True)):
+        with LLM(str(tmp_path / "wide"), work=work, page=16, max_len=2048, slots=2, pages=400, graphs=graphs, warmup=warmup) as llm:
+            replies[graphs, warmup] = [llm.generate([p], SamplingParams(max_tokens=3))[0].token_ids for p in prompts]
+            assert ((2048, 4) in llm.engine.step_fn._step_graphs) == graphs
+            assert (llm.engine.stats.graph_steps > 0) == graphs
+    if work == "fp32":
+        assert replies[True, False] == replies[False, False] == replies[True, True]
+
+
+@pytest.mark.gpu
 def test_trace_program_and_command_line(folders, tmp_path):
     name = "A"
     folder, _ = folders[name]

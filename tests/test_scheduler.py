@@ -362,3 +362,51 @@ def test_tiles_of_one_prompt_are_those_it_has_beside_others(n, which):
     tiles.put((64, which), torch.from_numpy(np.concatenate(one)))
     for a, b, c in zip(one, many, tiles.cache[(64, which)]):
         assert a.dtype == b.dtype and np.array_equal(a, b[:k]) and np.array_equal(c.numpy(), a)
+
+
+def test_a_recorded_step_has_the_tile_lists_of_its_own_size(monkeypatch):
+    """A part that cuts 1,500 tokens into other lengths than the 2,048 of the bucket: the bucket's step is recorded with the
+    lists it asks for itself, and one recorded earlier stays in use when a step of another size has asked for others."""
+    from tokenomos_b200 import ops
+    from tokenomos_b200.engine import step as st
+    from tokenomos_b200.sampling import sampler
+
+    class Model:
+        vocab = 10
+
+        def embed(self, ids, ctx):
+            return torch.zeros(ids.numel(), 8)
+
+        def embed_fed(self, ids, use_prev, last, slots, ctx):
+            return self.embed(ids, ctx)
+
+        def forward(self, h, ctx):
+            ctx.tiles(ops.seq_conv_tile(16, ctx.n_tokens, 6144))
+            return h
+
+        def logits(self, out, want):
+            return torch.zeros(want.numel(), self.vocab)
+
+    monkeypatch.setattr(sampler, "sample_packed", lambda *a, **k: None)
+    monkeypatch.setattr(torch.cuda, "graph_pool_handle", lambda: None)
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda t: t)
+    # (a capture runs the step twice: to learn and warm up, and to record)
+    monkeypatch.setattr(st._StepGraph, "capture", lambda g, model, pool: (g.learn(model), g.body(model)))
+    cache = CacheManager(SPECS, 16, 400, 3, torch.float32, "cpu")
+    steps = st.StepFunction(Model(), cache)
+    cache.admit("r")
+    graphs = {}
+    for n in (1500, 1500, 1500, 400, 400, 400, 1500):
+        entries = [st.StepEntry("r", [1] * n, [n - 1])]
+        graph = steps.step_graph_for(entries)
+        if graph is None:
+            steps.run(entries, commit=False)
+        else:
+            graphs.setdefault(n, graph)
+    assert ops.seq_conv_tile(16, 1500, 6144) != ops.seq_conv_tile(16, 2048, 6144)
+    for n, bucket in ((1500, 2048), (400, 512)):
+        assert graphs[n].tokens_cap == bucket and graphs[n].tile_keys == [(ops.seq_conv_tile(16, bucket, 6144), "all")]
+        assert all(lst.numel() == graphs[n].tile_cap[graphs[n].tile_keys[0]] for lst in graphs[n].ctx.tiles(*graphs[n].tile_keys[0]))
+    assert steps.step_graph_for([st.StepEntry("r", [1] * 1500, [1499])]) is graphs[1500]
+    monkeypatch.setattr(steps, "decode_graph", lambda rows: steps._graphs.setdefault(rows, None))
+    assert steps.capture_shapes(1, 2048, 1)[1] == len(st.STEP_TOKEN_BUCKETS[:7])

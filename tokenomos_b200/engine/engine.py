@@ -186,8 +186,7 @@ class Engine:
         """Touch every kernel variant and record every step shape serving will meet, before the
         first request (the reference's engine does the same before it serves, Tokenomos
         core/engine.py:635-664): two short requests run one eager mixed step (it builds the
-        kernel library if need be, loads the library handles and tells which tile lists the
-        model's parts ask for), then the decode step of every batch-size bucket up to ``slots``
+        kernel library if need be and loads the library handles), then the decode step of every batch-size bucket up to ``slots``
         and the mixed step of every (token, sequence) bucket under the token budget are
         captured. Without it each shape is captured when serving first meets it (a mixed one
         the third time). Returns the numbers of decode and mixed shapes recorded; the statistics

@@ -62,11 +62,10 @@ def _forget_capture_run() -> None:
 class _Tiles:
     """Cuts the step's sequences into runs of at most ``size`` tokens, on demand, once per size."""
 
-    def __init__(self, seq_lens: list[int], device, upload, asked: set | None = None):
+    def __init__(self, seq_lens: list[int], device, upload):
         self.seq_lens, self.device, self.upload = seq_lens, device, upload
         self.cache: dict[int, tuple] = {}
-        self.asked = asked          # every (size, which) any step's parts have asked for
-        self.used: set = set()      # what this step's parts have asked for
+        self.used: set = set()      # the (size, which) this step's parts have asked for
 
     @staticmethod
     def cut(seq_lens: list[int], size: int, which: str):
@@ -90,8 +89,6 @@ class _Tiles:
 
     def tiles(self, size: int, which: str = "all"):
         key = (size, which)
-        if self.asked is not None:
-            self.asked.add(key)
         self.used.add(key)
         if key not in self.cache:
             flat = np.concatenate(self.cut(self.seq_lens, size, which))
@@ -104,8 +101,6 @@ class _Tiles:
         self.cache[key] = (flat[:k], flat[k:2 * k], flat[2 * k:3 * k], flat[3 * k:])
 
     def singles(self):
-        if self.asked is not None:
-            self.asked.add("singles")
         if "singles" not in self.cache:
             idx, start = [], 0
             for length in self.seq_lens:
@@ -239,13 +234,17 @@ STEP_SEQ_BUCKETS = (4, 16, 64, 128, 256, 512, 1024)
 class _FixedTiles:
     """Tile lists of a captured step: device arrays of the greatest length the bucket allows,
     refilled before every replay; entries past the step's own are empty tiles (0 tokens) and
-    negative token indices, which the kernels skip."""
+    negative token indices, which the kernels skip. ``make``: forms a list that is asked for and not
+    there (only while the step learns which lists it needs)."""
 
-    def __init__(self, views: dict):
-        self.views = views
+    def __init__(self, views: dict, make=None):
+        self.views, self.make = views, make
 
     def tiles(self, size: int, which: str = "all"):
-        return self.views[(size, which)]
+        key = (size, which)
+        if key not in self.views and self.make is not None:
+            self.views[key] = self.make(key)
+        return self.views[key]
 
     def singles(self):
         return self.views["singles"]
@@ -259,16 +258,29 @@ class _StepGraph:
     (its tokens are carried through the row-wise kernels and belong to no tile); unused sequences
     are empty. Logits are taken at one row per sequence at most (the row whose token is sampled);
     unused rows repeat row 0. As in the decode graph, the id of a single token may come from
-    ``last_token`` on the device."""
+    ``last_token`` on the device.
+
+    Which tile lists the layout holds is what the parts ask for at the bucket's own token count
+    (``learn``): a part may cut a step of another size into other lengths."""
 
     RING = 2
 
-    def __init__(self, step_fn: "StepFunction", tokens: int, seqs: int, tile_keys: set):
-        cache, dev = step_fn.cache, step_fn.device
+    def __init__(self, step_fn: "StepFunction", tokens: int, seqs: int):
+        self.cache, self.device = step_fn.cache, step_fn.device
         self.tokens_cap, self.seqs_cap = tokens, seqs
-        self.width = cache.max_blocks
-        self.groups = list(cache.groups)
-        T, S = tokens, seqs
+        self.width = self.cache.max_blocks
+        self.groups = list(self.cache.groups)
+        self.windowless = {g: self.cache.groups[g].window is None for g in self.groups}
+        self.turn = 0
+        self.sampled = torch.zeros(seqs, dtype=torch.int32, device=self.device)
+        self.last_token = step_fn.last_token
+        self.graph = None
+        self.launches = 0
+
+    def _lay_out(self, tile_keys: list, learning: bool = False) -> None:
+        """The device buffer with the layout's fields and a tile list for each of ``tile_keys``, all zero, and the context
+        that reads it. ``learning``: any other list is formed when it is asked for."""
+        T, S = self.tokens_cap, self.seqs_cap
         self.off = {}
         o = 0
 
@@ -283,41 +295,46 @@ class _StepGraph:
             field_(name, n)
         for g in self.groups:
             field_(("table", g), S * self.width)
-        self.tile_keys = sorted(k for k in tile_keys if k != "singles")
+        self.tile_keys = tile_keys
         self.tile_cap = {}
         for key in self.tile_keys:
-            self.tile_cap[key] = T // key[0] + S + 1
+            self.tile_cap[key] = self._tiles_most(key)
             field_(("tiles", key), 4 * self.tile_cap[key])
         field_("singles", S)
         self.size = o
-        self.host = [torch.zeros(self.size, dtype=torch.int32).pin_memory() for _ in range(self.RING)]
-        self.host_np = [h.numpy() for h in self.host]
-        # what each staging buffer's block-table rows hold: (request, entries written) per row
-        self.table_rows = [{g: [(None, 0)] * S for g in self.groups} for _ in range(self.RING)]
-        self.windowless = {g: cache.groups[g].window is None for g in self.groups}
-        self.tokens_host = [torch.zeros(S, dtype=torch.int32).pin_memory() for _ in range(self.RING)]
-        self.turn = 0
-        self.dev = torch.zeros(self.size, dtype=torch.int32, device=dev)
-        self.sampled = torch.zeros(S, dtype=torch.int32, device=dev)
-        self.last_token = step_fn.last_token
+        self.dev = torch.zeros(self.size, dtype=torch.int32, device=self.device)
 
         def view(name):
             a, n = self.off[name]
             return self.dev[a:a + n]
 
-        views = {"singles": view("singles")}
-        for key in self.tile_keys:
-            flat, k = view(("tiles", key)), self.tile_cap[key]
-            views[key] = (flat[:k], flat[k:2 * k], flat[2 * k:3 * k], flat[3 * k:])
+        def quarters(flat):
+            k = flat.numel() // 4
+            return flat[:k], flat[k:2 * k], flat[2 * k:3 * k], flat[3 * k:]
+
+        def empty(key):
+            return quarters(torch.zeros(4 * self._tiles_most(key), dtype=torch.int32, device=self.device))
+
+        views = {"singles": view("singles"), **{key: quarters(view(("tiles", key))) for key in self.tile_keys}}
+        cache = self.cache
         self.ctx = StepContext(
             n_tokens=T, n_seqs=S, positions=view("positions"), tok_seq=view("tok_seq"),
             cu_seqlens=view("cu"), seq_ctx=view("seq_ctx"), seq_slot=view("seq_slot"),
             block_tables={g: view(("table", g)).view(S, self.width) for g in self.groups},
             states=cache.states, state_groups=cache.state_groups, page_size=cache.page_size,
-            host=HostLayout.of_captured_step(False, cache.max_len), tile_source=_FixedTiles(views))
+            host=HostLayout.of_captured_step(False, cache.max_len),
+            tile_source=_FixedTiles(views, empty if learning else None))
         self.view = view
-        self.graph = None
-        self.launches = 0
+
+    def _tiles_most(self, key: tuple) -> int:
+        return self.tokens_cap // key[0] + self.seqs_cap + 1
+
+    def learn(self, model) -> None:
+        """Run the step once on an all-zero layout (which also warms it up: library handles, sizes) and lay it out for good with
+        the tile lists its parts asked for."""
+        self._lay_out([], learning=True)
+        self.body(model)
+        self._lay_out(sorted(k for k in self.ctx.tile_source.views if k != "singles"))
 
     def body(self, model):
         from tokenomos_b200.sampling import sampler
@@ -335,9 +352,14 @@ class _StepGraph:
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
-            self.body(model)              # warm-up outside the capture (library handles, sizes)
+            self.learn(model)             # outside the capture
         torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
+        self.host = [torch.zeros(self.size, dtype=torch.int32).pin_memory() for _ in range(self.RING)]
+        self.host_np = [h.numpy() for h in self.host]
+        # what each staging buffer's block-table rows hold: (request, entries written) per row
+        self.table_rows = [{g: [(None, 0)] * self.seqs_cap for g in self.groups} for _ in range(self.RING)]
+        self.tokens_host = [torch.zeros(self.seqs_cap, dtype=torch.int32).pin_memory() for _ in range(self.RING)]
         graph = torch.cuda.CUDAGraph()
         before = _lib.calls()
         with _no_collection(), torch.cuda.graph(graph, pool=pool):
@@ -432,9 +454,7 @@ class StepFunction:
         self._step_graphs: dict[tuple, _StepGraph] = {}
         self._step_graph_uses: dict[tuple, int] = {}
         self._graph_pool = None
-        self._tile_keys: set = set()     # what the model's parts ask the tile source for
-        self._last_tiles: set = set()    # what the parts of the last step with a prompt portion asked for
-        self._tiles_known = False        # an eager step with a prompt portion has run: the set is complete
+        self._last_tiles: set = set()    # the tile lists the parts of the last step with a prompt portion asked for
         # a mixed step's bucket is captured once this many steps have fallen into it
         self.capture_after = 2
         # the token each request's last step sampled, by state slot (slot 0: padded rows)
@@ -552,7 +572,7 @@ class StepFunction:
         d_pos, d_tok_seq, d_cu = take(T), take(T), take(S + 1)
         d_ctx, d_slot, d_ids, d_want = take(S), take(S), take(T), take(len(want))
         block_tables = {g: take(S * width).view(S, width) for g in groups}
-        tiles = _Tiles(seq_lens, self.device, self._upload, self._tile_keys)
+        tiles = _Tiles(seq_lens, self.device, self._upload)
         for key, cut in cuts.items():
             tiles.put(key, take(len(cut)))
         if not decode_only:
@@ -573,8 +593,6 @@ class StepFunction:
         the requests' lengths to the caller (the scheduler does it when it takes the tokens)."""
         ctx, ids, want = self.layout(entries)
         out = self.model.forward(self.model.embed(ids, ctx), ctx)
-        if not ctx.host.decode_only:
-            self._tiles_known = True
         logits = self.model.logits(out, want) if want.numel() else None
         if commit:
             for e in entries:
@@ -697,7 +715,7 @@ class StepFunction:
         wanted row per entry at most), capturing it when its bucket has been met
         ``capture_after`` times; None while it is not worth a capture, or if no bucket fits."""
         total = sum(len(e.tokens) for e in entries)
-        if any(len(e.want) > 1 for e in entries) or not self._tiles_known:
+        if any(len(e.want) > 1 for e in entries):
             return None
         tokens = self._bucket(total, STEP_TOKEN_BUCKETS)
         # a step that does not fill its bucket needs one more sequence: the dummy one
@@ -711,48 +729,42 @@ class StepFunction:
             self._step_graph_uses[key] = uses
             if uses <= self.capture_after:
                 return None
-            g = _StepGraph(self, tokens, seqs, self._tile_keys)
-            if self._graph_pool is None:
-                self._graph_pool = torch.cuda.graph_pool_handle()
-            g.capture(self.model, self._graph_pool)
-            self._step_graphs[key] = g
-        elif not self._tile_keys <= set(g.tile_keys) | {"singles"}:
-            return None          # a part asked for tiles the capture did not know: run eagerly
+            g = self._capture_step(key)
+        return g
+
+    def _capture_step(self, key: tuple) -> "_StepGraph":
+        g = _StepGraph(self, *key)
+        if self._graph_pool is None:
+            self._graph_pool = torch.cuda.graph_pool_handle()
+        g.capture(self.model, self._graph_pool)
+        self._step_graphs[key] = g
         return g
 
     def capture_shapes(self, decode_rows: int, step_tokens: int, step_seqs: int) -> tuple[int, int]:
         """Record ahead of time what serving would record at first use: the decode step of every
         bucket up to ``decode_rows`` sequences, and the mixed step of every (token, sequence)
         bucket a step of at most ``step_tokens`` tokens and ``step_seqs`` sequences can fall
-        into. Mixed shapes need to know which tile lists the model's parts ask for, which the
-        first eager step with a prompt portion tells; without one they are left for later.
-        Returns how many decode and mixed shapes are now recorded."""
+        into. Returns how many decode and mixed shapes are now recorded."""
         for b in DECODE_BUCKETS:
             bucket = min(b, max(1, self.cache.max_requests))
             if bucket not in self._graphs:
                 self.decode_graph(bucket)
             if b >= decode_rows:
                 break
-        if self._tiles_known:
-            top_tokens = self._bucket(step_tokens, STEP_TOKEN_BUCKETS)
-            top_seqs = self._bucket(step_seqs + 1, STEP_SEQ_BUCKETS)      # + the dummy sequence
-            below = 0
-            for seqs in STEP_SEQ_BUCKETS:
-                if top_seqs is None or seqs > top_seqs:
+        top_tokens = self._bucket(step_tokens, STEP_TOKEN_BUCKETS)
+        top_seqs = self._bucket(step_seqs + 1, STEP_SEQ_BUCKETS)      # + the dummy sequence
+        below = 0
+        for seqs in STEP_SEQ_BUCKETS:
+            if top_seqs is None or seqs > top_seqs:
+                break
+            for tokens in STEP_TOKEN_BUCKETS:
+                if top_tokens is None or tokens > top_tokens:
                     break
-                for tokens in STEP_TOKEN_BUCKETS:
-                    if top_tokens is None or tokens > top_tokens:
-                        break
-                    # a step of this sequence bucket has more than `below` sequences (one of
-                    # them may be the dummy), each with a token
-                    if tokens < below or (tokens, seqs) in self._step_graphs:
-                        continue
-                    g = _StepGraph(self, tokens, seqs, self._tile_keys)
-                    if self._graph_pool is None:
-                        self._graph_pool = torch.cuda.graph_pool_handle()
-                    g.capture(self.model, self._graph_pool)
-                    self._step_graphs[(tokens, seqs)] = g
-                below = seqs
+                # a step of this sequence bucket has more than `below` sequences (one of
+                # them may be the dummy), each with a token
+                if tokens >= below and (tokens, seqs) not in self._step_graphs:
+                    self._capture_step((tokens, seqs))
+            below = seqs
         return len(self._graphs), len(self._step_graphs)
 
     def launch_step_graph(self, g: "_StepGraph", entries: list[StepEntry], sampling_rows: list[tuple],
