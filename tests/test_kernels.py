@@ -403,6 +403,41 @@ def test_attention_f32_equals_the_general_kernel(monkeypatch, H, Hkv, P, window,
     assert (got - seen["want"]).norm() <= 2e-6 * seen["want"].norm()
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("window", [None, 40, -48])
+@pytest.mark.parametrize("H, Hkv", [(4, 4), (16, 8), (8, 1)])
+def test_attention_f32_values_that_are_not_finite_reach_the_rows_that_see_them(H, Hkv, window, bad):
+    """One key's value is not finite: the rows that do not see that key (before it, or past their window or chunk) keep their
+    results (their tile's products are added up in another order: a few 2^-24 of a sum), those that see it are not finite."""
+    from tokenomos_b200 import ops
+    ctx, n, P = 21, 150, 16
+    total = ctx + n
+    q = torch.randn(n, H, 64, device="cuda")
+    pool = torch.randn(-(-total // P), 2, Hkv, P, 64, device="cuda")
+    table = i32([list(range(pool.shape[0]))])
+    per = ops.attention_f32_tokens(H, Hkv)
+    tiles = i32(list(range(0, n, per))), i32([min(per, n - o) for o in range(0, n, per)])
+
+    def run(pool):
+        out = torch.empty_like(q)
+        ops.attention_f32_prefill(q, pool, out, i32(list(range(ctx, total))), i32([0] * n), table, *tiles, window, 0.125)
+        return out
+
+    was = run(pool)
+    for key in (3, ctx + 40, ctx + 77):
+        hurt = pool.clone()
+        hurt[key // P, 1, :, key % P, 5] = bad
+        got = run(hurt)
+        i = torch.arange(ctx, total, device="cuda")
+        sees = key <= i
+        if window is not None:
+            sees &= key > i - window if window > 0 else key >= i // -window * -window
+        assert (got[~sees] - was[~sees]).norm() <= 1e-6 * was.norm()
+        assert not torch.isfinite(got[sees][:, :, 5]).any()
+        rest = [c for c in range(64) if c != 5]
+        assert (got[:, :, rest] - was[:, :, rest]).norm() <= 1e-6 * was.norm()
+
+
 def test_swiglu32_vectorised_equals_the_scalar_kernel():
     """Whole and partial blocks of a row; rows that do not begin on 16 bytes go the scalar way, with the same bits."""
     from tokenomos_b200 import ops

@@ -108,6 +108,7 @@ attn32_prefill_kernel(const float* q, const float* kv_pool, float* out, const in
         }
         __syncthreads();
         float4 kv[4], vv[4];
+        float bad = 0.f;                     // NaN once a value is not finite
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             // keys: 16 lanes a row; values: a lane a row, so that its four columns turn round without conflicts
@@ -126,8 +127,9 @@ attn32_prefill_kernel(const float* q, const float* kv_pool, float* out, const in
             turned[F_LD] = vv[e].y;
             turned[2 * F_LD] = vv[e].z;
             turned[3 * F_LD] = vv[e].w;
+            bad = fmaf(vv[e].x, 0.f, fmaf(vv[e].y, 0.f, fmaf(vv[e].z, 0.f, fmaf(vv[e].w, 0.f, bad))));
         }
-        __syncthreads();
+        const int guarded = __syncthreads_or(bad != bad);
         float2 s2[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -165,7 +167,19 @@ attn32_prefill_kernel(const float* q, const float* kv_pool, float* out, const in
             }
         }
         __syncwarp();                        // a row's weights are written and read by the same half-warp
-        tile_product(Ps + ty * 4 * F_LD, Vt + tx * F_LD, o);
+        if (!guarded) {
+            tile_product(Ps + ty * 4 * F_LD, Vt + tx * F_LD, o);
+            continue;
+        }
+        // a weight of zero does not hide a value that is not finite: the keys a row sees, and no others
+        for (int k = 0; k < F_KEYS; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (j0 + k > pos[i] || j0 + k < seen[i]) continue;
+                const float p = Ps[(ty * 4 + i) * F_LD + k];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) o[i][j].x = fmaf(p, Vt[(tx + 16 * j) * F_LD + k], o[i][j].x);
+            }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
