@@ -175,6 +175,28 @@ def test_gemm_32_bit_operands_in_parts(m, n, k):
     assert ops.gemm_tc_status() == 0
 
 
+@pytest.mark.parametrize("m, n, k", [(9, 256, 256), (64, 1024, 1024), (129, 300, 2048), (300, 260, 516)])
+def test_gemm_32_bit_sums_that_overflow(m, n, k):
+    """Finite operands whose products, or sums, pass the largest float: infinities (and no NaN but where multiply-adds in the order of
+    K have one) come out of every width and split, and the other elements keep their values."""
+    from tokenomos_b200 import ops
+    x, w = torch.randn(m, k), torch.randn(n, k)
+    x[1] = 2.0 ** 100 * (1 + 5 / 1024)           # rounds up in 16 bits: the rest is negative, and so are its products
+    w[3], w[9] = 2.0 ** 40, -(2.0 ** 40)
+    x[2] = 3e38
+    w[5] = 0.25                                   # a sum that passes the largest float on its way
+    x[4, : k // 2], x[4, k // 2:] = 3e38, -3e38   # half the sum is +inf, the other half -inf
+    x, w, out = dev(x), dev(w), torch.empty(m, n, device="cuda")
+    got = ops.gemm(x, w).cpu()
+    ops._lib.call("tk_gemm_simt", x.data_ptr(), k, w.data_ptr(), k, None, out.data_ptr(), n, m, n, k, 0, 0, ops._stream())
+    want = out.cpu()
+    assert torch.isinf(want[1, 3]) and torch.isinf(want[1, 9]) and torch.isinf(want[2, 5]) and torch.isinf(want[4, 5])
+    odd = ~torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), ~odd) and torch.equal(got[odd].nan_to_num(7.0), want[odd].nan_to_num(7.0))
+    plain = [r for r in range(m) if r not in (1, 2, 4)]
+    assert (got[plain] - want[plain]).norm() <= 4e-6 * want[plain].norm()
+
+
 @pytest.mark.parametrize("swiglu", [False, True])
 @pytest.mark.parametrize("m", [1, 2, 3, 8])
 @pytest.mark.parametrize("n, k", [(9216, 1024), (1024, 4608), (70, 36), (1030, 1028), (2, 4)])

@@ -22,8 +22,9 @@
 // that neighbouring CTAs read the same rows of W from L2. A product with few tiles is split along K over a cluster whose
 // CTAs add up their parts through distributed shared memory in a fixed order.
 //
-// An input that is infinite, NaN or rounds up to infinity in 16 bits would leave NaN where 32-bit arithmetic has an
-// infinity: the threads that take such an input apart notice, and their CTA forms its tile again by multiply-adds.
+// An input that is infinite, NaN or rounds up to infinity in 16 bits leaves NaN in every sum it enters, and finite inputs
+// whose products overflow may leave infinities of both signs in the two accumulators: a sum that does not come out finite is
+// formed again by multiply-adds in the order of K, which put infinities and NaN where gemm_simt.cu puts them.
 #include <cooperative_groups.h>
 
 #include "tcgen05.cuh"
@@ -47,13 +48,11 @@ __device__ __forceinline__ bool split_wait(uint32_t bar, uint32_t parity, int wh
     return true;
 }
 
-// Two floats -> (h, m, l) pairs of bfloat16; `bad` turns NaN when one of them has no finite parts.
-__device__ __forceinline__ void take_apart(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l, float& bad) {
+// Two floats -> (h, m, l) pairs of bfloat16.
+__device__ __forceinline__ void take_apart(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
     const __nv_bfloat162 hh = __floats2bfloat162_rn(a, b);
     h = *reinterpret_cast<const uint32_t*>(&hh);
     const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-    bad = fmaf(ra, 0.f, bad);
-    bad = fmaf(rb, 0.f, bad);
     const __nv_bfloat162 mm = __floats2bfloat162_rn(ra, rb);
     m = *reinterpret_cast<const uint32_t*>(&mm);
     const __nv_bfloat162 ll = __floats2bfloat162_rn(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
@@ -79,6 +78,14 @@ __device__ __forceinline__ void tmem_add(uint32_t taddr, float (&acc)[COLS]) {
             for (int e = 0; e < 8; ++e) acc[c + e] += v[e];
         }
     }
+}
+
+// One element by multiply-adds in the order of K.
+__device__ __noinline__ float sum_again(const float* w, int64_t ldw, int row, const float* x, int64_t ldx, int token, int K) {
+    const float *wr = w + (size_t)row * ldw, *xr = x + (size_t)token * ldx;
+    float s = 0.f;
+    for (int k = 0; k < K; ++k) s = fmaf(wr[k], xr[k], s);
+    return s;
 }
 
 template <int BN>
@@ -145,7 +152,6 @@ gemm_split32_kernel(const float* x, int64_t ldx, const float* w, int64_t ldw, co
 #pragma unroll
     for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
     const uint32_t my_tmem = ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * COLS);
-    float bad = 0.f;
     bool ok = true;
 
     pdl_wait();
@@ -158,10 +164,10 @@ gemm_split32_kernel(const float* x, int64_t ldx, const float* w, int64_t ldw, co
         for (int i = 0; i < UNITS; ++i) {
             if ((warp + SP_WARPS * i) * 8 >= ROWS) continue;
             uint4 h, m, l;
-            take_apart(next[i][0].x, next[i][0].y, h.x, m.x, l.x, bad);
-            take_apart(next[i][0].z, next[i][0].w, h.y, m.y, l.y, bad);
-            take_apart(next[i][1].x, next[i][1].y, h.z, m.z, l.z, bad);
-            take_apart(next[i][1].z, next[i][1].w, h.w, m.w, l.w, bad);
+            take_apart(next[i][0].x, next[i][0].y, h.x, m.x, l.x);
+            take_apart(next[i][0].z, next[i][0].w, h.y, m.y, l.y);
+            take_apart(next[i][1].x, next[i][1].y, h.z, m.z, l.z);
+            take_apart(next[i][1].z, next[i][1].w, h.w, m.w, l.w);
             const uint32_t row_at = (uint32_t)((warp + SP_WARPS * i) * 8 + sub_row) * 128;
             auto put = [&](uint32_t tile, uint32_t chunk16, const uint4& v) {        // (sub_row is the row modulo 8)
                 asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(tile + row_at + ((chunk16 ^ sub_row) << 4)), "r"(v.x),
@@ -217,26 +223,17 @@ gemm_split32_kernel(const float* x, int64_t ldx, const float* w, int64_t ldw, co
         tmem_add<COLS>(tmem_corr + my_tmem, acc);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
-    const int again = __syncthreads_or(bad != bad);
+    __syncthreads();
     const int i_row = row0 + (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS;
-    if (again) {
-        // some input has no finite parts: this tile by multiply-adds in the order of K
-        const float* wr = w + (size_t)min(i_row, N - 1) * ldw;
-        const int k_end = min(K, (first + n_chunks) * SP_KC);
-#pragma unroll
-        for (int c = 0; c < COLS; ++c) {
-            const float* xr = x + (size_t)min(tok0 + col0 + c, M - 1) * ldx;
-            float s = 0.f;
-            for (int k = first * SP_KC; k < k_end; ++k) s = fmaf(wr[k], xr[k], s);
-            acc[c] = s;
-        }
-    }
     if (splitk == 1) {
         if (i_row < N) {
             const float add = bias != nullptr ? bias[i_row] : 0.f;
 #pragma unroll
             for (int c = 0; c < COLS; ++c)
-                if (tok0 + col0 + c < M) out[(size_t)(tok0 + col0 + c) * ldo + i_row] = acc[c] + add;
+                if (tok0 + col0 + c < M) {
+                    if (!isfinite(acc[c])) acc[c] = sum_again(w, ldw, i_row, x, ldx, tok0 + col0 + c, K);
+                    out[(size_t)(tok0 + col0 + c) * ldo + i_row] = acc[c] + add;
+                }
         }
     } else {
         // every CTA of the cluster leaves its part [BN][128] in its own shared memory (the operand tiles are done with);
@@ -252,7 +249,9 @@ gemm_split32_kernel(const float* x, int64_t ldx, const float* w, int64_t ldw, co
         for (int j = from + (warp >> 2); j < from + share; j += 4) {
             float s = 0.f;
             for (int p = 0; p < splitk; ++p) s += cluster.map_shared_rank(mine, p)[j * SP_BM + r];
-            if (i_row < N && tok0 + j < M) out[(size_t)(tok0 + j) * ldo + i_row] = s + add;
+            if (i_row >= N || tok0 + j >= M) continue;
+            if (!isfinite(s)) s = sum_again(w, ldw, i_row, x, ldx, tok0 + j, K);
+            out[(size_t)(tok0 + j) * ldo + i_row] = s + add;
         }
         cluster.sync();
     }
