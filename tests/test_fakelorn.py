@@ -1001,6 +1001,29 @@ def test_scan_by_chunks(H, V, N, G, lens, ctx, dtype):
 
 
 @pytest.mark.gpu
+def test_scan_by_chunks_with_decays_of_zero():
+    """A head whose rate overflows forgets everything at every token, as it does in the walk over one token at a time:
+    y_t = (dt_t B_t . C_t + D) x_t, and the state is the last token's."""
+    from tokenomos_b200 import ops
+    T, H, V, N = 500, 2, 64, 64
+    g = torch.Generator().manual_seed(3)
+    xbc, raw = torch.randn(T, H * V + 2 * N, generator=g), torch.randn(T, H, generator=g)
+    a_log, skip = torch.tensor([100.0, 0.0]), torch.randn(H, generator=g)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    st = torch.randn(2, H, N, V, generator=g).cuda()
+    assert ops._lib.call("tk_ssd_chunked_scratch", T, 1, H, V, N, 1) > 0
+    y = ops.ssd_scan(xbc.cuda(), raw.cuda(), torch.zeros(H).cuda(), a_log.cuda(), skip.cuda(), st, i32([0, T]), i32([4]), i32([1]), 1,
+                     H, V, N, 1)[0].double().cpu().view(T, H, V)
+    x, B, C = xbc[:, :H * V].double().view(T, H, V), xbc[:, H * V:H * V + N].double(), xbc[:, H * V + N:].double()
+    dt = torch.nn.functional.softplus(raw.double())
+    want = ((dt[:, 0] * (B * C).sum(1) + skip[0].double())[:, None]) * x[:, 0]
+    assert (y[:, 0] - want).norm() <= 1e-6 * want.norm()
+    last = dt[-1, 0] * B[-1][:, None] * x[-1, 0][None, :]
+    assert (st[1, 0].double().cpu() - last).norm() <= 1e-6 * last.norm()
+    assert torch.isfinite(y).all() and torch.isfinite(st).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("K", [2, 3, 4])
 @pytest.mark.parametrize("C, tile", [(4, 4), (516, 16), (1028, 5)])
 def test_four_channels_a_thread_give_the_scalar_convolutions_bits(C, tile, K):

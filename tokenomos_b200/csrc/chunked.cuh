@@ -56,7 +56,9 @@ struct SsdDecay {
     __device__ __forceinline__ void at(int token, int h, double& log_a, float& w) const {
         const float v = dt_raw[(size_t)token * dt_stride + h] + bias[h];
         const float dt = v > 20.f ? v : log1pf(expf(v));
-        log_a = -(double)expf(A_log[h]) * (double)dt;
+        // (a decay of 0 keeps a finite logarithm: differences of two infinite ones would be NaN)
+        const double la = -(double)expf(A_log[h]) * (double)dt;
+        log_a = la < -1e6 ? -1e6 : la;
         w = dt;
     }
     __device__ __forceinline__ float skip(int h) const { return D_skip[h]; }
