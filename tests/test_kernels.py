@@ -1126,7 +1126,7 @@ def test_gemm_skinny(m, n, k, out_dtype):
 
 
 @pytest.mark.parametrize("m", [1, 5, 8])
-@pytest.mark.parametrize("n, k", [(7120, 1032), (9504, 2048), (7136, 1992)])
+@pytest.mark.parametrize("n, k", [(7120, 1032), (9504, 2048), (7136, 1992), (7136, 1400), (7136, 1408)])
 def test_gemm_skinny_tall_matrices(m, n, k):
     """Tall matrices of one to two thousand columns, whose blocks a CTA takes one after the other: a last round and a last block
     that are not full, slices of K that end inside a warp's second one; with a bias and 32-bit rows, the activation and the

@@ -492,9 +492,11 @@ gemm_skinny_ring_kernel(const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// Three rounds of blocks at least, two slices of K a warp.
+// Three rounds of blocks at least, two slices of K a warp, and of the second slices three in eight at least: with fewer every block
+// is a slice of nothing longer (16,384 x 1,032 with norm and SwiGLU: 11.9 us, the form above 10.0; 7,120 x 1,152 6.1 and 5.4;
+// 11,856 x 1,280 with SwiGLU 8.0 and 7.3; 9,504 x 1,408 6.7 and 7.0, plain 6.3 and 7.2).
 bool ring_takes(int N, int K) {
-    return N > 3 * 148 * ROWS && K > RING_WARPS * KSLICE && K <= RING_SX * RING_WARPS * KSLICE;
+    return N > 3 * 148 * ROWS && 8 * K >= 11 * RING_WARPS * KSLICE && K <= RING_SX * RING_WARPS * KSLICE;
 }
 
 template <typename TO, int EPI, bool NORM>
