@@ -156,7 +156,7 @@ def test_gemm_float32_is_not_tf32():
 
 
 @pytest.mark.parametrize("m, n, k", [(9, 256, 256), (33, 257, 1000), (64, 1024, 1024), (100, 1024, 4608), (129, 300, 2048),
-                                     (300, 260, 516), (513, 257, 260)])
+                                     (300, 260, 516), (513, 257, 260), (2565, 1030, 260)])
 def test_gemm_32_bit_operands_in_parts(m, n, k):
     """The tensor-core form of the 32-bit product at every width of its token tile, split along K and not, with partial tiles
     and chunks: no further from 64 bits than a few 2^-24 (tf32 operands would be off by 2^-11); infinities and NaN end up

@@ -308,8 +308,13 @@ TK_API int tk_gemm_split32(const void* x, int64_t ldx, const void* w, int64_t ld
     TK_CHECK_ARG(K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0,
                  "gemm_split32: K and the leading dimensions must be multiples of 4, bases 16-byte aligned");
     TK_CHECK_ARG((N + SP_BM - 1) / SP_BM <= 65535, "gemm_split32: N=%d", N);
-    const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
-    const int tiles = ceil_div(M, BN) * ceil_div(N, SP_BM), groups = ceil_div(K, SP_KC * SP_GROUP);
+    const int groups = ceil_div(K, SP_KC * SP_GROUP);
+    // more than 128 tokens in tiles of 256, but for a K too short to be split while tiles of 128 all run at once: those tiles
+    // are the only way to more of the GPU then (256 to 1,000 x 300 x 300: 22.9 us in tiles of 256, gemm_simt.cu 21.3, 15.0 in
+    // tiles of 128; from 129 x 256 x 384 to 2,048 x 1,000 x 256 26.3 to 63.1 there, 15.6 and 13.0 here)
+    const bool small = groups < 4 && ceil_div(M, 128) * ceil_div(N, SP_BM) <= 148;
+    const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 || small ? 128 : 256;
+    const int tiles = ceil_div(M, BN) * ceil_div(N, SP_BM);
     // K is split while the CTAs fill no more than the GPU (two of them an SM up to 64 tokens) and each keeps 256 columns
     const int room = BN <= 64 ? 2 * 148 : 148;
     int splitk = 1;
