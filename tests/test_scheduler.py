@@ -410,3 +410,22 @@ def test_a_recorded_step_has_the_tile_lists_of_its_own_size(monkeypatch):
     assert steps.step_graph_for([st.StepEntry("r", [1] * 1500, [1499])]) is graphs[1500]
     monkeypatch.setattr(steps, "decode_graph", lambda rows: steps._graphs.setdefault(rows, None))
     assert steps.capture_shapes(1, 2048, 1)[1] == len(st.STEP_TOKEN_BUCKETS[:7])
+
+
+def test_state_space_scan_by_chunks_while_the_walk_leaves_places_free():
+    """The walk's length over its places, against a place-by-place count, and the choice it leads to."""
+    from tokenomos_b200 import ops
+    rng = random.Random(4)
+    for _ in range(50):
+        lens = [rng.choice((0, 1, 5, 40, 300)) for _ in range(rng.randint(1, 6))]
+        blocks, places = rng.randint(1, 12), rng.randint(1, 20)
+        free = [0] * places
+        for n in lens:
+            for _ in range(blocks if n else 0):
+                i = free.index(min(free))
+                free[i] += n
+        assert ops.ssd_walk_tokens(lens, blocks, places) == max(free)
+    f = ops.ssd_by_chunks
+    assert f(2048, 32, 64, [2048]) and f(2048, 64, 64, [2048]) and f(2048, 112, 64, [2048]) and not f(2048, 128, 64, [2048])
+    assert f(2050, 64, 64, [2000, 20, 20, 10]) and not f(4096, 64, 64, [1024] * 4) and not f(1000, 64, 64, [500, 500])
+    assert f(1000, 80, 64, [500, 500]) and f(2048, 64, 64) and not f(2048, 128, 64)

@@ -306,8 +306,8 @@ TK_API int tk_ssd_scan(const void* xbc, int64_t xbc_stride, const float* dt_raw,
 }
 
 // The same recurrence chunk by chunk (chunked.cuh): float32 words of scratch it needs, 0 where it does not take the sizes or
-// the walk is the better way. The walk's time is its longest sequence's (0.19 us a token) until the sequences fill the GPU,
-// the chunks' that of all tokens together. 32 heads of 64 x 128, chunks against walk: one sequence of 200 tokens 50 us
+// the walk is the better way at any number of heads (ops.ssd_by_chunks asks how far they fill the GPU). The walk's time is its
+// longest sequence's (0.19 us a token) until the sequences fill the GPU, the chunks' that of all tokens together. 32 heads of 64 x 128, chunks against walk: one sequence of 200 tokens 50 us
 // against 44, of 700 72 against 139, of 2,048 142 against 396; four of 256 94 against 74, of 512 about equal; sixteen of 128
 // 200 against 132. So the line lies at 256 tokens a sequence and 64 more for every one; and at 512 MB of scratch.
 TK_API int tk_ssd_chunked_scratch(int tokens, int n_seqs, int H, int V, int N, int G) {

@@ -8,6 +8,8 @@ path (the plain implementation under ``tests/`` is the oracle, not a fallback).
 
 from __future__ import annotations
 
+import heapq
+
 import torch
 
 from tokenomos_b200.ops import _lib
@@ -1566,16 +1568,46 @@ def mlstm_norm_gate(num: torch.Tensor, m: torch.Tensor, m_state: torch.Tensor, w
 SSD_MAX_STATE = 256
 
 
+def ssd_walk_tokens(seq_lens: list[int], blocks: int, resident: int) -> int:
+    """How many tokens the state-space walk is long: ``blocks`` blocks a sequence, taken in order by whichever of ``resident``
+    places is free."""
+    free, end = [(0, resident)], 0                 # (when, how many places)
+    for n in seq_lens:
+        left = blocks if n else 0
+        while left:
+            at, places = heapq.heappop(free)
+            took = min(places, left)
+            heapq.heappush(free, (at + n, took))
+            if places > took:
+                heapq.heappush(free, (at, places - took))
+            left, end = left - took, max(end, at + n)
+    return end
+
+
+def ssd_by_chunks(tokens: int, heads: int, v_dim: int, seq_lens: list[int] | None = None, sm_count: int = 148) -> bool:
+    """Whether the chunks are the better way as far as the walk's blocks (one per 32 columns, head and sequence) fill the GPU:
+    the chunks' time is that of all tokens, the walk's that of its longest chain, and a token of one block in the chunks is a
+    240th of a token's time in the walk, whatever the head's size (measured at 8 to 128 heads of 64 x 64, 64 x 128 and 128 x
+    128, one to four sequences of 320 to 4,096 tokens: no choice slower than the other way by more than 4 %; 128 heads on 320
+    to 2,048 tokens, us with the norm behind it: chunks 122, 187, 733, walk 114, 171, 728; 64 heads, portions of 2,000, 20,
+    20 and 10 tokens 300 against 546, four of 1,024 553 against 557). ``seq_lens`` None (a recorded step, which is replayed
+    for any lengths): as if one portion had them all."""
+    blocks = -(-int(v_dim) // 32) * int(heads)
+    walk = int(tokens) if seq_lens is None else ssd_walk_tokens(seq_lens, blocks, 2 * sm_count)
+    return blocks * int(tokens) <= 240 * walk
+
+
 def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, cu_seqlens: torch.Tensor, seq_ctx: torch.Tensor, seq_slot: torch.Tensor, n_seqs: int,
-             heads: int, v_dim: int, n_state: int, groups: int, sm_count: int = 148) -> torch.Tensor:
+             heads: int, v_dim: int, n_state: int, groups: int, sm_count: int = 148,
+             seq_lens: list[int] | None = None) -> torch.Tensor:
     """The state-space recurrence over a step's tokens: ``dt = softplus(dt_raw + dt_bias)``, ``S_t = exp(-exp(a_log)
     dt) S_(t-1) + dt B_t x_t^T``, ``y_t = S_t^T C_t + d_skip x_t`` per head. ``xbc`` [T, >= heads v_dim + 2 groups
     n_state] (rows may be strided): x, then B, then C; ``dt_raw`` float32 [T, >= heads]; ``state`` float32 [slots,
     heads, n_state, v_dim]. Returns ``y`` float32 [parts, T, heads v_dim]: a step of few, long portions is walked
     by several blocks a head, each over a part of the state's rows, and their sums are still to be added
     (``gated_group_norm`` does; ``y.sum(0)`` is the result). Few, long portions of states the chunked kernels take are formed
-    chunk by chunk instead (one part)."""
+    chunk by chunk instead (one part; ``ssd_by_chunks``). ``seq_lens``: the portions' lengths, where the host knows them."""
     _cuda(xbc, dt_raw, dt_bias, a_log, d_skip, state)
     T = xbc.shape[0]
     if xbc.stride(1) != 1 or xbc.shape[1] < heads * v_dim + 2 * groups * n_state:
@@ -1585,7 +1617,8 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, n_state, v_dim) or not state.is_contiguous():
         raise KernelError(f"ssd_scan: the state is float32 [slots, {heads}, {n_state}, {v_dim}]")
     words = _lib.call("tk_ssd_chunked_scratch", T, int(n_seqs), heads, v_dim, n_state, groups)
-    if words and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0:
+    if (words and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0
+            and ssd_by_chunks(T, heads, v_dim, seq_lens, sm_count)):
         # portions of some length: chunk by chunk, all side by side
         scratch = torch.empty(words, dtype=torch.float32, device=xbc.device)
         y = torch.empty(1, T, heads * v_dim, dtype=torch.float32, device=xbc.device)

@@ -76,7 +76,7 @@ class StateSpaceDuality:
                            proj.dtype, act=True)
         y = ops.ssd_scan(xbc, dt, self.dt_bias, self.a_log, self.d_skip, ctx.states[(call, "S")], ctx.cu_seqlens,
                          ctx.seq_ctx, ctx.seq_slot, ctx.n_seqs, self.heads, self.v_dim, self.state, self.groups,
-                         self.sm_count)
+                         self.sm_count, None if ctx.host.captured else ctx.host.seq_lens)
         out = ops.gated_group_norm(y, proj[:, :self.inner], self.norm, self.eps, self.norm_groups)
         return self.out_proj(out)
 
