@@ -891,15 +891,23 @@ def test_trace_program_and_command_line(folders, tmp_path):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("H, K, D, V, lens, ctx", [(4, 2, 128, 128, (300, 1, 33, 16, 177), (0, 5, 9, 0, 3)), (2, 1, 64, 40, (121,), (7,)),
-                                                   (2, 2, 200, 24, (0, 96, 0, 130), (0, 0, 0, 2)), (3, 3, 24, 24, (47, 18), (0, 4))])
-def test_delta_rule_two_tokens_a_step(H, K, D, V, lens, ctx, dtype):
+@pytest.mark.parametrize("H, K, D, V, lens, ctx, pairs", [
+    (4, 2, 128, 128, (300, 1, 33, 16, 177), (0, 5, 9, 0, 3), False), (2, 1, 64, 40, (121,), (7,), False),
+    (2, 2, 200, 24, (0, 96, 0, 130), (0, 0, 0, 2), False), (3, 3, 24, 24, (47, 18), (0, 4), False),
+    (2, 1, 128, 128, (277,), (3,), True), (4, 2, 128, 40, (143, 301, 32), (5, 0, 2), True), (2, 2, 96, 96, (161, 1, 240), (0, 7, 2), True),
+    (4, 2, 64, 40, (303, 33, 177), (0, 9, 0), True), (3, 3, 24, 24, (250, 0, 145), (0, 4, 1), True)])
+def test_delta_rule_two_tokens_a_step(H, K, D, V, lens, ctx, pairs, dtype):
     """The delta rule with a decay per head over portions that begin on odd rows and end inside a stage of 16 tokens and on its
-    edge, at every register form of a column: against the recurrence in 64-bit from the same rows, decays from 1 to e^-40 a
+    edge, at every register form of a column, token by token and in pairs (whose scratch holds two more floats a token and
+    q/k head): against the recurrence in 64-bit from the same rows, decays from 1 to e^-40 a
     token among them, sums of up to 200 products in 32-bit; a token that is not finite reaches none before it."""
     from tokenomos_b200 import ops
     g = torch.Generator().manual_seed(7)
     T, S = sum(lens), len(lens)
+    padded = 32 if D <= 32 else 64 if D <= 64 else 128 if D <= 128 else 256
+    walk = (T + 16) * (2 * K * padded + H * (-(-V // 4) * 4 + 4))
+    scratch = ops._lib.call("tk_linmem_scratch", T, S, H, K, D, V, ops.LINMEM_DECAYS["head"], 148)
+    assert scratch == -(-(walk + (T + 16) * 2 * K * pairs) // 32)
     nk, nv = K * D, H * V
     u = torch.randn(T, 2 * nk + nv + 4, generator=g).to(getattr(torch, dtype))
     zb, za = torch.randn(T, H + 4, generator=g), torch.randn(T, H + 4, generator=g) - 1.0
@@ -935,7 +943,6 @@ def test_delta_rule_two_tokens_a_step(H, K, D, V, lens, ctx, dtype):
         if lens[s]:
             after[slots[s]] = M
     err = (got.double().cpu().view(T, H, V) - want).norm() / want.norm()
-    print(f"pairs {dtype} {D}x{V}: {err:.2e}")
     assert err <= 1e-6, err
     assert (st.double().cpu() - after).norm() <= 1e-6 * after.norm()
     last = max(range(S), key=lambda s: lens[s])

@@ -36,15 +36,18 @@ constexpr int LM_SEG = 256;      // tokens of a segment (whole stages)
 
 enum : int { LM_ADD = 0, LM_DELTA = 1 };
 enum : int { LM_FIXED = 0, LM_HEAD = 1, LM_CHANNEL = 2 };
-// Whether the walk may take two tokens a step (lm_pair), and whether it does: up to eight sequences of keys up to 64, where the
-// path from token to token bounds it (16 heads of 64 x 64, one sequence of 2,048 tokens: 282 us, 353 token by token; more
-// sequences hide the path from each other, 16 of 128: 64 us against 62). Keys up to 128 are bound by the multiply-adds of a
-// block (16 heads of 128 x 128: 406 and 410), until one column a thread spreads them over twice the SMs: while those blocks
-// are no more than the SMs (one sequence of 2,048 tokens 319 us; two of 1,024 243 against 219).
+// Whether the walk may take two tokens a step (lm_pair), and whether it does: keys up to 64 and at most 128 heads over all
+// sequences, where the path from token to token bounds it (16 heads of 64 x 64, one sequence of 2,048 tokens: 281 us, 350
+// token by token, eight of 128 37 and 38; more heads hide the path from each other, 32 in eight sequences of 512: 266 against
+// 237, 64 in four of 300 131 and 128). Keys up to 128 are bound by the multiply-adds of a block (16 heads of 128 x 128: 406
+// and 410), until one column a thread spreads them over twice the SMs: while those blocks are no more than the SMs (one
+// sequence of 2,048 tokens 319 us; two of 1,024 243 against 219). What the token before leaves in each token's keys is formed
+// beforehand, which portions of 128 tokens and up to 64 q/k heads over all sequences pay back (one sequence of 8 tokens 8.8 us
+// against 7.8; 32 q/k heads of 64 on 33 tokens 18.0 against 15.5, on 100 27.4 and 26.8, on 300 55 and 61).
 constexpr bool LM_PAIRS(int rule, int decay) { return rule == LM_DELTA && decay == LM_HEAD; }
-inline bool lm_pairs(int decay, int n_seqs, int H, int D, int V, int sm_count) {
-    if (decay != LM_HEAD || D > 128) return false;
-    return D <= 64 ? n_seqs <= 8 : (V + 15) / 16 * H * n_seqs <= sm_count;
+inline bool lm_pairs(int decay, int tokens, int n_seqs, int H, int K, int D, int V, int sm_count) {
+    if (decay != LM_HEAD || D > 128 || tokens < 128 * n_seqs || K * n_seqs > 64) return false;
+    return D <= 64 ? H * n_seqs <= 128 : (V + 15) / 16 * H * n_seqs <= sm_count;
 }
 
 struct LinMem {
@@ -750,7 +753,7 @@ void lm_launch(const LinMem& m, int n_seqs, int tokens, float* scratch, int sm_c
     p.v = p.kq + (size_t)m.K * p.rows * 2 * DP;
     p.sc = reinterpret_cast<float4*>(p.v + (size_t)m.H * p.rows * p.VP);
     p.g = reinterpret_cast<float*>(p.sc + (size_t)m.H * p.rows);
-    p.near = LM_PAIRS(RULE, DECAY) && lm_pairs(DECAY, n_seqs, m.H, m.D, m.V, sm_count) ? reinterpret_cast<float2*>(p.g) : nullptr;      // (a decay per head stages none per channel)
+    p.near = LM_PAIRS(RULE, DECAY) && lm_pairs(DECAY, tokens, n_seqs, m.H, m.K, m.D, m.V, sm_count) ? reinterpret_cast<float2*>(p.g) : nullptr;      // (a decay per head stages none per channel)
     p.seg = nullptr;
     p.n_seqs = n_seqs;
     tk_launch(linmem_prepare_kernel<T, R / 4, RULE, DECAY>, dim3(tokens), dim3(256),
@@ -826,7 +829,7 @@ TK_API int tk_linmem_scratch(int tokens, int n_seqs, int H, int K, int D, int V,
     if (tokens < 4 * n_seqs || n_seqs == 0) return 0;
     const int64_t DP = D <= 32 ? 32 : D <= 64 ? 64 : D <= 128 ? 128 : 256, VP = (V + 3) / 4 * 4;
     const int64_t floats = (int64_t)(tokens + LM_TOK) * (2 * K * DP + H * (VP + 4) + (decay == LM_CHANNEL ? H * DP : 0) +
-                                                      (lm_pairs(decay, n_seqs, H, D, V, sm_count) ? 2 * K : 0)) +
+                                                      (lm_pairs(decay, tokens, n_seqs, H, K, D, V, sm_count) ? 2 * K : 0)) +
                            (int64_t)lm_slots(tokens, n_seqs, H, D, V, decay, sm_count) * H * V * D;
     return (int)((floats + 31) / 32);
 }
