@@ -335,7 +335,9 @@ __device__ __forceinline__ LmSegment lm_segment(const LinMem& m, int n_seqs, int
     return g;
 }
 
-template <typename T, int DPL, int RULE, int DECAY>
+// NEAR: for pairs of tokens (a form of its own: its registers would cost the other one a quarter of the warps an SM holds, 202 us
+// against 194 for 64 heads of 64 x 64 in sixteen portions of 128).
+template <typename T, int DPL, int RULE, int DECAY, bool NEAR>
 __global__ void __launch_bounds__(256)
 linmem_prepare_kernel(const LinMem m, const LinMemPrep p) {
     constexpr int DP = 32 * DPL;
@@ -359,7 +361,7 @@ linmem_prepare_kernel(const LinMem m, const LinMemPrep p) {
             lm_fetch_partners<T, DPL>(m, t, kh * (m.H / m.K), lane, kp, qp);
             lm_rotate<DPL>(m, lane, cs, kv, qv, kp, qp);
         }
-        if (LM_PAIRS(RULE, DECAY) && p.near != nullptr) {
+        if constexpr (NEAR) {
             // (the first token of the step has none before it, and no pair reaches across a sequence's start)
             float kb[DPL], unused[DPL], skb = 0.f, kk = 0.f, qk = 0.f, sk = 0.f, sq = 0.f;
             lm_fetch<T, DPL>(m, max(t - 1, 0), kh * (m.H / m.K), lane, kb, unused);
@@ -753,11 +755,14 @@ void lm_launch(const LinMem& m, int n_seqs, int tokens, float* scratch, int sm_c
     p.v = p.kq + (size_t)m.K * p.rows * 2 * DP;
     p.sc = reinterpret_cast<float4*>(p.v + (size_t)m.H * p.rows * p.VP);
     p.g = reinterpret_cast<float*>(p.sc + (size_t)m.H * p.rows);
-    p.near = LM_PAIRS(RULE, DECAY) && lm_pairs(DECAY, tokens, n_seqs, m.H, m.K, m.D, m.V, sm_count) ? reinterpret_cast<float2*>(p.g) : nullptr;      // (a decay per head stages none per channel)
+    const bool pairs = LM_PAIRS(RULE, DECAY) && lm_pairs(DECAY, tokens, n_seqs, m.H, m.K, m.D, m.V, sm_count);
+    p.near = pairs ? reinterpret_cast<float2*>(p.g) : nullptr;      // (a decay per head stages none per channel)
     p.seg = nullptr;
     p.n_seqs = n_seqs;
-    tk_launch(linmem_prepare_kernel<T, R / 4, RULE, DECAY>, dim3(tokens), dim3(256),
-              (m.K + 2 * m.half) * sizeof(float), stream, m, p);
+    auto prepare = linmem_prepare_kernel<T, R / 4, RULE, DECAY, false>;
+    if constexpr (LM_PAIRS(RULE, DECAY) && R <= 16)
+        if (pairs) prepare = linmem_prepare_kernel<T, R / 4, RULE, DECAY, true>;
+    tk_launch(prepare, dim3(tokens), dim3(256), (m.K + 2 * m.half) * sizeof(float), stream, m, p);
     // Two columns a thread (one where a column alone is 32 registers) in blocks of four warps; eight warps, which share
     // a stage's copies among more columns, only where even a quarter of the sequences (the least a recorded step of
     // this shape was recorded for) would fill the GPU with them
@@ -791,7 +796,7 @@ void lm_launch(const LinMem& m, int n_seqs, int tokens, float* scratch, int sm_c
         }
     }
     if constexpr (LM_PAIRS(RULE, DECAY) && R <= 16) {
-        if (p.near != nullptr) {
+        if (pairs) {
             constexpr int PC = R == 16 ? 1 : CPT;
             int pw = R == 16 ? 4 : warps;
             while (pw > 1 && m.V <= LM_COLS * PC * pw / 2) pw /= 2;
