@@ -429,3 +429,14 @@ def test_state_space_scan_by_chunks_while_the_walk_leaves_places_free():
     assert f(2048, 32, 64, [2048]) and f(2048, 64, 64, [2048]) and f(2048, 112, 64, [2048]) and not f(2048, 128, 64, [2048])
     assert f(2050, 64, 64, [2000, 20, 20, 10]) and not f(4096, 64, 64, [1024] * 4) and not f(1000, 64, 64, [500, 500])
     assert f(1000, 80, 64, [500, 500]) and f(2048, 64, 64) and not f(2048, 128, 64)
+
+
+def test_sequence_convolution_takes_four_channels_a_thread_where_they_fill_the_gpu():
+    from tokenomos_b200 import ops
+    f = lambda T, C, K, dtype=torch.bfloat16, single=False: ops.seq_conv_plan(  # noqa: E731
+        torch.empty(T, C, dtype=dtype, device="meta"), torch.empty(C, K, device="meta"), 16, single)
+    assert f(64, 4096, 4) == (16, False) and f(2048, 256, 4) == (16, False) and f(300, 1024, 2) == (16, False)
+    assert f(300, 3072, 4) == (16, True) and f(2048, 512, 3) == (16, True) and f(2048, 6144, 4) == (32, True)
+    assert f(1, 64, 4, single=True) == (16, True) and f(64, 4096, 4, single=True) == (16, True)
+    assert f(2048, 6144, 5) == (32, False) and f(2048, 6144, 1) == (32, False)
+    assert f(2048, 6144, 4, torch.float32) == (ops.seq_conv_tile(16, 2048, 6144), False)

@@ -138,7 +138,8 @@ seq_conv_kernel(const TI* in, int64_t in_stride, const float* __restrict__ taps,
 
 // The same for bfloat16 rows that all go to `out`, four neighbouring channels a thread (8 bytes a load and a store, K known so
 // that the taps and the past of all four stay in registers), the same sums in the same order. The form above moves two bytes
-// a thread and load: 2,048 tokens of 3,072 channels take it 28.1 us (25 MB), this one 17.6; 3,000 of 4,096 53 and 31.
+// a thread and load: 2,048 tokens of 3,072 channels take it 28.1 us (25 MB), this one 17.6; 3,000 of 4,096 53 and 31. A quarter
+// of the threads walk as long a tile: the caller says where they are enough (ops.seq_conv_plan).
 template <int K>
 __global__ void __launch_bounds__(128)
 seq_conv_quad_kernel(const __nv_bfloat16* in, int64_t in_stride, const float* __restrict__ taps, const float* __restrict__ bias,
@@ -224,13 +225,14 @@ seq_conv_quad_kernel(const __nv_bfloat16* in, int64_t in_stride, const float* __
 // in: [T, >= C] with row stride in_stride (type in_dtype); taps float32 [C, K]; bias float32 [C] or
 // null; state float32 [slots, K - 1, C] (null with K == 1); tiles: runs of one sequence's
 // consecutive tokens, each at least K - 1 long but for a portion's last; out: [T, >= c_paged or C]
-// (type out_dtype), plain likewise or null; pool (type out_dtype) null: every channel goes to out.
+// (type out_dtype), plain likewise or null; pool (type out_dtype) null: every channel goes to out. quad: four channels a thread
+// where that form takes the call.
 TK_API int tk_seq_conv(const void* in, int64_t in_stride, int in_dtype, const float* taps, const float* bias,
                        float* state, const int* cu_seqlens, const int* seq_ctx, const int* seq_slot,
                        const int* tile_seq, const int* tile_tok0, const int* tile_off, const int* tile_n,
                        int n_tiles, void* out, int64_t out_stride, void* plain, int64_t plain_stride, int out_dtype,
-                       int K, int C, int residual, int act, int c_paged, void* pool, const int* block_table,
-                       int bt_stride, int P, int Hkv, int Dk, int Dv, int Dp, cudaStream_t stream) {
+                       int K, int C, int residual, int act, int quad, int c_paged, void* pool,
+                       const int* block_table, int bt_stride, int P, int Hkv, int Dk, int Dv, int Dp, cudaStream_t stream) {
     TK_CHECK_ARG(K >= 1 && K <= MAX_TAPS, "sequence conv: %d taps; 1..%d are built", K, MAX_TAPS);
     TK_CHECK_ARG(K == 1 || state != nullptr, "sequence conv: %d taps need a state", K);
     TK_CHECK_ARG(C > 0 && n_tiles >= 0, "sequence conv: bad sizes");
@@ -245,7 +247,7 @@ TK_API int tk_seq_conv(const void* in, int64_t in_stride, int in_dtype, const fl
     TK_CHECK_ARG(out != nullptr || c_paged == 0, "sequence conv: no output");
     if (n_tiles == 0) return 0;
     PagedDest dest{pool, block_table, bt_stride, P, Hkv, Dk, Dv, Dp};
-    if (in_dtype == TK_BF16 && out_dtype == TK_BF16 && pool == nullptr && plain == nullptr && K >= 2 && K <= 4 && C % 4 == 0 &&
+    if (quad && in_dtype == TK_BF16 && out_dtype == TK_BF16 && pool == nullptr && plain == nullptr && K >= 2 && K <= 4 && C % 4 == 0 &&
         in_stride % 4 == 0 && out_stride % 4 == 0 && (uintptr_t)in % 8 == 0 && (uintptr_t)out % 8 == 0 &&
         (uintptr_t)state % 16 == 0 && (uintptr_t)bias % 16 == 0) {
 #define TK_SCQ(KV)                                                                                                         \

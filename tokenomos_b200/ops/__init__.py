@@ -1357,13 +1357,29 @@ _SEQ_CONV_RESIDENT = 148 * 4      # blocks of the sequence convolution that run 
 def seq_conv_tile(base: int, tokens: int, channels: int, quad: bool = False) -> int:
     """The tile length for ``seq_conv`` on a step of ``tokens`` tokens: ``base``, doubled (up to 128)
     while the tiles of all channel blocks would not run at once. A thread walks its tile in order,
-    so short tiles are quick, but a second wave of blocks costs more than a longer walk. ``quad``: for bfloat16 rows that
-    the four-channel form takes (blocks of 512 channels in 128 threads, ten an SM)."""
+    so short tiles are quick, but a second wave of blocks costs more than a longer walk. ``quad``: for bfloat16 rows, whose
+    four-channel form has blocks of 512 channels in 128 threads, ten an SM (the other form is no slower for it: five taps over
+    2,048 tokens of 3,072 channels 24 us, 37 in the tiles of the rule without it)."""
     tile = max(int(base), 1)
     blocks, resident = (-(-int(channels) // 512), 148 * 10) if quad else (-(-int(channels) // 256), _SEQ_CONV_RESIDENT)
     while tile < 128 and -(-int(tokens) // tile) * blocks > resident:
         tile *= 2
     return tile
+
+
+SEQ_CONV_QUAD_FILL = 49152        # channels of all tiles from which on the four-channel form is the quicker one
+
+
+def seq_conv_plan(u: torch.Tensor, taps: torch.Tensor, base: int, single: bool) -> tuple[int, bool]:
+    """The tile length for ``seq_conv`` on ``u`` [T, C], and whether four channels a thread (``quad``) are the better way: with
+    bfloat16 rows and two to four taps, where every sequence brings one token (``single``; 64 of 3,072 channels 5.9 us, 7.4 one
+    channel a thread), else from 49,152 channels over all tiles on, below which a quarter of the threads leaves the walk of a
+    tile in the open (64 tokens of 4,096 channels 8.2 us against 7.1, 2,048 of 256 7.9 against 6.9, 1,600 of 512 8.2 against
+    8.1, 1,000 of 1,024 8.3 against 9.0, 2,048 of 3,072 16.0 against 36.6)."""
+    T, C = u.shape
+    half = u.dtype == torch.bfloat16
+    tile = seq_conv_tile(base, T, C, half)
+    return tile, half and 2 <= taps.shape[1] <= 4 and (single or -(-T // tile) * C >= SEQ_CONV_QUAD_FILL)
 
 
 MATRIX_MEMORY_MAX_DIM = 256
@@ -1384,12 +1400,13 @@ def scale_rows_f32(x: torch.Tensor, scale: float) -> torch.Tensor:
 def seq_conv(u: torch.Tensor, taps: torch.Tensor, bias: torch.Tensor | None, state: torch.Tensor | None,
              cu_seqlens: torch.Tensor, seq_ctx: torch.Tensor, seq_slot: torch.Tensor, tiles: tuple,
              out_dtype: torch.dtype, residual: bool = False, plain: bool = False, out_channels: int | None = None,
-             kv: tuple | None = None, act: bool = False):
+             kv: tuple | None = None, act: bool = False, quad: bool = True):
     """Causal convolution over time on each channel: ``y_t = [u_t +] bias + sum_j taps[:, j] u_(t - K + 1 + j)``
     within each sequence (zeros before its start). ``u`` [T, C] (rows may be strided), ``taps`` float32
     [C, K]; the last K - 1 rows of ``u`` of every sequence are kept in ``state`` (float32
     [slots, K - 1, C]). ``tiles``: ``ctx.tiles(size)`` with size >= K - 1. ``plain``: also returns ``u``
-    itself in ``out_dtype``. ``act``: ``y <- silu(y)``. ``kv`` = ``(pool, block_table, page, kv_heads, k_dim, v_dim)``: the
+    itself in ``out_dtype``. ``act``: ``y <- silu(y)``. ``quad``: four channels a thread where the kernel has that form
+    (``seq_conv_plan``; the bits are the same). ``kv`` = ``(pool, block_table, page, kv_heads, k_dim, v_dim)``: the
     channels from ``out_channels`` on are ``kv_heads`` key heads then as many value heads and go into
     the paged pool at each token's position instead of the result."""
     _cuda(u, taps, bias, state, cu_seqlens, seq_ctx, seq_slot, *tiles)
@@ -1421,7 +1438,7 @@ def seq_conv(u: torch.Tensor, taps: torch.Tensor, bias: torch.Tensor | None, sta
               _ptr(_i32(cu_seqlens, "cu_seqlens")), _ptr(_i32(seq_ctx, "seq_ctx")), _ptr(_i32(seq_slot, "seq_slot")),
               _ptr(_i32(seq, "tile_seq")), _ptr(_i32(tok0, "tile_tok0")), _ptr(_i32(off, "tile_off")),
               _ptr(_i32(n, "tile_n")), seq.numel(), _ptr(out), n_out, _ptr(same), n_out, code[out_dtype], K, C,
-              int(bool(residual)), int(bool(act)), n_out, _ptr(pool), _ptr(table), bt, int(P), int(hkv), int(dk), int(dv), int(dp),
+              int(bool(residual)), int(bool(act)), int(bool(quad)), n_out, _ptr(pool), _ptr(table), bt, int(P), int(hkv), int(dk), int(dv), int(dp),
               _stream())
     return (out, same) if plain else out
 

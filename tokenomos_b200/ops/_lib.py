@@ -99,7 +99,7 @@ _SIGNATURES = {
     "tk_moe_combine": [P, P, P, P, P, P, I, I, I, I, P],
     "tk_relu2": [P, L, I, P],
     "tk_scale_rows_f32": [P, L, P, F, I, I, I, P],
-    "tk_seq_conv": [P, L, I, P, P, P, P, P, P, P, P, P, P, I, P, L, P, L, I, I, I, I, I, I, P, P, I, I, I, I, I, I, P],
+    "tk_seq_conv": [P, L, I, P, P, P, P, P, P, P, P, P, P, I, P, L, P, L, I, I, I, I, I, I, I, P, P, I, I, I, I, I, I, P],
     "tk_attn_pointwise_rows": [],
     "tk_attn_pointwise": [P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, F, F, F, I, P, P, P, I, P],
     "tk_attn_pointwise_mma_supported": [I, I, I, I, I],

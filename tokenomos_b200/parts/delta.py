@@ -87,12 +87,13 @@ class GatedDelta:
         return specs
 
     def forward(self, x: torch.Tensor, ctx: StepContext, call: int) -> torch.Tensor:
-        T, C, H = x.shape[0], self.channels, self.heads
+        C, H = self.channels, self.heads
         nk = self.kv_heads * self.dim
         proj = self.in_proj(x)
         z = self.gate_proj(x, out_dtype=torch.float32)
+        tile, quad = ops.seq_conv_plan(proj[:, :C], self.taps, self.tile, ctx.host.decode_only)
         u = ops.seq_conv(proj[:, :C], self.taps, None, ctx.states.get((call, "conv")), ctx.cu_seqlens, ctx.seq_ctx,
-                         ctx.seq_slot, ctx.tiles(ops.seq_conv_tile(self.tile, T, C, proj.dtype == torch.bfloat16)), proj.dtype, act=True)
+                         ctx.seq_slot, ctx.tiles(tile), proj.dtype, act=True, quad=quad)
         if self.decay == "channel":
             n = C + self.decay_up.in_features
             decay = self.decay_up(proj[:, C:n], out_dtype=torch.float32)

@@ -68,8 +68,9 @@ class GatedLinearRecurrence:
     def forward(self, x: torch.Tensor, ctx: StepContext, call: int) -> torch.Tensor:
         W, T = self.width, x.shape[0]
         proj = self.in_proj(x)                                    # [T, y | x]
-        u = ops.seq_conv(proj[:, W:], self.conv, self.conv_bias, ctx.states.get((call, "conv")), ctx.cu_seqlens,
-                         ctx.seq_ctx, ctx.seq_slot, ctx.tiles(ops.seq_conv_tile(self.tile, T, W)), proj.dtype)
+        tile, quad = ops.seq_conv_plan(proj[:, W:], self.conv, self.tile, ctx.host.decode_only)
+        u = ops.seq_conv(proj[:, W:], self.conv, self.conv_bias, ctx.states.get((call, "conv")), ctx.cu_seqlens, ctx.seq_ctx,
+                         ctx.seq_slot, ctx.tiles(tile), proj.dtype, quad=quad)
         ub = u.view(T, self.blocks, W // self.blocks).transpose(0, 1)          # [blocks, T, w]
         if u.dtype == torch.float32:
             z = ops.gemm_batched(ub, self.gates)                               # 32-bit FMA

@@ -67,13 +67,12 @@ class StateSpaceDuality:
         return specs
 
     def forward(self, x: torch.Tensor, ctx: StepContext, call: int) -> torch.Tensor:
-        T = x.shape[0]
         proj = self.in_proj(x)                                        # [T, z | x B C]
         dt = self.dt_proj(x, out_dtype=torch.float32)
-        xbc = ops.seq_conv(proj[:, self.inner:], self.conv, self.conv_bias, ctx.states.get((call, "conv")),
-                           ctx.cu_seqlens, ctx.seq_ctx, ctx.seq_slot,
-                           ctx.tiles(ops.seq_conv_tile(self.tile, T, self.channels, proj.dtype == torch.bfloat16)),
-                           proj.dtype, act=True)
+        rows = proj[:, self.inner:]
+        tile, quad = ops.seq_conv_plan(rows, self.conv, self.tile, ctx.host.decode_only)
+        xbc = ops.seq_conv(rows, self.conv, self.conv_bias, ctx.states.get((call, "conv")), ctx.cu_seqlens, ctx.seq_ctx,
+                           ctx.seq_slot, ctx.tiles(tile), proj.dtype, act=True, quad=quad)
         y = ops.ssd_scan(xbc, dt, self.dt_bias, self.a_log, self.d_skip, ctx.states[(call, "S")], ctx.cu_seqlens,
                          ctx.seq_ctx, ctx.seq_slot, ctx.n_seqs, self.heads, self.v_dim, self.state, self.groups,
                          self.sm_count, None if ctx.host.captured else ctx.host.seq_lens)
