@@ -385,7 +385,8 @@ gated_group_norm_kernel(const float* y, int parts, const T* z, int64_t z_stride,
 }
 
 // The same four neighbouring elements a lane and step (16 bytes of y, 8 or 16 of z), QUADS of them in registers: rows of 2,048 in
-// four groups, 2,048 tokens (34 MB): 11.2 us, one element at a time 20.8.
+// four groups, 2,048 tokens (34 MB): 11.2 us, one element at a time 20.8. Groups of less than 128 leave lanes without any (rows of
+// 4,096 in groups of 64, 2,048 tokens: 52.8 us against 36.5) and stay with the form above.
 template <typename T, int QUADS>
 __global__ void __launch_bounds__(128)
 gated_group_norm_quad_kernel(const float* y, int parts, const T* z, int64_t z_stride, const float* __restrict__ w, float eps,
@@ -444,7 +445,7 @@ TK_API int tk_gated_group_norm(const float* y, int parts, const void* z, int64_t
     const int warps = rows * groups;
     dim3 grid((warps + 3) / 4), block(128);
     const size_t es = dtype == TK_F32 ? 4 : 2;
-    if (gw % 4 == 0 && gw <= 32 * 16 && z_stride % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)w % 16 == 0 &&
+    if (gw % 4 == 0 && gw >= 128 && gw <= 32 * 16 && z_stride % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)w % 16 == 0 &&
         (uintptr_t)z % (4 * es) == 0 && (uintptr_t)out % (4 * es) == 0 && (dtype == TK_F32 || dtype == TK_BF16)) {
 #define TK_GGQ(TT, QUADS)                                                                                               \
     tk_launch(gated_group_norm_quad_kernel<TT, QUADS>, grid, block, 0, stream, y, parts, (const TT*)z, z_stride, w, eps, \
