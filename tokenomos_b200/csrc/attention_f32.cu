@@ -18,39 +18,11 @@
 // to 64 requests, the general kernel walked a token's keys in one block of 16 rows.
 #include <math.h>
 
-#include "common.cuh"
+#include "packed.cuh"
 
 namespace {
 
 constexpr int F_D = 64, F_ROWS = 64, F_KEYS = 64, F_LD = F_D + 4, F_THREADS = 256;
-
-__device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
-          "l"(reinterpret_cast<unsigned long long&>(c)));
-    return d;
-}
-
-// acc[i][j] += sum over 64 of a[rows ra + i][.] * b[row rb + 16 j][.], both with rows of F_LD floats
-__device__ __forceinline__ void tile_product(const float* a, const float* b, float2 (&acc)[4][4]) {
-#pragma unroll 4
-    for (int k = 0; k < 64; k += 4) {
-        float4 av[4], bv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) av[i] = *reinterpret_cast<const float4*>(a + i * F_LD + k);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = *reinterpret_cast<const float4*>(b + 16 * j * F_LD + k);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc[i][j] = pk_fma(make_float2(av[i].x, av[i].y), make_float2(bv[j].x, bv[j].y), acc[i][j]);
-                acc[i][j] = pk_fma(make_float2(av[i].z, av[i].w), make_float2(bv[j].z, bv[j].w), acc[i][j]);
-            }
-    }
-}
 
 __global__ void __launch_bounds__(F_THREADS, 2)
 attn32_prefill_kernel(const float* q, const float* kv_pool, float* out, const int* positions, const int* tok_seq,
@@ -135,7 +107,7 @@ attn32_prefill_kernel(const float* q, const float* kv_pool, float* out, const in
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) s2[i][j] = make_float2(0.f, 0.f);
-        tile_product(Qs + ty * 4 * F_LD, Ks + tx * F_LD, s2);
+        tile_product<4>(Qs + ty * 4 * F_LD, F_LD, Ks + tx * F_LD, F_LD, F_D, s2);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             float s[4], mx = -INFINITY;
@@ -168,7 +140,7 @@ attn32_prefill_kernel(const float* q, const float* kv_pool, float* out, const in
         }
         __syncwarp();                        // a row's weights are written and read by the same half-warp
         if (!guarded) {
-            tile_product(Ps + ty * 4 * F_LD, Vt + tx * F_LD, o);
+            tile_product<4>(Ps + ty * 4 * F_LD, F_LD, Vt + tx * F_LD, F_LD, F_KEYS, o);
             continue;
         }
         // a weight of zero does not hide a value that is not finite: the keys a row sees, and no others

@@ -24,7 +24,7 @@
 
 #include <math.h>
 
-#include "common.cuh"
+#include "packed.cuh"
 
 namespace {
 
@@ -43,8 +43,7 @@ struct Chunked {
     float* carry;                  // [slots][H][V][N]
     float* chunk_decay;            // [slots][H]
     float* y;                      // [T, H V]
-    float* state;                  // [request slots][H][N][V], or [H][V][N] with state_vn
-    int state_vn;
+    float* state;                  // [request slots][H][N][V]
     int check;                     // the kernel's number in the index checks
 };
 
@@ -64,33 +63,6 @@ struct SsdDecay {
     __device__ __forceinline__ float skip(int h) const { return D_skip[h]; }
 };
 
-__device__ __forceinline__ float2 ch_fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
-          "l"(reinterpret_cast<unsigned long long&>(c)));
-    return d;
-}
-
-// acc[i][j] += sum over k < K of a[i lda + k] b[16 j ldb + k] (K a multiple of 4)
-__device__ __forceinline__ void ch_product(const float* a, int lda, const float* b, int ldb, int K, float2 (&acc)[4][4]) {
-#pragma unroll 2
-    for (int k = 0; k < K; k += 4) {
-        float4 av[4], bv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) av[i] = *reinterpret_cast<const float4*>(a + i * lda + k);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = *reinterpret_cast<const float4*>(b + 16 * j * ldb + k);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc[i][j] = ch_fma2(make_float2(av[i].x, av[i].y), make_float2(bv[j].x, bv[j].y), acc[i][j]);
-                acc[i][j] = ch_fma2(make_float2(av[i].z, av[i].w), make_float2(bv[j].z, bv[j].w), acc[i][j]);
-            }
-    }
-}
 __device__ __forceinline__ void ch_zero(float2 (&acc)[4][4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -120,8 +92,7 @@ __device__ __forceinline__ ChunkAt chunk_at(const Chunked& m, int slot) {
 }
 
 // cum[t]: log of the decays up to and with token t of the chunk; w[t] (0 past the end, where cum stays). By warps 0 and 1.
-template <typename Decay>
-__device__ __forceinline__ void chunk_decays(const Decay& d, const ChunkAt& c, int h, double* cum, float* w) {
+__device__ __forceinline__ void chunk_decays(const SsdDecay& d, const ChunkAt& c, int h, double* cum, float* w) {
     __shared__ double half_s;
     const int t = threadIdx.x, lane = t & 31;
     double la = 0.0;
@@ -185,7 +156,7 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_gram_kernel(const Chunked
     if ((ty & ~1) * 4 >= c.nt) return;
     float2 acc[4][4];
     ch_zero(acc);
-    ch_product(Cs + ty * 4 * ld, ld, Bs + tx * ld, ld, m.N, acc);
+    tile_product<2>(Cs + ty * 4 * ld, ld, Bs + tx * ld, ld, m.N, acc);
     float* out = m.gram + ((size_t)slot * m.groups + g) * CH_T * CH_T;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -193,8 +164,8 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_gram_kernel(const Chunked
         for (int j = 0; j < 4; ++j) out[(ty * 4 + i) * CH_T + tx + 16 * j] = acc[i][j].x + acc[i][j].y;
 }
 
-template <typename T, typename TX, typename Decay>
-__global__ void __launch_bounds__(CH_THREADS, 2) chunk_add_kernel(const Chunked m, const Decay d) {
+template <typename T>
+__global__ void __launch_bounds__(CH_THREADS, 2) chunk_add_kernel(const Chunked m, const SsdDecay d) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -208,14 +179,14 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_add_kernel(const Chunked 
     if (threadIdx.x < CH_T) w[threadIdx.x] *= expf((float)(cum[CH_T - 1] - cum[threadIdx.x]));
     if (threadIdx.x == 0 && v0 == 0) m.chunk_decay[(size_t)slot * m.H + h] = expf((float)cum[CH_T - 1]);
     __syncthreads();
-    chunk_turned<TX>(m.x, h, c, v0, CH_V, w, Xt);
+    chunk_turned<T>(m.x, h, c, v0, CH_V, w, Xt);
     chunk_turned<T>(m.b, h / (m.H / m.groups), c, 0, m.N, nullptr, Bt);
     __syncthreads();
     const int K = (c.nt + 3) & ~3;
     for (int n0 = 0; n0 < m.N; n0 += 64) {
         float2 acc[4][4];
         ch_zero(acc);
-        ch_product(Xt + ty * 4 * CH_LD, CH_LD, Bt + (n0 + tx) * CH_LD, CH_LD, K, acc);
+        tile_product<2>(Xt + ty * 4 * CH_LD, CH_LD, Bt + (n0 + tx) * CH_LD, CH_LD, K, acc);
         float* out = m.carry + (((size_t)slot * m.H + h) * m.V + v0 + ty * 4) * m.N + n0 + tx;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -235,7 +206,7 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(const Chunked m) {
     const int n_chunks = (len + CH_T - 1) / CH_T, slot0 = first / CH_T + s;
     const int h = (int)(e / ((int64_t)m.V * m.N)), v = (int)(e / m.N % m.V), n = (int)(e % m.N);
     float* st = m.state + (size_t)TK_SLOT(m.check, m.seq_slot[s]) * cells + (size_t)h * m.V * m.N;
-    const int64_t at = m.state_vn ? (int64_t)v * m.N + n : (int64_t)n * m.V + v, step = m.state_vn ? 1 : m.V;
+    const int64_t at = (int64_t)n * m.V + v, step = m.V;
     float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
     if (m.seq_ctx[s] > 0) S = make_float4(st[at], st[at + step], st[at + 2 * step], st[at + 3 * step]);
     float* cell = m.carry + (size_t)slot0 * cells + e;
@@ -265,8 +236,8 @@ __global__ void __launch_bounds__(128) chunk_carry_kernel(const Chunked m) {
     st[at + 3 * step] = S.w;
 }
 
-template <typename T, typename TX, typename Decay>
-__global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const Chunked m, const Decay d) {
+template <typename T>
+__global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const Chunked m, const SsdDecay d) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -285,7 +256,7 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const Chunked 
         for (int i = tid; i < CH_V * (m.N / 4); i += CH_THREADS)
             *reinterpret_cast<float4*>(St + i / (m.N / 4) * ld + i % (m.N / 4) * 4) = *reinterpret_cast<const float4*>(S0 + 4 * i);
     }
-    chunk_turned<TX>(m.x, h, c, v0, CH_V, nullptr, Xt);
+    chunk_turned<T>(m.x, h, c, v0, CH_V, nullptr, Xt);
     const float* gram = m.gram + ((size_t)slot * m.groups + g) * CH_T * CH_T;
     for (int i = tid; i < CH_T * CH_T; i += CH_THREADS) {
         const int t = i / CH_T, s = i % CH_T;
@@ -297,7 +268,7 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const Chunked 
     float2 acc[4][4];
     ch_zero(acc);
     if (!fresh) {
-        ch_product(Cs + ty * 4 * ld, ld, St + tx * ld, ld, m.N, acc);
+        tile_product<2>(Cs + ty * 4 * ld, ld, St + tx * ld, ld, m.N, acc);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float a = expf((float)cum[ty * 4 + i]);
@@ -305,7 +276,7 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const Chunked 
             for (int j = 0; j < 4; ++j) acc[i][j].x *= a, acc[i][j].y *= a;
         }
     }
-    ch_product(Ms + ty * 4 * CH_LD, CH_LD, Xt + tx * CH_LD, CH_LD, row0, acc);
+    tile_product<2>(Ms + ty * 4 * CH_LD, CH_LD, Xt + tx * CH_LD, CH_LD, row0, acc);
     // the warp's own eight columns, where a row ends: what comes after a token stays out of its sum, whatever it holds
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
@@ -340,8 +311,8 @@ inline int64_t chunked_scratch(int64_t tokens, int64_t n_seqs, int64_t H, int64_
     return slots * (groups * CH_T * CH_T + H * V * N + (H + 3) / 4 * 4);
 }
 
-template <typename T, typename TX, typename Decay>
-int launch_chunked(Chunked m, const Decay& d, float* scratch, int tokens, cudaStream_t stream) {
+template <typename T>
+int launch_chunked(Chunked m, const SsdDecay& d, float* scratch, int tokens, cudaStream_t stream) {
     const int slots = tokens / CH_T + m.n_seqs, ld = m.N + 4, vb = m.V / CH_V;
     m.gram = scratch;
     m.carry = m.gram + (size_t)slots * m.groups * CH_T * CH_T;
@@ -349,16 +320,16 @@ int launch_chunked(Chunked m, const Decay& d, float* scratch, int tokens, cudaSt
     const int gram_smem = 2 * CH_T * ld * 4, add_smem = (CH_V + m.N) * CH_LD * 4;
     const int out_smem = ((CH_T + CH_V) * ld + (CH_T + CH_V) * CH_LD) * 4;
     cudaFuncSetAttribute(chunk_gram_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, gram_smem);
-    cudaFuncSetAttribute(chunk_add_kernel<T, TX, Decay>, cudaFuncAttributeMaxDynamicSharedMemorySize, add_smem);
-    cudaFuncSetAttribute(chunk_out_kernel<T, TX, Decay>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_smem);
+    cudaFuncSetAttribute(chunk_add_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, add_smem);
+    cudaFuncSetAttribute(chunk_out_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_smem);
     tk_launch(chunk_gram_kernel<T>, dim3(slots, m.groups), dim3(CH_THREADS), gram_smem, stream, m);
     TK_CHECK_LAUNCH("chunk_gram");
-    tk_launch(chunk_add_kernel<T, TX, Decay>, dim3(slots, m.H, vb), dim3(CH_THREADS), add_smem, stream, m, d);
+    tk_launch(chunk_add_kernel<T>, dim3(slots, m.H, vb), dim3(CH_THREADS), add_smem, stream, m, d);
     TK_CHECK_LAUNCH("chunk_add");
     const int64_t quads = (int64_t)m.H * m.V * m.N / 4;
     tk_launch(chunk_carry_kernel, dim3((unsigned)((quads + 127) / 128), m.n_seqs), dim3(128), 0, stream, m);
     TK_CHECK_LAUNCH("chunk_carry");
-    tk_launch(chunk_out_kernel<T, TX, Decay>, dim3(slots, m.H, vb), dim3(CH_THREADS), out_smem, stream, m, d);
+    tk_launch(chunk_out_kernel<T>, dim3(slots, m.H, vb), dim3(CH_THREADS), out_smem, stream, m, d);
     TK_CHECK_LAUNCH("chunk_out");
     return 0;
 }

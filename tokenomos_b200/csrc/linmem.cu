@@ -25,7 +25,7 @@
 // segment before added), formed over the segments before it, all in 32-bit like the walk itself.
 #include <math.h>
 
-#include "common.cuh"
+#include "packed.cuh"
 
 namespace {
 enum : int { TK_K_LINMEM = 13 };
@@ -76,22 +76,6 @@ struct LinMem {
 __device__ __forceinline__ float lm_silu(float x) { return x / (1.0f + expf(-x)); }
 __device__ __forceinline__ float lm_decay(float z, float A) { return expf(-A * (z > 20.f ? z : log1pf(expf(z)))); }
 
-// Two 32-bit multiply-adds in one instruction (sm_100's packed form), each half rounded as the scalar one.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
-          "l"(reinterpret_cast<unsigned long long&>(c)));
-    return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
-    return d;
-}
 __device__ __forceinline__ float2 two(float x) { return make_float2(x, x); }
 __device__ __forceinline__ float sum8(float v) {      // over the eight lanes of a column
     v += __shfl_xor_sync(0xffffffffu, v, 1);

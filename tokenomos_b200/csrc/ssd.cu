@@ -29,24 +29,6 @@ constexpr int SSD_TOK = 16;      // tokens staged at a time
 constexpr int SSD_MAX_SLICES = 8;
 }  // namespace
 
-// Two 32-bit multiply-adds in one instruction (sm_100's packed form): d = a * b + c on both halves, each
-// rounded as the scalar instruction rounds.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
-          "l"(reinterpret_cast<unsigned long long&>(c)));
-    return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;"
-        : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
-    return d;
-}
-
 // XC: values of x a thread keeps for the stage ahead (TOK * COLS over the block's threads: 2 with eight
 // slices, 4 with four or more, else 16); 0: nothing is kept ahead, a stage's rows go from memory to
 // shared memory directly, which costs fewer registers and is what a step of single tokens wants.
@@ -334,10 +316,10 @@ TK_API int tk_ssd_chunked(const void* xbc, int64_t xbc_stride, const float* dt_r
     m.c = {base + ((int64_t)H * V + (int64_t)G * N) * es, N, xbc_stride};
     m.cu_seqlens = cu_seqlens, m.seq_ctx = seq_ctx, m.seq_slot = seq_slot;
     m.n_seqs = n_seqs, m.H = H, m.V = V, m.N = N, m.groups = G;
-    m.y = y, m.state = state, m.state_vn = 0, m.check = TK_K_SSD;
+    m.y = y, m.state = state, m.check = TK_K_SSD;
     const SsdDecay d = {dt_raw, dt_stride, dt_bias, A_log, D_skip};
-    return dtype == TK_F32 ? launch_chunked<float, float>(m, d, scratch, tokens, stream)
-                           : launch_chunked<__nv_bfloat16, __nv_bfloat16>(m, d, scratch, tokens, stream);
+    return dtype == TK_F32 ? launch_chunked<float>(m, d, scratch, tokens, stream)
+                           : launch_chunked<__nv_bfloat16>(m, d, scratch, tokens, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
