@@ -463,7 +463,7 @@ def test_attention_f32_values_that_are_not_finite_reach_the_rows_that_see_them(H
 def test_swiglu32_vectorised_equals_the_scalar_kernel():
     """Whole and partial blocks of a row; rows that do not begin on 16 bytes go the scalar way, with the same bits."""
     from tokenomos_b200 import ops
-    for rows, inter in ((3, 8), (2, 2048), (5, 2052), (1, 4608)):
+    for rows, inter in ((3, 8), (2, 2048), (5, 2052), (1, 4608), (300, 2052), (13000, 8), (38, 2048)):
         gu = torch.randn(rows, 2 * inter, device="cuda") * 4
         odd = torch.empty(rows * 2 * inter + 1, device="cuda")[1:].view(rows, 2 * inter).copy_(gu)
         assert odd.data_ptr() % 16 and torch.equal(ops.swiglu(gu), ops.swiglu(odd))

@@ -393,8 +393,9 @@ swiglu_vec_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out, int rows, int int
 
 // 32-bit storage with all gate channels before all up channels: 16 bytes of gate and of up per thread and step, two steps in
 // flight, one block row of the grid per token row, the arithmetic of the kernel above to the bit (accurate exponential and
-// division); bound by memory, where one element a step with a 64-bit index division was bound by its instructions: the
-// feed-forward of 2,048 rows of 2,048 x 8,192 went from 1,388 to 1,335 us with it.
+// division); bound by memory, where one element a step with a 64-bit index division was bound by its instructions: 2,048 rows of
+// 8,192 channels 29 us, 72 before, 500 of 260 2.26 and 2.57. Of few elements it is the slower one, whose blocks leave most SMs
+// without any (1 row of 4,608 2.1 us against 1.8, 8 of 8,192 2.0 and 1.8): those stay one element a step.
 __global__ void __launch_bounds__(256)
 swiglu32_vec_kernel(const float* gu, float* out, int inter, int blocks_per_row) {
     pdl_launch_dependents();
@@ -441,7 +442,7 @@ TK_API int tk_swiglu(const void* gu, void* out, int rows, int inter, int block, 
         TK_CHECK_LAUNCH("swiglu_vec");
         return 0;
     }
-    if (dtype == TK_F32 && block == 0 && inter % 4 == 0 && (uintptr_t)gu % 16 == 0 && (uintptr_t)out % 16 == 0) {
+    if (dtype == TK_F32 && block == 0 && total >= 148 * 2 * threads && inter % 4 == 0 && (uintptr_t)gu % 16 == 0 && (uintptr_t)out % 16 == 0) {
         const int blocks_per_row = (inter / 4 + 2 * threads - 1) / (2 * threads);
         TK_CHECK_ARG((int64_t)rows * blocks_per_row <= 0x7fffffffLL, "swiglu: %d rows of %d channels exceed the grid", rows, inter);
         tk_launch(swiglu32_vec_kernel, dim3((unsigned)(rows * blocks_per_row)), dim3(threads), 0, stream, (const float*)gu,
