@@ -26,7 +26,7 @@ pytestmark = pytest.mark.gpu
 # attention has a prefill and a decode form. Their difference is that of two roundings of the
 # same value, so it is held to about the bound each has against the oracle (measured: A 0.33 %,
 # B 3.4 %, C 0.88 %, D 1.4 %), not to accumulation order; the 32-bit path, where the cut changes
-# no rounding, is what holds the cache and the batch to 1e-5.
+# at most the order of sums (and none in these sizes' products), is what holds the cache and the batch to 1e-5.
 TOL_F32, TOL_F32_SAME = 2e-5, 1e-5
 TOL_BF16 = {"A": 8e-3, "B": 4e-2, "C": 4e-2, "D": 2.5e-2}
 TOL_BF16_SAME = {"A": 6e-3, "B": 5e-2, "C": 1.5e-2, "D": 2.2e-2}
