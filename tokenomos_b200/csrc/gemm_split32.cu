@@ -1,4 +1,4 @@
-// out[M, N] = x[M, K] . W[N, K]^T (+ bias), all float32, on the bfloat16 tensor cores without giving up a bit of 32-bit:
+// out[M, N] = x[M, K] . W[N, K]^T (+ bias), all float32, on the bfloat16 tensor cores with the errors of 32-bit sums:
 //
 //   every operand is taken apart as x = h + m + l, three bfloat16 numbers of 8 significant bits each (h = bf16(x), m =
 //   bf16(x - h), l = bf16(x - h - m): the differences are exact), and of the nine products the six that reach 2^-24 of
@@ -13,8 +13,8 @@
 //   against 64 bits (normal values, K 1,024 to 10,752), where the multiply-adds of gemm_simt.cu are off by 0.6e-6 to 1.9e-6.
 //
 // Bound by the tensor pipe: six bfloat16 products, i.e. a sixth of its rate, against which the CUDA cores' multiply-adds
-// have a twentieth: 2,048 x 16,384 x 2,048 in 717 us (192 TFLOP/s; gemm_simt.cu 5,414), 16 x 2,048 x 2,048 in 17 us (119),
-// never slower than it from 9 rows and 128 x 128 weights on (14.2 us against 14.5; taken from 256 x 256 on). A CTA owns
+// have a twentieth: 2,048 x 16,384 x 2,048 in 694 us (198 TFLOP/s; gemm_simt.cu 5,414), 16 x 2,048 x 2,048 in 15.5 us (119),
+// never slower than it from 9 rows and 128 x 128 weights on (9 x 256 x 256 9.4 us against 15.8; taken from 256 x 256 on). A CTA owns
 // 128 rows of W (the MMA's M) and BN tokens; 16 warps read 32 columns of both operands from memory into registers a chunk
 // ahead, take them apart and store the three parts as K-major tiles in the 128-byte swizzle (h and m side by side in one row, l in a tile that the two buffers share by halves), one thread issues the
 // twelve MMAs of a chunk, and all warps work on the next chunk meanwhile. BN = 256 keeps shared memory (96 bytes a cycle

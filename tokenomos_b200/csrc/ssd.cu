@@ -16,8 +16,9 @@
 // formed once per token; the next 16 are asked for before the walk and wait in registers meanwhile);
 // every thread then walks the 16 tokens with multiply-adds only, leaves its
 // partial sums of S^T C in shared memory, and the block adds the slices' partial sums in a fixed
-// order. The state's arithmetic does not depend on how a request's tokens were cut into steps: a
-// step continues from the stored S exactly where the step before left it.
+// order. The walk's arithmetic does not depend on how a request's tokens were cut into steps: a
+// step continues from the stored S exactly where the step before left it. (Chunk by chunk, chunked.cuh,
+// sums have another order: the cut then moves results by a few 2^-24.)
 #include <math.h>
 
 #include "chunked.cuh"

@@ -768,9 +768,8 @@ SPLIT32_MIN_ROWS, SPLIT32_MIN_SIDE = 9, 256
 
 
 def gemm_split32_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether a 32-bit product goes to the tensor cores in parts that keep all of its 32 bits (csrc/gemm_split32.cu): 16-byte
-    rows, and sizes at which that is the faster way (below 256 rows of ``w`` or columns either takes as long as a launch, and
-    the sums keep the one order they have in steps of any size)."""
+    """Whether a 32-bit product goes to the tensor cores in three 16-bit parts an operand (csrc/gemm_split32.cu): 16-byte rows,
+    and sizes at which that is the faster way (below 256 rows of ``w`` or columns either takes as long as a launch)."""
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] >= SPLIT32_MIN_ROWS
             and w.shape[0] >= SPLIT32_MIN_SIDE and x.shape[1] >= SPLIT32_MIN_SIDE and x.shape[1] % 4 == 0
             and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
@@ -779,7 +778,9 @@ def gemm_split32_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
 def gemm(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
          out_dtype: torch.dtype | None = None) -> torch.Tensor:
     """``x @ w.T (+ bias)`` with 32-bit accumulation, any shape: on the CUDA cores, or, for 32-bit operands of some size, on
-    the tensor cores in parts that lose nothing of them. ``x`` [M, K] (row stride free), ``w`` [N, K]; ``bias`` float32 [N]."""
+    the tensor cores in parts, closer to 64 bits than the CUDA cores' chain of multiply-adds (inputs below 2^-110 in size lose
+    their last bits). The order of an element's additions depends on the sizes, the number of rows among them: the same row in
+    a step of another size differs by a few 2^-24. ``x`` [M, K] (row stride free), ``w`` [N, K]; ``bias`` float32 [N]."""
     _cuda(x, w, bias)
     M, K = x.shape
     N = w.shape[0]

@@ -3,8 +3,9 @@
 Routes, by storage type:
 
 - float32: the weight-streaming kernel for up to 8 rows (``ops.gemm_stream32``), else ``ops.gemm``: 32-bit
-  multiply-adds on the CUDA cores, or tensor-core products of operands taken apart so that none of their 32
-  bits is lost. No reduced-precision mode can reach it, whatever the process-wide torch flags say.
+  multiply-adds on the CUDA cores, or tensor-core products of operands taken apart into three 16-bit parts,
+  with smaller errors than the multiply-adds'. No reduced-precision mode can reach it, whatever the
+  process-wide torch flags say. Which of them it is depends on the rows of the step.
 - bfloat16: by shape (``route``): the hand-written weight-streaming kernel for a few rows
   (``ops.gemm_skinny``), the TMA + tcgen05 kernel for very tall matrices (``ops.gemm_tc``), else
   the library GEMM (cuBLAS through ``torch.nn.functional.linear``), as the reference engine does
@@ -95,7 +96,7 @@ class Linear:
 
     def _product32(self, x: torch.Tensor) -> torch.Tensor:
         """32-bit operands: the weight-streaming kernel for a few rows of a matrix of some size, else ``ops.gemm`` (small ones take as
-        long as a launch either way, and keep one order of their sums in steps of any size)."""
+        long as a launch either way)."""
         if min(self.out_features, self.in_features) >= ops.STREAM32_MIN_SIDE and ops.gemm_stream32_ok(x, self.weight):
             return ops.gemm_stream32(x, self.weight, self.bias)
         return ops.gemm(x, self.weight, self.bias, torch.float32)
