@@ -892,7 +892,7 @@ def test_trace_program_and_command_line(folders, tmp_path):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H, K, D, V, lens, ctx, pairs", [
-    (4, 2, 128, 128, (300, 1, 33, 16, 177), (0, 5, 9, 0, 3), False), (2, 1, 64, 40, (121,), (7,), False),
+    (4, 2, 128, 128, (300, 1, 33, 16, 177), (0, 5, 9, 0, 3), False), (2, 1, 64, 40, (121,), (7,), True), (2, 1, 64, 40, (61,), (7,), False),
     (2, 2, 200, 24, (0, 96, 0, 130), (0, 0, 0, 2), False), (3, 3, 24, 24, (47, 18), (0, 4), False),
     (2, 1, 128, 128, (277,), (3,), True), (4, 2, 128, 40, (143, 301, 32), (5, 0, 2), True), (2, 2, 96, 96, (161, 1, 240), (0, 7, 2), True),
     (4, 2, 64, 40, (303, 33, 177), (0, 9, 0), True), (3, 3, 24, 24, (250, 0, 145), (0, 4, 1), True)])

@@ -42,11 +42,12 @@ enum : int { LM_FIXED = 0, LM_HEAD = 1, LM_CHANNEL = 2 };
 // 237, 64 in four of 300 131 and 128). Keys up to 128 are bound by the multiply-adds of a block (16 heads of 128 x 128: 406
 // and 410), until one column a thread spreads them over twice the SMs: while those blocks are no more than the SMs (one
 // sequence of 2,048 tokens 319 us; two of 1,024 243 against 219). What the token before leaves in each token's keys is formed
-// beforehand, which portions of 128 tokens and up to 64 q/k heads over all sequences pay back (one sequence of 8 tokens 8.8 us
-// against 7.8; 32 q/k heads of 64 on 33 tokens 18.0 against 15.5, on 100 27.4 and 26.8, on 300 55 and 61).
+// beforehand, which portions of 64 tokens (four a q/k head from 16 heads on) and up to 64 q/k heads over all sequences pay back
+// (one sequence of 8 tokens 8.8 us against 7.8, 16 heads over 8 on 100 20.9 and 23.3; 32 q/k heads of 64 on 33 tokens 18.0
+// against 15.5, on 100 27.4 and 26.8, on 128 30.4 and 31.6).
 constexpr bool LM_PAIRS(int rule, int decay) { return rule == LM_DELTA && decay == LM_HEAD; }
 inline bool lm_pairs(int decay, int tokens, int n_seqs, int H, int K, int D, int V, int sm_count) {
-    if (decay != LM_HEAD || D > 128 || tokens < 128 * n_seqs || K * n_seqs > 64) return false;
+    if (decay != LM_HEAD || D > 128 || tokens < (K <= 16 ? 64 : 4 * K) * n_seqs || K * n_seqs > 64) return false;
     return D <= 64 ? H * n_seqs <= 128 : (V + 15) / 16 * H * n_seqs <= sm_count;
 }
 
