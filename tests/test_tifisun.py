@@ -950,3 +950,81 @@ def test_delta_rule_two_tokens_a_step(H, K, D, V, lens, ctx, pairs, dtype):
     rows[t, nk] = float("nan")
     again = run(rows, state.cuda())
     assert torch.equal(again[:t], got[:t]) and torch.isnan(again[t]).any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H, K, D, V, lens, ctx", [
+    (2, 1, 128, 32, (64,), (0,)), (2, 2, 128, 96, (65, 127, 1), (4, 0, 7)), (6, 2, 128, 128, (63, 0, 129, 192), (0, 0, 9, 1)),
+    (3, 1, 64, 64, (320,), (2,)), (4, 4, 64, 32, (128, 200, 131), (1, 0, 3)), (16, 8, 128, 128, (150, 90), (0, 6)),
+    (20, 4, 64, 128, (191, 257), (0, 1))])
+def test_delta_rule_chunk_by_chunk(H, K, D, V, lens, ctx):
+    """The delta rule over chunks of 64 tokens (16-bit rows) at the edges of a chunk, of 16 tokens within it and of the blocks' rows, one
+    to five heads a q/k head: against the recurrence in 64-bit, sums of up to 128 products in 32-bit; decays from 1 to 0, a value of
+    2^120; numbers that are not finite reach their own column from their token
+    on, a key all columns, a query its own output."""
+    from tokenomos_b200 import ops
+    g = torch.Generator().manual_seed(11)
+    T, S, nk, nv = sum(lens), len(lens), K * D, H * V
+    assert ops._lib.call("tk_delta_chunks_scratch", T, S, H, K, D, V) > 0
+    u = torch.randn(T, 2 * nk + nv + 8, generator=g).bfloat16()
+    zb, za = torch.randn(T, H + 4, generator=g), torch.randn(T, H + 4, generator=g) - 2.0
+    za[::19] += 8.0
+    za[::47, 0] = 1e4                                            # a decay of 0
+    zb[5::31] = -200.0                                           # beta of 0
+    A, bias = torch.rand(H, generator=g) * 3, torch.randn(H, generator=g)
+    state = torch.randn(S + 1, H, V, D, generator=g) * 0.3
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    slots = list(range(S, 0, -1))
+
+    def run(rows, st):
+        return ops.linmem_scan(rows.cuda(), (0, nk, 2 * nk), "delta", "head", A.cuda(), st, i32(cu), i32(list(ctx)), i32(slots), S,
+                               H, K, D, V, D ** -0.5, unit=True, beta=zb.cuda(), gates=za.cuda(), bias=bias.cuda())
+
+    def exact(rows):
+        unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+        q = (unit(rows[:, :nk].double().view(T, K, D)) * D ** -0.5).repeat_interleave(H // K, 1)
+        k = unit(rows[:, nk:2 * nk].double().view(T, K, D)).repeat_interleave(H // K, 1)
+        v = rows[:, 2 * nk:2 * nk + nv].double().view(T, H, V)
+        beta = torch.sigmoid(zb[:, :H].double())
+        decay = torch.exp(-A.double() * torch.nn.functional.softplus(za[:, :H].double() + bias.double()))
+        want, after = torch.empty(T, H, V, dtype=torch.float64), state.double()
+        for s in range(S):
+            M = after[slots[s]] if ctx[s] else torch.zeros(H, V, D, dtype=torch.float64)          # [head, value, key]
+            for t in range(cu[s], cu[s + 1]):
+                M = decay[t, :, None, None] * M
+                w = beta[t, :, None] * (v[t] - torch.einsum("hvk,hk->hv", M, k[t]))
+                M = M + w[:, :, None] * k[t][:, None, :]
+                want[t] = torch.einsum("hvk,hk->hv", M, q[t])
+            if lens[s]:
+                after[slots[s]] = M
+        return want, after
+
+    st = state.cuda()
+    got = run(u, st)
+    want, after = exact(u)
+    assert (got.double().cpu().view(T, H, V) - want).norm() <= 1e-6 * want.norm()
+    assert (st.double().cpu() - after).norm() <= 1e-6 * after.norm()
+
+    last = max(range(S), key=lambda s: lens[s])
+    t = cu[last] + lens[last] // 2
+    large = u.clone()
+    large[t, 2 * nk] = 2.0 ** 120                                 # head 0, column 0 (products are formed with k before its length is divided out)
+    st = state.cuda()
+    again = run(large, st)
+    assert torch.isfinite(again).all() and torch.isfinite(st[1:]).all()
+    for value, column in ((float("nan"), 2 * nk + V + 1), (float("inf"), 2 * nk), (float("nan"), nk), (float("nan"), 0)):
+        rows, st = u.clone(), state.cuda()
+        rows[t, column] = value
+        again = run(rows, st).view(T, H, V)
+        clean = torch.ones(T, H, V, dtype=torch.bool)
+        if column >= 2 * nk:                                      # a value: its column from its token on
+            clean[t:cu[last + 1], (column - 2 * nk) // V, (column - 2 * nk) % V] = False
+        elif column >= nk:                                        # a key: the heads that read it, from its token on
+            clean[t:cu[last + 1], :H // K] = False
+        else:                                                     # a query: its own output
+            clean[t, :H // K] = False
+        assert torch.equal(again.cpu()[clean], got.view(T, H, V).cpu()[clean])
+        assert not torch.isfinite(again.cpu()[~clean]).any()

@@ -27,6 +27,7 @@
 // formed again by multiply-adds in the order of K, which put infinities and NaN where gemm_simt.cu puts them.
 #include <cooperative_groups.h>
 
+#include "parts.cuh"
 #include "tcgen05.cuh"
 
 namespace cg = cooperative_groups;
@@ -46,17 +47,6 @@ __device__ __forceinline__ bool split_wait(uint32_t bar, uint32_t parity, int wh
         }
     }
     return true;
-}
-
-// Two floats -> (h, m, l) pairs of bfloat16.
-__device__ __forceinline__ void take_apart(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-    const __nv_bfloat162 hh = __floats2bfloat162_rn(a, b);
-    h = *reinterpret_cast<const uint32_t*>(&hh);
-    const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-    const __nv_bfloat162 mm = __floats2bfloat162_rn(ra, rb);
-    m = *reinterpret_cast<const uint32_t*>(&mm);
-    const __nv_bfloat162 ll = __floats2bfloat162_rn(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));
-    l = *reinterpret_cast<const uint32_t*>(&ll);
 }
 
 template <int COLS>

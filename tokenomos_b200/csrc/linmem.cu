@@ -18,6 +18,7 @@
 //
 // A step continues from the stored S exactly where the step before left it, and a token's arithmetic is the same
 // wherever the request was cut, to rounding; a sequence at position 0 starts from zeros whatever its state row holds.
+// (Portions of the delta rule with a decay per head, 16-bit rows and unit keys, are formed chunk by chunk in delta_chunked.cu.)
 //
 // The additive rule with a fixed decay is linear in S, so a long portion need not be walked by one block per columns from
 // end to end: it is cut into segments of LM_SEG tokens, a first pass walks all of them but the last side by side for what

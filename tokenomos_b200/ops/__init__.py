@@ -1789,6 +1789,18 @@ def linmem_scan(qkv: torch.Tensor, offsets: tuple, rule: str, decay: str, A: tor
         if need and (t is None or t.dtype != torch.float32 or t.stride(1) != 1 or t.shape[0] != T or t.shape[1] < need):
             raise KernelError(f"linmem_scan: {name} is float32 [{T}, >= {need}] with contiguous columns")
     y = torch.empty(T, heads * v_dim, dtype=torch.float32, device=qkv.device)
+    if (rule == "delta" and decay == "head" and unit and not act and half == 0 and qkv.dtype == torch.bfloat16
+            and qkv.stride(0) % 8 == 0 and not any(int(o) % 8 for o in offsets) and qkv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0):
+        words = _lib.call("tk_delta_chunks_scratch", T, int(n_seqs), heads, kv_heads, dim, v_dim)
+        if words:
+            # portions of some length: chunk by chunk on the tensor cores
+            scratch = torch.empty(words, dtype=torch.float32, device=qkv.device)
+            _lib.call("tk_delta_chunks", _ptr(qkv), qkv.stride(0), int(offsets[0]), int(offsets[1]), int(offsets[2]), _ptr(beta),
+                      beta.stride(0), _ptr(gates), gates.stride(0), _ptr(_f32vec(bias, "decay bias", cols)),
+                      _ptr(_f32vec(A, "A", heads)), _ptr(state), _ptr(_i32(cu_seqlens, "cu_seqlens")), _ptr(_i32(seq_ctx, "seq_ctx")),
+                      _ptr(_i32(seq_slot, "seq_slot")), int(n_seqs), T, _ptr(y), _ptr(scratch), heads, kv_heads, dim, v_dim,
+                      float(q_scale), int(sm_count), _stream())
+            return y
     # a step with portions stages its vectors in memory first
     n = _lib.call("tk_linmem_scratch", T, int(n_seqs), heads, kv_heads, dim, v_dim, LINMEM_DECAYS[decay], int(sm_count))
     scratch = torch.empty(n, 32, dtype=torch.float32, device=qkv.device) if n else None
