@@ -1001,6 +1001,73 @@ def test_scan_by_chunks(H, V, N, G, lens, ctx, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("H, V, N, G, lens, ctx, shift", [
+    (1, 32, 64, 1, (64,), (0,), 0), (5, 32, 128, 1, (65, 127, 1), (4, 0, 7), 0), (6, 96, 128, 2, (63, 0, 129, 192), (0, 0, 9, 1), 0),
+    (40, 64, 64, 8, (48, 50), (2, 0), 0), (32, 128, 128, 4, (150, 90), (0, 6), 0), (4, 64, 128, 2, (700,), (1,), 4)])
+def test_scan_by_chunks_of_16_bit_rows(H, V, N, G, lens, ctx, shift):
+    """Chunks of 64 tokens on the tensor cores at the edges of a chunk, of 16 tokens within it and of the blocks' rows, one to eight
+    heads a group (rows that begin on 8 bytes instead of 16: by multiply-adds): against the recurrence in 64-bit, sums of up to 128 products in
+    32-bit; decays from 1 to 0. Numbers that are not finite reach their own row of x from their token on, b all rows, c its own output."""
+    from tokenomos_b200 import ops
+    g = torch.Generator().manual_seed(13)
+    T, S = sum(lens), len(lens)
+    assert ops._lib.call("tk_ssd_tc_scratch", T, S, H, V, N, G) > 0
+    xbc = torch.randn(T, H * V + 2 * G * N, generator=g).to(torch.bfloat16)
+    raw = torch.randn(T, H + 4, generator=g)
+    raw[::17] += 8.0
+    raw[::47, 0] = 1e4                                            # a decay of 0
+    raw[3::29] = -120.0                                           # dt of 0
+    bias, a_log, skip = (torch.randn(H, generator=g) for _ in range(3))
+    state = torch.randn(S + 1, H, N, V, generator=g)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    slots = list(range(S, 0, -1))
+
+    def run(rows, st):
+        wide = torch.nn.functional.pad(rows, (shift, 16 - 2 * shift)).cuda()[:, shift:shift + rows.shape[1]]
+        return ops.ssd_scan(wide, raw.cuda(), bias.cuda(), a_log.cuda(), skip.cuda(), st, i32(cu), i32(list(ctx)), i32(slots), S, H, V, N, G)
+
+    st = state.cuda()
+    got = run(xbc, st)
+    assert tuple(got.shape) == (1, T, H * V)
+    x = xbc[:, :H * V].double().view(T, H, V)
+    B = xbc[:, H * V:H * V + G * N].double().view(T, G, N).repeat_interleave(H // G, 1)
+    C = xbc[:, H * V + G * N:H * V + 2 * G * N].double().view(T, G, N).repeat_interleave(H // G, 1)
+    step = torch.nn.functional.softplus(raw[:, :H].double() + bias.double())
+    decay = torch.exp(-torch.exp(a_log.double()) * step)
+    want, after = torch.empty(T, H, V, dtype=torch.float64), state.double()
+    for s in range(S):
+        M = after[slots[s]] if ctx[s] else torch.zeros(H, N, V, dtype=torch.float64)
+        for t in range(cu[s], cu[s + 1]):
+            M = decay[t, :, None, None] * M + step[t, :, None, None] * B[t][:, :, None] * x[t][:, None, :]
+            want[t] = torch.einsum("hn,hnv->hv", C[t], M) + skip.double()[:, None] * x[t]
+        if lens[s]:
+            after[slots[s]] = M
+    assert (got[0].double().cpu().view(T, H, V) - want).norm() <= 1e-6 * want.norm()
+    assert (st.double().cpu() - after).norm() <= 1e-6 * after.norm()
+
+    last = max(range(S), key=lambda s: lens[s])
+    t = cu[last] + lens[last] // 2
+    raw[t] = 0.0                                                  # (with a dt of 0 the walk keeps what is not finite too, as NaN)
+    got = run(xbc, state.cuda())
+    for value, column in ((float("nan"), V - 1), (float("inf"), 0), (float("nan"), H * V), (float("nan"), H * V + G * N)):
+        rows = xbc.clone()
+        rows[t, column] = value
+        again = run(rows, state.cuda())[0].view(T, H, V).cpu()
+        clean = torch.ones(T, H, V, dtype=torch.bool)
+        if column < H * V:                                        # x: its row of the state, from its token on
+            clean[t:cu[last + 1], 0, column] = False
+        elif column < H * V + G * N:                              # b: the heads that read it, from its token on
+            clean[t:cu[last + 1], :H // G] = False
+        else:                                                     # c: its own output
+            clean[t, :H // G] = False
+        assert torch.equal(again[clean], got[0].view(T, H, V).cpu()[clean])
+        assert not torch.isfinite(again[t][~clean[t]]).any()
+
+
+@pytest.mark.gpu
 def test_scan_by_chunks_with_decays_of_zero():
     """A head whose rate overflows forgets everything at every token, as it does in the walk over one token at a time:
     y_t = (dt_t B_t . C_t + D) x_t, and the state is the last token's."""

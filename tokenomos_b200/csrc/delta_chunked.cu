@@ -28,23 +28,14 @@
 // R and U are taken out of the products and every output of the row from the first one on, and the row of S, are set to NaN.
 // (Products with k come before its length is divided out: values and states beyond 2^128 / |k| overflow.)
 //
-// Chunks count from each sequence's first token of the step; sequence s has the slots cu_seqlens[s] / 64 + s and up.
-//
 // Measured (both kernels, us; token by token in brackets): 16 heads of 128 x 128 over 8 on 750 and 2,250 tokens 138 (462), on 2,048
 // 112 (324); heads of 64 x 64 88 (314) and 78 (280); 16 x 16 heads of 128, sixteen sequences of 512, 251 (614). Against 64 bits y
 // is 1.7e-7 off and S 1.3e-7, the walk 2.1e-7 to 6.8e-7 and 2.1e-7 to 3.7e-7 (growing with the tokens). A chunk takes 4,800 cycles of
 // a state warp (P 1,050, R 450, U 900, its parts 600, the update of S 1,200 with its sums), of which 2,000 are its 252 products.
-#include <math.h>
-
-#include "packed.cuh"
-#include "paged_tiles.cuh"
-#include "parts.cuh"
+#include "chunk_tc.cuh"
 
 namespace {
 enum : int { TK_K_DELTA_CHUNKS = 16 };
-constexpr int DC_T = 64;                       // tokens of a chunk
-constexpr int DC_LD = DC_T + 4;                // row of a 64 x 64 matrix of floats in shared memory
-constexpr int DC_PART = DC_T * DC_T * 2;       // bytes of one 16-bit part of T or G
 constexpr int DC_MATS = 6 * DC_PART;           // bytes of a chunk's and head's T and G: three parts each
 // factors of a chunk's tokens (one array of 64 each): A_t |k_t|^-1; A_t scale |q_t|^-1; (A_end / A_t) |k_t|^-1; A_end (first element)
 enum : int { DC_K = 0, DC_Q = 1, DC_W = 2, DC_END = 3, DC_FACTORS = 4 };
@@ -68,8 +59,6 @@ struct DeltaChunks {
     uint8_t* mats;             // [slots][H][T's parts, G's parts], each part as the walk's shared memory holds it
     float* factors;            // [slots][H][DC_FACTORS][64]
 };
-
-__device__ __forceinline__ uint32_t shared_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // The matrix at L (rows DC_LD apart): its lower left block of B x B becomes -T22 (L21 T11), T11 and T22 being the blocks above and
 // beside it; thread (r, c) has COLS neighbouring elements of row r. T11 is zero above its diagonal; the block above T22 is used, and
@@ -122,24 +111,6 @@ __device__ __forceinline__ void join_blocks(float* L, int r, int c, bool live) {
     __syncthreads();
 }
 
-// Row and first column of a lane's pair of neighbouring columns in the n-th of a warp's steps over the blocks of 16 x 16 on and left
-// of the diagonal, four warps sharing them: four rows a step in the first 16, two in the next, then one (in rows 32 to 47 the last
-// lanes have none: column 64).
-constexpr int DC_STEPS = 1 + 2 + 4 + 4;
-__device__ __forceinline__ int2 triangle_step(int n, int warp, int lane) {
-    if (n < 1) return make_int2(4 * warp + (lane >> 3), 2 * (lane & 7));
-    if (n < 3) return make_int2(16 + 8 * (n - 1) + 2 * warp + (lane >> 4), 2 * (lane & 15));
-    return make_int2(32 + 4 * (n - 3) + warp, n < 7 && lane >= 24 ? DC_T : 2 * lane);
-}
-__device__ __forceinline__ void store_parts(uint8_t* part, int2 at, float a, float b) {
-    uint32_t hi, mi, lo;
-    take_apart(a, b, hi, mi, lo);
-    uint8_t* dst = part + tile_off<DC_T>(at.x, at.y >> 3) + (at.y & 6) * 2;
-    *reinterpret_cast<uint32_t*>(dst) = hi;
-    *reinterpret_cast<uint32_t*>(dst + DC_PART) = mi;
-    *reinterpret_cast<uint32_t*>(dst + 2 * DC_PART) = lo;
-}
-
 // T and G of one chunk and the heads of one q/k head, two heads at a time, four warps each.
 template <int D>
 __global__ void __launch_bounds__(256, 3)
@@ -157,18 +128,9 @@ delta_chunk_prepare_kernel(const DeltaChunks m) {
     pdl_launch_dependents();
     pdl_wait();
     const int slot = blockIdx.x, kh = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // the last sequence whose first slot is not past this one (every warp looks for itself)
-    int s = -1;
-    for (int s0 = 0; s0 < m.n_seqs; s0 += 32) {
-        const int i = s0 + lane;
-        const unsigned before = __ballot_sync(0xffffffffu, i < m.n_seqs && m.cu_seqlens[i] / DC_T + i <= slot);
-        s += __popc(before);
-        if (before != 0xffffffffu) break;
-    }
-    const int begin = m.cu_seqlens[s], len = m.cu_seqlens[s + 1] - begin, j = slot - (begin / DC_T + s);
-    const int nt = min(DC_T, len - j * DC_T);
+    const Chunk64 at = chunk_of(m.cu_seqlens, m.n_seqs, slot);
+    const int first = at.first, nt = at.nt;
     if (nt <= 0) return;
-    const int first = begin + j * DC_T;
     const __nv_bfloat16* rows = m.qkv + (size_t)first * m.stride;
     const uint32_t kt = shared_u32(rest), qt = kt + TILE;
 #pragma unroll
@@ -223,28 +185,7 @@ delta_chunk_prepare_kernel(const DeltaChunks m) {
             rq_s[i] = 1.0f / sqrtf(sq + 1e-6f) * m.q_scale;
         }
     }
-    // k k^T and q k^T: the ten blocks of 16 x 16 on and left of the diagonal of each, a block a warp and turn
-    for (int n = warp; n < 20; n += 8) {
-        const int i = n % 10, bi = i < 1 ? 0 : i < 3 ? 1 : i < 6 ? 2 : 3, bj = i - bi * (bi + 1) / 2;
-        const uint32_t left = n < 10 ? kt : qt;
-        float c[2][2][4];                      // (even and odd steps apart: half the sums that are cut off)
-#pragma unroll
-        for (int e = 0; e < 16; ++e) c[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-            uint32_t a[4], b[4];
-            ldmatrix_x4(a, left + tile_off<D>(bi * 16 + (lane & 15), ks * 2 + (lane >> 4)));
-            ldmatrix_x4(b, kt + tile_off<D>(bj * 16 + (lane & 7) + (lane >> 4) * 8, ks * 2 + ((lane >> 3) & 1)));
-            mma16816(c[ks & 1][0], a, b[0], b[1]);
-            mma16816(c[ks & 1][1], a, b[2], b[3]);
-        }
-        float* out = (n < 10 ? kk : qk) + (bi * 16 + (lane >> 2)) * DC_LD + bj * 16 + 2 * (lane & 3);
-#pragma unroll
-        for (int t8 = 0; t8 < 2; ++t8) {
-            *reinterpret_cast<float2*>(out + t8 * 8) = make_float2(c[0][t8][0] + c[1][t8][0], c[0][t8][1] + c[1][t8][1]);
-            *reinterpret_cast<float2*>(out + 8 * DC_LD + t8 * 8) = make_float2(c[0][t8][2] + c[1][t8][2], c[0][t8][3] + c[1][t8][3]);
-        }
-    }
+    for (int n = warp; n < 20; n += 8) lower_block<D>(n < 10 ? kk : qk, n < 10 ? kt : qt, kt, n % 10, lane);
     float* L = reinterpret_cast<float*>(rest) + which * DC_T * DC_LD;
     for (int r0 = 0; r0 < per; r0 += 2) {
         const int h = kh * per + r0 + which;
@@ -371,13 +312,6 @@ __device__ __forceinline__ void dc_six(DcSums& c, const uint32_t (&a)[3][4], uin
     mma16816(c.lo[1], a[0], b[2][2], b[2][3]);
 }
 
-__device__ __forceinline__ void dc_cut(uint32_t (&a)[3][4], const float (&c0)[4], const float (&c1)[4]) {
-    cut_apart(c0[0], c0[1], a[0][0], a[1][0], a[2][0]);
-    cut_apart(c0[2], c0[3], a[0][1], a[1][1], a[2][1]);
-    cut_apart(c1[0], c1[1], a[0][2], a[1][2], a[2][2]);
-    cut_apart(c1[2], c1[3], a[0][3], a[1][3], a[2][3]);
-}
-
 // Shared memory of the walk (bytes): tiles, then what warps hand to each other in the registers' own layout ([..][lane] 16 bytes):
 // S's parts, a state warp's half of P, the parts of U and of U diag(A_end / A); the first token of a row that is not finite.
 template <int D, int PAIRS>
@@ -388,36 +322,6 @@ struct DcSmem {
     static constexpr int W = U + PAIRS * 4 * 3 * 512, ODD = W + PAIRS * 4 * 3 * 512, V = ODD + PAIRS * 2 * 16 * 4;
     static constexpr int ALL = V + DC_T * VROW;
 };
-
-__device__ __forceinline__ void dc_sync() { asm volatile("bar.sync 0;" ::: "memory"); }
-__device__ __forceinline__ void dc_give(uint8_t* at, const uint32_t (&a)[3][4]) {
-#pragma unroll
-    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(at + p * 512) = make_uint4(a[p][0], a[p][1], a[p][2], a[p][3]);
-}
-__device__ __forceinline__ void dc_take(uint32_t (&a)[3][4], const uint8_t* at) {
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        const uint4 v = *reinterpret_cast<const uint4*>(at + p * 512);
-        a[p][0] = v.x, a[p][1] = v.y, a[p][2] = v.z, a[p][3] = v.w;
-    }
-}
-template <int N>
-__device__ __forceinline__ void dc_zero(float (&c)[N][4]) {
-#pragma unroll
-    for (int n = 0; n < N; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) c[n][e] = 0.f;
-}
-// (high, rest) of two neighbouring tiles += a float's three parts times a 16-bit operand
-__device__ __forceinline__ void dc_three(float (&hi0)[4], float (&hi1)[4], float (&lo0)[4], float (&lo1)[4], const uint32_t (&a)[3][4],
-                                         const uint32_t (&b)[4]) {
-    mma16816(lo0, a[2], b[0], b[1]);
-    mma16816(lo1, a[2], b[2], b[3]);
-    mma16816(hi0, a[0], b[0], b[1]);
-    mma16816(hi1, a[0], b[2], b[3]);
-    mma16816(lo0, a[1], b[0], b[1]);
-    mma16816(lo1, a[1], b[2], b[3]);
-}
 
 // Four warps per 16 rows of V: two carry the state (each half of D's columns, and half of the chunk's tokens of U), two write the
 // outputs (half of the tokens each) one barrier behind them, and fetch the tiles.

@@ -17,8 +17,8 @@
 // every thread then walks the 16 tokens with multiply-adds only, leaves its
 // partial sums of S^T C in shared memory, and the block adds the slices' partial sums in a fixed
 // order. The walk's arithmetic does not depend on how a request's tokens were cut into steps: a
-// step continues from the stored S exactly where the step before left it. (Chunk by chunk, chunked.cuh,
-// sums have another order: the cut then moves results by a few 2^-24.)
+// step continues from the stored S exactly where the step before left it. (Chunk by chunk, chunked.cuh and, for
+// 16-bit rows, ssd_chunked.cu, sums have another order: the cut then moves results by a few 2^-24.)
 #include <math.h>
 
 #include "chunked.cuh"

@@ -1624,8 +1624,8 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
     n_state] (rows may be strided): x, then B, then C; ``dt_raw`` float32 [T, >= heads]; ``state`` float32 [slots,
     heads, n_state, v_dim]. Returns ``y`` float32 [parts, T, heads v_dim]: a step of few, long portions is walked
     by several blocks a head, each over a part of the state's rows, and their sums are still to be added
-    (``gated_group_norm`` does; ``y.sum(0)`` is the result). Few, long portions of states the chunked kernels take are formed
-    chunk by chunk instead (one part; ``ssd_by_chunks``). ``seq_lens``: the portions' lengths, where the host knows them."""
+    (``gated_group_norm`` does; ``y.sum(0)`` is the result). Portions of 48 tokens and more in 16-bit rows of whole 16-byte pieces, and few, long ones of any (``ssd_by_chunks``),
+    whose states the chunked kernels take are formed chunk by chunk instead (one part). ``seq_lens``: the portions' lengths, where the host knows them."""
     _cuda(xbc, dt_raw, dt_bias, a_log, d_skip, state)
     T = xbc.shape[0]
     if xbc.stride(1) != 1 or xbc.shape[1] < heads * v_dim + 2 * groups * n_state:
@@ -1634,6 +1634,17 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
         raise KernelError(f"ssd_scan: dt is float32 [{T}, >= {heads}]")
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, n_state, v_dim) or not state.is_contiguous():
         raise KernelError(f"ssd_scan: the state is float32 [slots, {heads}, {n_state}, {v_dim}]")
+    if xbc.dtype == torch.bfloat16 and xbc.stride(0) % 8 == 0 and xbc.data_ptr() % 16 == 0:
+        words = _lib.call("tk_ssd_tc_scratch", T, int(n_seqs), heads, v_dim, n_state, groups)
+        if words:
+            # portions of some length: chunk by chunk on the tensor cores
+            scratch = torch.empty(words, dtype=torch.float32, device=xbc.device)
+            y = torch.empty(1, T, heads * v_dim, dtype=torch.float32, device=xbc.device)
+            _lib.call("tk_ssd_tc", _ptr(xbc), xbc.stride(0), _ptr(dt_raw), dt_raw.stride(0), _ptr(_f32vec(dt_bias, "dt_bias", heads)),
+                      _ptr(_f32vec(a_log, "A_log", heads)), _ptr(_f32vec(d_skip, "D", heads)), _ptr(state),
+                      _ptr(_i32(cu_seqlens, "cu_seqlens")), _ptr(_i32(seq_ctx, "seq_ctx")), _ptr(_i32(seq_slot, "seq_slot")),
+                      int(n_seqs), T, _ptr(y), heads, v_dim, n_state, groups, _ptr(scratch), int(sm_count), _stream())
+            return y
     words = _lib.call("tk_ssd_chunked_scratch", T, int(n_seqs), heads, v_dim, n_state, groups)
     if (words and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0
             and ssd_by_chunks(T, heads, v_dim, seq_lens, sm_count)):

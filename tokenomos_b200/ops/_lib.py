@@ -111,6 +111,8 @@ _SIGNATURES = {
     "tk_ssd_max_state": [],
     "tk_ssd_scan": [P, L, P, L, P, P, P, P, P, P, P, I, I, P, I, I, I, I, I, I, P],
     "tk_ssd_chunked_scratch": [I, I, I, I, I, I],
+    "tk_ssd_tc_scratch": [I, I, I, I, I, I],
+    "tk_ssd_tc": [P, L, P, L, P, P, P, P, P, P, P, I, I, P, I, I, I, I, P, I, P],
     "tk_ssd_chunked": [P, L, P, L, P, P, P, P, P, P, P, I, I, P, I, I, I, I, P, I, P],
     "tk_ssd_split": [I, I, I, I, I, I],
     "tk_gated_group_norm": [P, I, P, L, P, F, P, I, I, I, I, P],
@@ -185,7 +187,7 @@ _QUERIES = {"tk_check_device", "tk_built_for", "tk_set_pdl", "tk_checks_enabled"
             "tk_attn_latent_mma_supported", "tk_attn_pointwise_rows", "tk_attn_pointwise_mma_supported",
             "tk_attn_pointwise_mma_tokens", "tk_ssd_max_state", "tk_ssd_split", "tk_linmem_max_dim", "tk_linmem_scratch", "tk_delta_chunks_scratch",
             "tk_attn_biased_mma_supported", "tk_attn_biased_mma_tokens", "tk_gemm_stream32_max_rows",
-            "tk_gemm_split32_status", "tk_attn_f32_supported", "tk_attn_f32_tokens", "tk_ssd_chunked_scratch"}
+            "tk_gemm_split32_status", "tk_attn_f32_supported", "tk_attn_f32_tokens", "tk_ssd_chunked_scratch", "tk_ssd_tc_scratch"}
 
 
 _fns: dict = {}
