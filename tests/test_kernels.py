@@ -460,6 +460,33 @@ def test_attention_f32_values_that_are_not_finite_reach_the_rows_that_see_them(H
         assert (got[:, :, rest] - was[:, :, rest]).norm() <= 1e-6 * was.norm()
 
 
+@pytest.mark.parametrize("window", [None, 700, -640])
+@pytest.mark.parametrize("H, Hkv, n", [(4, 4, 65), (16, 8, 33), (8, 1, 7)])
+def test_attention_f32_blocks_that_share_a_tile_s_keys(H, Hkv, n, window):
+    """Shares of a prompt tile's keys, tiles too short for all of them, keys that are not finite (their scores by multiply-adds),
+    queries and keys whose products overflow one way: against the general kernel, sums of up to 1,600 products in another order."""
+    from tokenomos_b200 import ops
+    ctx, P = 1503, 16
+    total = ctx + n
+    q, pool = torch.randn(n, H, 64, device="cuda"), torch.randn(-(-total // P), 2, Hkv, P, 64, device="cuda")
+    table, positions, seq = i32([list(range(pool.shape[0]))]), i32(list(range(ctx, total))), i32([0] * n)
+    firsts = lambda per: (i32(list(range(0, n, per)) + [0]), i32([min(per, n - o) for o in range(0, n, per)] + [0]))  # noqa: E731
+    for key, value in ((None, 0.0), (1490, float("-inf")), (1505, float("nan")), (2, float("inf")), (1500, 3e38)):
+        if key is not None:
+            pool[key // P, 0, :, key % P, 9] = value
+            q[1, :, 9] = -20.0
+        per = max(1, ops.attention_rows() // (H // Hkv))
+        want = ops.attention(q, pool, positions, seq, table, *firsts(per), per, window, 0.125)
+        for nsplit in (1, 2, 4, 8):
+            got = torch.full_like(q, float("nan"))
+            ops.attention_f32_prefill(q, pool, got, positions, seq, table, *firsts(ops.attention_f32_tokens(H, Hkv)), window, 0.125, nsplit)
+            assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+            fine = torch.isfinite(want)
+            assert (got[fine] - want[fine]).norm() <= 4e-6 * want[fine].norm()
+        if key is not None:
+            pool[key // P, 0, :, key % P, 9] = 0.5
+
+
 def test_swiglu32_vectorised_equals_the_scalar_kernel():
     """Whole and partial blocks of a row; rows that do not begin on 16 bytes go the scalar way, with the same bits."""
     from tokenomos_b200 import ops

@@ -307,15 +307,15 @@ def _check_attention_f32(q, kv_pool, out, name):
 
 def attention_f32_prefill(q: torch.Tensor, kv_pool: torch.Tensor, out: torch.Tensor, positions: torch.Tensor,
                           tok_seq: torch.Tensor, block_table: torch.Tensor, tile_tok0: torch.Tensor,
-                          tile_ntok: torch.Tensor, window: int | None, scale: float) -> None:
+                          tile_ntok: torch.Tensor, window: int | None, scale: float, nsplit: int = 1) -> None:
     """``attention`` for the tiles of prompt portions (at most ``attention_f32_tokens`` tokens each) of a 32-bit model with
-    heads of 64; writes those rows of ``out`` [T, H, 64]."""
+    heads of 64; writes those rows of ``out`` [T, H, 64]. Up to ``nsplit`` (1, 2, 4 or 8) blocks share a tile's keys."""
     _cuda(q, kv_pool, out, positions, tok_seq, block_table, tile_tok0, tile_ntok)
     T, H, D, Hkv, P = _check_attention_f32(q, kv_pool, out, "attention_f32_prefill")
     _lib.call("tk_attn_f32_prefill", _ptr(q), _ptr(kv_pool), _ptr(out), _ptr(_i32(positions, "positions")),
               _ptr(_i32(tok_seq, "tok_seq")), _ptr(_i32(block_table, "block_table")), block_table.stride(0),
               _ptr(_i32(tile_tok0, "tile_tok0")), _ptr(_i32(tile_ntok, "tile_ntok")), tile_tok0.numel(), H, Hkv, P,
-              int(window or 0), float(scale), _stream())
+              int(window or 0), float(scale), int(nsplit), _stream())
 
 
 def attention_f32_decode(q: torch.Tensor, kv_pool: torch.Tensor, out: torch.Tensor, positions: torch.Tensor,

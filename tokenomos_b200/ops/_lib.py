@@ -38,7 +38,7 @@ _SIGNATURES = {
     "tk_attn_generic": [P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, I, I, I, F, F, P, I, I, P],
     "tk_attn_f32_supported": [I, I, I],
     "tk_attn_f32_tokens": [I, I],
-    "tk_attn_f32_prefill": [P, P, P, P, P, P, I, P, P, I, I, I, I, I, F, P],
+    "tk_attn_f32_prefill": [P, P, P, P, P, P, I, P, P, I, I, I, I, I, F, I, P],
     "tk_attn_f32_decode": [P, P, P, P, P, P, I, P, I, I, I, I, I, F, I, P, P],
     "tk_rotary_write": [P, L, P, P, P, F, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P],
     "tk_stream32_add_norm": [P, P, L, P, P, P, F, P, P, P, I, I, I, P],

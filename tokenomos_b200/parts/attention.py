@@ -381,9 +381,12 @@ class Attention:
         """32-bit models with heads of 64: prompt portions in tiles of 64 rows, single tokens shared out over their keys."""
         out = torch.empty_like(q)
         if not ctx.host.decode_only:
-            _, tok0, _, ntok = ctx.tiles(ops.attention_f32_tokens(self.heads, self.kv_heads), "multi")
+            per_tile = ops.attention_f32_tokens(self.heads, self.kv_heads)
+            _, tok0, _, ntok = ctx.tiles(per_tile, "multi")
             if tok0.numel():
-                ops.attention_f32_prefill(q, pool, out, ctx.positions, ctx.tok_seq, table, tok0, ntok, self.reach, self.scale)
+                longest = min(ctx.host.longest, self.span) if self.span is not None else ctx.host.longest
+                nsplit = self.prefill_f32_splits(ctx.n_tokens, per_tile, self.kv_heads, longest, self.tuning)
+                ops.attention_f32_prefill(q, pool, out, ctx.positions, ctx.tok_seq, table, tok0, ntok, self.reach, self.scale, nsplit)
         singles = None if ctx.host.decode_only else ctx.singles()
         rows = ctx.n_tokens if singles is None else singles.numel()
         if rows:
@@ -501,6 +504,19 @@ class Attention:
         per_split = max(1, rows * kv_heads)
         resident = tuning.decode_fused_ctas_per_sm * tuning.sm_count // per_split
         return max(1, min(resident, -(-longest // tuning.decode_min_keys)))
+
+    @staticmethod
+    def prefill_f32_splits(tokens: int, per_tile: int, kv_heads: int, longest: int, tuning: Tuning = DEFAULT_TUNING) -> int:
+        """The most blocks that may share one tile's keys in the 32-bit prompt kernel, two of which an SM holds: while all blocks
+        are no more than 4.8 an SM and each keeps four tiles of 64 keys (the kernel gives a tile as many as leave each three).
+        16 heads over 8 (us, unshared in brackets): 33 tokens behind 2,500 positions 37 shared by eight (171), 128 behind 4,000 59
+        (275), 700 behind 2,500 226 by four (297), a prompt of 1,000 73 by two (92), of 300 26 unshared (29 by two), of 2,048
+        190 unshared (216 by two)."""
+        ctas = max(1, -(-tokens // per_tile)) * max(1, kv_heads)
+        split = 1
+        while split < 8 and 10 * ctas * split * 2 <= 48 * tuning.sm_count and longest >= split * 2 * 4 * 64:
+            split *= 2
+        return split
 
     @staticmethod
     def prefill_splits(tokens: int, entries: int, per_tile: int, kv_heads: int,
