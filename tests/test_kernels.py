@@ -1045,6 +1045,16 @@ def test_attention_tc_prefill_with_a_tiles_keys_shared_by_several_ctas(H, Hkv, P
         assert int(ops._tickets[got.device].abs().sum()) == 0
 
 
+@pytest.mark.parametrize("P", [4, 8, 128])
+@pytest.mark.parametrize("split, window", [(1, None), (16, None), (16, 70), (1, 130)])
+def test_attention_tc_prefill_pages_and_shares(P, split, window):
+    """Pages smaller than a TMA load takes, of one load, and of several tiles, rows beside the positions NaN: ragged first and last
+    tiles, one tile alone (the second softmax group has none), an odd number of them, more CTAs than shares of eight tiles."""
+    seqs = [(0, 3), (61, 2), (64, 64), (130, 70), (9000, 35), (4095, 33), (0, 129)]
+    got, want = attention_mma_case(16, 4, 64, P, seqs, window=window, tc=True, tc_split=split)
+    close(got, want, torch.bfloat16, f"tcgen05 prefill P{P} split {split} window {window}")
+
+
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_tc_prefill_window_and_far_key(window):
     seqs = [(0, 150), (20, 30), (3, 2), (200, 70)]

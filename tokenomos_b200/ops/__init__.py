@@ -567,24 +567,17 @@ def attention_prefill_tc(q: torch.Tensor, kv_pool: torch.Tensor, out: torch.Tens
     """``attention_prefill_mma`` on tcgen05.mma with the accumulators in tensor memory, for tiles
     of ``attention_prefill_tc_tokens`` tokens of one sequence; writes the tiles' rows of ``out``
     (gated like ``attention_prefill_mma``'s; ``keep_first``, ``sink``, ``gate_by_element`` as
-    there). ``nsplit`` > 1: that many CTAs share each tile's keys and the last one to finish
-    merges their shares (through scratch memory that this function allocates): for steps with
-    few tiles behind long contexts."""
+    there). ``nsplit`` > 1: up to that many CTAs (in powers of two, at most 8) share each tile's keys and merge
+    their shares through each other's shared memory: for steps with few tiles behind long contexts."""
     _cuda(q, kv_pool, out, positions, tok_seq, block_table, tile_tok0, tile_ntok)
     T, H, D, Hkv, P = _check_attention(q, kv_pool, "attention_prefill_tc")
     g_ptr, ldg, mode = _gate_options(gate, gate_by_element, T, H, D, "attention_prefill_tc")
     n_tiles = tile_tok0.numel()
-    nsplit = max(1, int(nsplit))
-    scratch = tickets = None
-    if nsplit > 1 and n_tiles:
-        scratch = torch.empty(n_tiles * Hkv * nsplit * (128 * D + 256), dtype=torch.float32, device=q.device)
-        tickets = _decode_tickets(n_tiles * Hkv, q.device)
     _lib.call("tk_attn_prefill_tc_opt", _ptr(q), _ptr(kv_pool), _ptr(out), _ptr(_i32(positions, "positions")),
               _ptr(_i32(tok_seq, "tok_seq")), _ptr(_i32(block_table, "block_table")),
               block_table.stride(0), _ptr(_i32(tile_tok0, "tile_tok0")),
               _ptr(_i32(tile_ntok, "tile_ntok")), n_tiles, H, Hkv, D, P, int(window or 0),
-              float(scale), g_ptr, ldg, nsplit, _ptr(scratch), _ptr(tickets), int(keep_first), int(bool(sink)),
-              mode, _stream())
+              float(scale), g_ptr, ldg, max(1, int(nsplit)), int(keep_first), int(bool(sink)), mode, _stream())
 
 
 def attention_prefill_tc_status() -> int:
@@ -625,16 +618,21 @@ def attention_decode_fused_supported(heads: int, kv_heads: int, head_dim: int, r
 
 # per device: [n * kv_heads] zeros the fused decode kernel counts finished splits in and zeroes
 # again; a buffer that a captured step may point at is never freed, only outgrown
-_tickets: dict = {}
+class _Tickets(dict):
+    def __missing__(self, device: torch.device) -> torch.Tensor:
+        self[device] = made = torch.zeros(4096, dtype=torch.int32, device=device)
+        return made
+
+
+_tickets = _Tickets()
 _tickets_outgrown: list = []
 
 
 def _decode_tickets(n: int, device: torch.device) -> torch.Tensor:
-    have = _tickets.get(device)
-    if have is None or have.numel() < n:
-        if have is not None:
-            _tickets_outgrown.append(have)
-        have = _tickets[device] = torch.zeros(max(n, 4096), dtype=torch.int32, device=device)
+    have = _tickets[device]
+    if have.numel() < n:
+        _tickets_outgrown.append(have)
+        have = _tickets[device] = torch.zeros(n, dtype=torch.int32, device=device)
     return have
 
 

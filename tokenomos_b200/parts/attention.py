@@ -526,9 +526,9 @@ class Attention:
         longer than what it uses). A tile is walked by one CTA, key tile after key tile; a step
         with few tiles behind a long context would leave the GPU idle for hundreds of
         microseconds (128 tokens behind 32,000 positions: 474 us a layer, 98 us shared 8 ways).
-        So: as many as fill the GPU once (``prefill_split_ctas_per_sm`` CTAs an SM), no more than
-        the scratch memory for the shares allows; the kernel gives each tile as many of them as
-        leave a CTA 8 key tiles, so a short context uses one whatever this says."""
+        So: as many as fill the GPU once (``prefill_split_ctas_per_sm`` CTAs an SM), fewer where a long list of tiles leaves
+        most of a launch without work (``prefill_split_scratch_mb``, once the shares' memory); the kernel takes the next
+        power of two below, at most 8, and gives each tile as many of them as leave a CTA 8 key tiles."""
         tiles = max(1, -(-tokens // per_tile))
         by_ctas = tuning.prefill_split_ctas_per_sm * tuning.sm_count // (tiles * max(1, kv_heads))
         by_memory = (tuning.prefill_split_scratch_mb << 20) // (max(1, entries) * max(1, kv_heads) * 128 * 66 * 4)
@@ -549,7 +549,9 @@ class Attention:
             self.heads, self.kv_heads)
         _, tok0, _, ntok = ctx.tiles(per_tile, "multi")
         if tok0.numel() and tc:
-            nsplit = self.prefill_splits(ctx.n_tokens, tok0.numel(), per_tile, self.kv_heads, self.tuning)
+            # (a cluster that no tile is long enough for costs 1 to 3 us)
+            longest = min(ctx.host.longest, self.span) if self.span is not None else ctx.host.longest
+            nsplit = min(self.prefill_splits(ctx.n_tokens, tok0.numel(), per_tile, self.kv_heads, self.tuning), max(1, longest // 480))
             ops.attention_prefill_tc(q, pool, out, ctx.positions, ctx.tok_seq, table, tok0, ntok, self.reach,
                                      self.scale, gate, nsplit, self.keep_first, self.sink, by_element)
         elif tok0.numel():
