@@ -3,21 +3,21 @@
 //
 // Such a product is bound by the stream of weight bytes (eight multiply-adds a weight at most, 128 lanes an SM:
 // a third of what the cores can do at the copy bandwidth), so the split is the one that reads every weight row in
-// whole 128-byte lines with many loads in flight: a CTA owns 4 weight rows and all of K, its 8 warps take alternate
-// 128-wide slices of K, a lane 4 neighbouring columns of all 4 rows, two slices asked for together. The activations
+// whole 128-byte lines with many loads in flight: a CTA owns 2 to 8 weight rows and all of K, its 8 warps take alternate
+// 128-wide slices of K, a lane 4 neighbouring columns of all rows, one to four slices asked for together (launch_stream32). The activations
 // (64 KB at most for 8 rows of 2,048) are read the same way through L1. A lane then holds 4 x M partial sums; the
 // warp adds them up with a halving exchange (31 shuffles for 32 sums instead of 160), the warps through shared memory.
-// SWIGLU: the rows of W are all gate rows, then all up rows; the CTA takes 2 channels of both and writes
+// SWIGLU: the rows of W are all gate rows, then all up rows; the CTA takes as many channels of both and writes
 // silu(gate) * up, so a decoded token needs no activation kernel.
 //
 // The kernel this replaces up to 8 rows (a 64 x 64 tile of gemm_simt.cu) filled its tile with rows that do not exist
 // and ran N / 64 CTAs: the feed-forward of 1,024 x 4,608 at one row took 416 us in three launches, with this kernel
-// 15.8 us in two (3.6 TB/s of weights).
+// 13.7 us in two (4.1 TB/s of weights).
 #include "common.cuh"
 
 namespace {
 
-constexpr int S32_WARPS = 8, S32_ROWS = 4, S32_SLICE = 128, S32_UNROLL = 2;
+constexpr int S32_WARPS = 8, S32_SLICE = 128;
 
 __device__ __forceinline__ float4 ld_weights(const float* p) {
     float4 v;
@@ -45,22 +45,23 @@ __device__ __forceinline__ float halving_sum(float (&v)[V], int lane) {
     return s;
 }
 
-template <int MT, bool SWIGLU>
-__global__ void __launch_bounds__(S32_WARPS * 32)
+// ROWS weight rows a CTA, UNROLL slices of K a warp asked for together (see launch_stream32)
+template <int MT, bool SWIGLU, int ROWS, int UNROLL>
+__global__ void __launch_bounds__(S32_WARPS * 32, MT == 8 && UNROLL == 1 ? 4 : 0)
 gemm_stream32_kernel(const float* x, int64_t ldx, const float* __restrict__ w, int64_t ldw,
                      const float* __restrict__ bias, float* out, int64_t ldo, int M, int N, int K) {
-    constexpr int V = S32_ROWS * MT;
+    constexpr int V = ROWS * MT;
     __shared__ float red[S32_WARPS][V];
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // the CTA's rows of W: 4 neighbours, or 2 gate rows and the up rows of the same channels
+    // the CTA's rows of W: neighbours, or half as many gate rows and the up rows of the same channels
     const int channels = SWIGLU ? N / 2 : N;
-    constexpr int OWN = SWIGLU ? S32_ROWS / 2 : S32_ROWS;
+    constexpr int OWN = SWIGLU ? ROWS / 2 : ROWS;
     const int c0 = blockIdx.x * OWN;
-    const float* wr[S32_ROWS];
-    int row[S32_ROWS];
+    const float* wr[ROWS];
+    int row[ROWS];
 #pragma unroll
-    for (int r = 0; r < S32_ROWS; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         const int c = c0 + r % OWN;
         row[r] = min(c, channels - 1) + (r / OWN) * channels;       // (a row past the end repeats the last one)
         wr[r] = w + (size_t)row[r] * ldw;
@@ -70,20 +71,20 @@ gemm_stream32_kernel(const float* x, int64_t ldx, const float* __restrict__ w, i
     for (int i = 0; i < V; ++i) acc[i] = 0.f;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     bool waited = false;
-    for (int k0 = warp * S32_SLICE; k0 < K; k0 += S32_WARPS * S32_SLICE * S32_UNROLL) {
-        float4 wv[S32_UNROLL][S32_ROWS];
+    for (int k0 = warp * S32_SLICE; k0 < K; k0 += S32_WARPS * S32_SLICE * UNROLL) {
+        float4 wv[UNROLL][ROWS];
 #pragma unroll
-        for (int u = 0; u < S32_UNROLL; ++u) {
+        for (int u = 0; u < UNROLL; ++u) {
             const int k = k0 + u * S32_WARPS * S32_SLICE + lane * 4;
 #pragma unroll
-            for (int r = 0; r < S32_ROWS; ++r) wv[u][r] = k < K ? ld_weights(wr[r] + k) : zero;
+            for (int r = 0; r < ROWS; ++r) wv[u][r] = k < K ? ld_weights(wr[r] + k) : zero;
         }
         if (!waited) {                    // the weights are no kernel's output, the activations are
             pdl_wait();
             waited = true;
         }
 #pragma unroll
-        for (int u = 0; u < S32_UNROLL; ++u) {
+        for (int u = 0; u < UNROLL; ++u) {
             const int k = k0 + u * S32_WARPS * S32_SLICE + lane * 4;
             if (k >= K) continue;         // (zero weights would turn an infinite activation into NaN)
 #pragma unroll
@@ -91,7 +92,7 @@ gemm_stream32_kernel(const float* x, int64_t ldx, const float* __restrict__ w, i
                 if (m >= M) break;
                 const float4 xv = *reinterpret_cast<const float4*>(x + (size_t)m * ldx + k);
 #pragma unroll
-                for (int r = 0; r < S32_ROWS; ++r) {
+                for (int r = 0; r < ROWS; ++r) {
                     float a = acc[r * MT + m];
                     a = fmaf(wv[u][r].x, xv.x, a);
                     a = fmaf(wv[u][r].y, xv.y, a);
@@ -111,7 +112,7 @@ gemm_stream32_kernel(const float* x, int64_t ldx, const float* __restrict__ w, i
 #pragma unroll
         for (int wv = 0; wv < S32_WARPS; ++wv) {
             sum += red[wv][r * MT + m];
-            if (SWIGLU) up += red[wv][(r + OWN) % S32_ROWS * MT + m];
+            if (SWIGLU) up += red[wv][(r + OWN) % ROWS * MT + m];
         }
         if (bias != nullptr) {
             sum += bias[c0 + r];
@@ -121,17 +122,31 @@ gemm_stream32_kernel(const float* x, int64_t ldx, const float* __restrict__ w, i
     }
 }
 
+// 4 rows a CTA and two slices a warp in flight, but where all of K is one slice a warp (1,024 columns), or several rounds of two.
+// Up to 1,024 columns: 8 rows for one to four tokens (one wave of CTAs instead of two; us at 9,216 x 1,024, SwiGLU: one token 7.0,
+// with 4 rows 9.3, two 7.8 and 8.4, four 10.9 and 11.4; two tokens from 8,192 rows on, four from 4,096), for more of them one slice's
+// registers and so four CTAs an SM (eight tokens 13.5 and 18.9; from 2,048 rows on, 1,024 x 1,024 3.5 and 2.9). One token beyond
+// 2,048 columns: four slices in flight (4,096 x 4,096 11.7 and 13.1), and 2 rows a CTA where the matrix has few (1,024 x 4,608
+// 3.8 and 4.9, 2,048 x 10,752 14.0 and 16.4); two tokens and more are slower that way (2,048 x 8,192 15.5 and 11.8).
 template <bool SWIGLU>
 void launch_stream32(const float* x, int64_t ldx, const float* w, int64_t ldw, const float* bias, float* out, int64_t ldo,
                      int M, int N, int K, cudaStream_t stream) {
-    constexpr int OWN = SWIGLU ? S32_ROWS / 2 : S32_ROWS;
-    const dim3 grid(ceil_div(SWIGLU ? N / 2 : N, OWN)), block(S32_WARPS * 32);
-#define TK_S32(MT) \
-    tk_launch(gemm_stream32_kernel<MT, SWIGLU>, grid, block, 0, stream, x, ldx, w, ldw, bias, out, ldo, M, N, K)
-    if (M == 1) TK_S32(1);
-    else if (M == 2) TK_S32(2);
-    else if (M <= 4) TK_S32(4);
-    else TK_S32(8);
+#define TK_S32(MT, ROWS, UNROLL)                                                                                              \
+    tk_launch(gemm_stream32_kernel<MT, SWIGLU, ROWS, UNROLL>, dim3(ceil_div(SWIGLU ? N / 2 : N, SWIGLU ? ROWS / 2 : ROWS)),   \
+              dim3(S32_WARPS * 32), 0, stream, x, ldx, w, ldw, bias, out, ldo, M, N, K)
+    const int once = S32_WARPS * S32_SLICE;
+#define TK_S32_K(MT)                                                                                              \
+    do {                                                                                                          \
+        if (K <= once && N >= (MT == 1 ? 0 : MT == 2 ? 8192 : MT == 4 ? 4096 : 2048)) TK_S32(MT, (MT <= 4 ? 8 : 4), 1); \
+        else if (MT == 1 && K > 2 * once && N <= 2048) TK_S32(MT, (MT == 1 ? 2 : 4), (MT == 1 ? 4 : 2));          \
+        else if (MT == 1 && K > 2 * once) TK_S32(MT, 4, (MT == 1 ? 4 : 2));                                       \
+        else TK_S32(MT, 4, 2);                                                                                    \
+    } while (0)
+    if (M == 1) TK_S32_K(1);
+    else if (M == 2) TK_S32_K(2);
+    else if (M <= 4) TK_S32_K(4);
+    else TK_S32_K(8);
+#undef TK_S32_K
 #undef TK_S32
 }
 
