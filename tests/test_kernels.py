@@ -218,6 +218,14 @@ def test_gemm_stream32(m, n, k, swiglu):
     assert torch.isinf(got[0]).all() and torch.isfinite(got[1:]).all()
 
 
+@pytest.mark.parametrize("m, n, k", [(1, 1030, 2052), (1, 2050, 4100), (4, 2374, 1028), (3, 1778, 2052), (4, 2370, 1028), (5, 1186, 1024),
+                                     (8, 1186, 1032), (2, 8194, 132), (4, 4098, 1024), (5, 1184, 1024)])
+def test_gemm_stream32_at_the_edges_of_its_waves(m, n, k):
+    """Every number of rows a CTA and of slices in flight, at the first sizes that take it."""
+    for swiglu in (False, True):
+        test_gemm_stream32(m, n, k, swiglu)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_scale_rows_and_logit_options(dtype):
     from tokenomos_b200 import ops

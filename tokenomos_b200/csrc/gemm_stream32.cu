@@ -47,7 +47,7 @@ __device__ __forceinline__ float halving_sum(float (&v)[V], int lane) {
 
 // ROWS weight rows a CTA, UNROLL slices of K a warp asked for together (see launch_stream32)
 template <int MT, bool SWIGLU, int ROWS, int UNROLL>
-__global__ void __launch_bounds__(S32_WARPS * 32, MT == 8 && UNROLL == 1 ? 4 : 0)
+__global__ void __launch_bounds__(S32_WARPS * 32, MT >= 4 && ROWS == 4 && UNROLL == 1 ? 4 : 0)
 gemm_stream32_kernel(const float* x, int64_t ldx, const float* __restrict__ w, int64_t ldw,
                      const float* __restrict__ bias, float* out, int64_t ldo, int M, int N, int K) {
     constexpr int V = ROWS * MT;
@@ -122,24 +122,29 @@ gemm_stream32_kernel(const float* x, int64_t ldx, const float* __restrict__ w, i
     }
 }
 
-// 4 rows a CTA and two slices a warp in flight, but where all of K is one slice a warp (1,024 columns), or several rounds of two.
-// Up to 1,024 columns: 8 rows for one to four tokens (one wave of CTAs instead of two; us at 9,216 x 1,024, SwiGLU: one token 7.0,
-// with 4 rows 9.3, two 7.8 and 8.4, four 10.9 and 11.4; two tokens from 8,192 rows on, four from 4,096), for more of them one slice's
-// registers and so four CTAs an SM (eight tokens 13.5 and 18.9; from 2,048 rows on, 1,024 x 1,024 3.5 and 2.9). One token beyond
-// 2,048 columns: four slices in flight (4,096 x 4,096 11.7 and 13.1), and 2 rows a CTA where the matrix has few (1,024 x 4,608
-// 3.8 and 4.9, 2,048 x 10,752 14.0 and 16.4); two tokens and more are slower that way (2,048 x 8,192 15.5 and 11.8).
+// 4 rows a CTA and two slices a warp in flight, but:
+// - up to 1,024 columns (one slice a warp) 8 rows for one to four tokens, one wave of CTAs instead of two (us at 9,216 x 1,024, SwiGLU:
+//   one token 7.0, with 4 rows 9.3, two 7.8 and 8.4, four 10.9 and 11.4; two tokens from 8,192 rows on, four from 4,096);
+// - one token beyond 2,048 columns four slices (4,096 x 4,096 11.7 and 13.1), and 2 rows a CTA where the matrix has few (1,024 x 4,608
+//   3.8 and 4.9, 2,048 x 10,752 14.0 and 16.4; two tokens and more are slower that way, 2,048 x 8,192 15.5 and 11.8);
+// - more than two tokens one slice, whose registers let four CTAs share an SM instead of two (three with four tokens), where the
+//   matrix has more rows than those hold at once (eight tokens: 2,048 x 8,192 21.1 and 31.4, 16,384 x 2,048 36.3 and 44.2, 9,216 x
+//   1,024 13.5 and 18.9, 1,024 x 4,608 12.3 and 10.5; four: 2,048 x 8,192 13.7 and 20.6), with four tokens and up to 2,048 columns only
+//   while four CTAs an SM are all there are (2,048 x 2,048 4.3 and 6.5, 3,072 x 2,048 7.8 and 7.1).
 template <bool SWIGLU>
 void launch_stream32(const float* x, int64_t ldx, const float* w, int64_t ldw, const float* bias, float* out, int64_t ldo,
                      int M, int N, int K, cudaStream_t stream) {
 #define TK_S32(MT, ROWS, UNROLL)                                                                                              \
     tk_launch(gemm_stream32_kernel<MT, SWIGLU, ROWS, UNROLL>, dim3(ceil_div(SWIGLU ? N / 2 : N, SWIGLU ? ROWS / 2 : ROWS)),   \
               dim3(S32_WARPS * 32), 0, stream, x, ldx, w, ldw, bias, out, ldo, M, N, K)
-    const int once = S32_WARPS * S32_SLICE;
+    const int once = S32_WARPS * S32_SLICE, wave = 4 * 148;          // columns of one slice a warp; rows of a CTA an SM
 #define TK_S32_K(MT)                                                                                              \
     do {                                                                                                          \
-        if (K <= once && N >= (MT == 1 ? 0 : MT == 2 ? 8192 : MT == 4 ? 4096 : 2048)) TK_S32(MT, (MT <= 4 ? 8 : 4), 1); \
+        if (MT <= 4 && K <= once && N >= (MT == 1 ? 0 : MT == 2 ? 8192 : 4096)) TK_S32(MT, (MT <= 4 ? 8 : 4), 1); \
         else if (MT == 1 && K > 2 * once && N <= 2048) TK_S32(MT, (MT == 1 ? 2 : 4), (MT == 1 ? 4 : 2));          \
         else if (MT == 1 && K > 2 * once) TK_S32(MT, 4, (MT == 1 ? 4 : 2));                                       \
+        else if ((MT == 8 && N > 2 * wave) || (MT == 4 && K > once && N > 3 * wave && (K > 2 * once || N <= 4 * wave))) \
+            TK_S32(MT, 4, (MT >= 4 ? 1 : 2));                                                                     \
         else TK_S32(MT, 4, 2);                                                                                    \
     } while (0)
     if (M == 1) TK_S32_K(1);
