@@ -1063,6 +1063,24 @@ def test_attention_tc_prefill_pages_and_shares(P, split, window):
     close(got, want, torch.bfloat16, f"tcgen05 prefill P{P} split {split} window {window}")
 
 
+def test_attention_tc_prefill_waits_for_its_last_products():
+    """One to eight key tiles a tile of queries, the weight on the last two, whose products are the ones a softmax group may find
+    unfinished: every one is in the output, and a second launch gives the same bits."""
+    seqs = [(64 * n - 20, 20) for n in range(1, 9)]
+
+    def boost(s, q, k, v):                                     # queries look along one direction, and the last 100 keys lie there
+        q[:, :, 0] = 8.0
+        k[-100:, :, 0] = 6.0
+
+    state = torch.random.get_rng_state()
+    first, want = attention_mma_case(32, 8, 64, 16, seqs, tc=True, boost=boost)
+    close(first, want, torch.bfloat16, "the last two key tiles")
+    for _ in range(3):
+        torch.random.set_rng_state(state)
+        again, _ = attention_mma_case(32, 8, 64, 16, seqs, tc=True, boost=boost)
+        assert torch.equal(again.view(torch.int16), first.view(torch.int16))
+
+
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_tc_prefill_window_and_far_key(window):
     seqs = [(0, 150), (20, 30), (3, 2), (200, 70)]

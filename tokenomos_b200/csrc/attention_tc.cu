@@ -490,7 +490,12 @@ attn_prefill_tc_kernel(const __nv_bfloat16* q, const __nv_bfloat16* pool, __nv_b
             if (lane == 0) mbar_arrive(p_full(b));
         }
         if (ok && n_tiles > grp) {
-            ok = at_wait(pv_full(grp), (uint32_t)(((n_tiles - 1 - grp) >> 1) & 1), 8);
+            // A wait names its phase by one bit, so the phase before has to be over first. Within the walk it is: the product of the tile
+            // before the last of this group was committed ahead of the scores of this one. But the commit of the product just before the
+            // last is issued behind the last scores, and while it is open the last phase's bit reads as over.
+            const int turn = (n_tiles - 1 - grp) >> 1;
+            if (turn > 0) ok = at_wait(pv_full(grp), (uint32_t)((turn - 1) & 1), 8);
+            if (ok) ok = at_wait(pv_full(grp), (uint32_t)(turn & 1), 8);
             ok = __all_sync(0xffffffffu, ok);
         }
         // The second group's maximum and sum of each row go to Q's tile, which no product reads any more: the last S of either group
