@@ -1081,6 +1081,28 @@ def test_attention_tc_prefill_waits_for_its_last_products():
         assert torch.equal(again.view(torch.int16), first.view(torch.int16))
 
 
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+@pytest.mark.parametrize("which, value", [("key", float("nan")), ("value", float("nan")), ("value", float("inf"))])
+def test_attention_tc_prefill_not_finite_behind_a_factor_of_zero(split, which, value):
+    """A key or value that is not finite among keys whose scores lie 288 (log2) below the others', so that a share of the keys that holds
+    only such ones is merged with a factor of 0: the rows that see it are not finite, as with one share; another sequence's are untouched."""
+    seqs = [(64 * 64, 33), (64 * 64 + 20, 2)]
+    every = split if split > 1 else 8
+    low = [j for t in range(3 % every, 64, every) for j in range(64 * t, 64 * t + 64)]        # the tiles of one share
+
+    def boost(s, q, k, v):
+        q[:, :, 0], k[:, :, 0] = 40.0, 0.0
+        k[low, :, 0] = -40.0
+        if s == 0:
+            (k if which == "key" else v)[low[70], :, 5] = value
+
+    got, want = attention_mma_case(8, 2, 64, 16, seqs, tc=True, tc_split=split, boost=boost)
+    assert not torch.isfinite(got[:33, :, 5].float()).any()
+    if which == "key":
+        assert torch.isnan(got[:33].float()).all()
+    close(got[33:], want[33:], torch.bfloat16, "the sequence beside it")
+
+
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_tc_prefill_window_and_far_key(window):
     seqs = [(0, 150), (20, 30), (3, 2), (200, 70)]

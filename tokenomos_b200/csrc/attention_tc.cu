@@ -608,8 +608,10 @@ attn_prefill_tc_kernel(const __nv_bfloat16* q, const __nv_bfloat16* pool, __nv_b
                 for (int sp = 0; sp < NS; ++sp) M = fmaxf(M, ml[sp].x);
 #pragma unroll
                 for (int sp = 0; sp < NS; ++sp) {
-                    ml[sp].x = ml[sp].x == -INFINITY ? 0.f : fast_exp2(ml[sp].x - M);          // (0: nothing visible in that share)
-                    L = fmaf(ml[sp].y, ml[sp].x, L);
+                    // a row that sees nothing of a share leaves it out (-1); any other takes part, also under a factor of 0: a key or
+                    // value that is not finite reaches the rows that see it, whichever CTA walked it
+                    ml[sp].x = ml[sp].x == -INFINITY && ml[sp].y == 0.f ? -1.f : fast_exp2(ml[sp].x - M);
+                    L = ml[sp].x < 0.f ? L : fmaf(ml[sp].y, ml[sp].x, L);
                 }
                 const float inv = L > 0.f ? 1.0f / L : 0.f;
                 if (r >= rows) return;
@@ -620,7 +622,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* q, const __nv_bfloat16* pool, __nv_b
 #pragma unroll
                     for (int sp = 0; sp < NS; ++sp)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) v[e] = ml[sp].x == 0.f ? v[e] : fmaf((&o[sp][k].x)[e], ml[sp].x, v[e]);
+                        for (int e = 0; e < 4; ++e) v[e] = ml[sp].x < 0.f ? v[e] : fmaf((&o[sp][k].x)[e], ml[sp].x, v[e]);
                     uint2 packed;
                     if (X && opt.gate_mode == 2) {
                         const uint2 raw = *reinterpret_cast<const uint2*>(gate + (size_t)tok * ldg + (size_t)head * AT_D + c);
