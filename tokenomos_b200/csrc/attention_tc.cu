@@ -336,10 +336,11 @@ attn_prefill_tc_kernel(const __nv_bfloat16* q, const __nv_bfloat16* pool, __nv_b
                                      (j > 1 || k > 0) ? 1u : 0u);
                 }
                 __syncwarp();
-                // (in order behind the product that reads P_j, where S_{j+2} goes; it is what the group waits for)
+                // (in order behind the product that reads P_j, where S_{j+2} goes; the group's next wait is for it, and for that product)
                 if (j + 2 < n_tiles) issue_s(j + 2);
+                // (one phase of pv_full: a group that skipped phases could not tell by a phase's one bit which is open)
                 if (elect_lane()) {
-                    umma_commit(pv_full(b));
+                    if (j + 2 >= n_tiles) umma_commit(pv_full(b));
                     umma_commit(kv_empty(s));
                 }
                 __syncwarp();
@@ -429,10 +430,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* q, const __nv_bfloat16* pool, __nv_b
                     l_run.x *= alpha0;
                 }
                 if (turn >= 1) {
-                    // the product of the group's tile before must have landed before the output is touched
-                    if (ok) ok = at_wait(pv_full(b), (uint32_t)((turn - 1) & 1), 7);
-                    ok = __all_sync(0xffffffffu, ok);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    // (the product of the group's tile before has landed: it was issued ahead of these scores, whose commit covers both)
                     const float alpha = m_new == -INFINITY ? 1.0f : fast_exp2(m_ref - m_new);
 #pragma unroll
                     for (int c = 0; c < AT_D; c += 16) {          // (narrow: the scores stay in registers)
@@ -490,12 +488,7 @@ attn_prefill_tc_kernel(const __nv_bfloat16* q, const __nv_bfloat16* pool, __nv_b
             if (lane == 0) mbar_arrive(p_full(b));
         }
         if (ok && n_tiles > grp) {
-            // A wait names its phase by one bit, so the phase before has to be over first. Within the walk it is: the product of the tile
-            // before the last of this group was committed ahead of the scores of this one. But the commit of the product just before the
-            // last is issued behind the last scores, and while it is open the last phase's bit reads as over.
-            const int turn = (n_tiles - 1 - grp) >> 1;
-            if (turn > 0) ok = at_wait(pv_full(grp), (uint32_t)((turn - 1) & 1), 8);
-            if (ok) ok = at_wait(pv_full(grp), (uint32_t)(turn & 1), 8);
+            ok = at_wait(pv_full(grp), 0, 8);
             ok = __all_sync(0xffffffffu, ok);
         }
         // The second group's maximum and sum of each row go to Q's tile, which no product reads any more: the last S of either group
@@ -671,7 +664,7 @@ TK_API int tk_attn_prefill_tc_supported(int H, int Hkv, int D) {
 TK_API int tk_attn_prefill_tc_tokens(int H, int Hkv) { return AT_ROWS / (H / Hkv); }
 
 // 0, or where a CTA gave up waiting on a barrier since the last call (1 and 10 staging, 2-4 MMA issuer,
-// 5-8 softmax, 9 shared memory out of place). Resets the word.
+// 6 and 8 softmax, 9 shared memory out of place). Resets the word.
 TK_API int tk_attn_prefill_tc_status() {
     int v = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_at_error, sizeof(int)) != cudaSuccess) return -1;
