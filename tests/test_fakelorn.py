@@ -1144,6 +1144,26 @@ def test_norms_with_a_gate_at_the_edges_of_their_forms(groups, part, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("C, shift", [(512, 0), (512, 1), (8, 0)])
+def test_silu_of_the_convolution_and_the_gated_norm_to_its_last_normal_numbers(C, shift):
+    """silu of 16-bit arguments down to -88.5, where the exponential is near the largest number and its reciprocal is none of the normal
+    ones: one rounding to the storage type of the exact value, four channels or elements a thread or one (rows off 8 bytes)."""
+    from tokenomos_b200 import ops
+    x = torch.linspace(-88.5, 4.1, 3 * C).view(3, C).to(torch.bfloat16)
+    exact = x.double() * torch.sigmoid(x.double())
+    rows = torch.nn.functional.pad(x, (shift, 8 - shift)).cuda()[:, shift:shift + C]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    taps = torch.tensor([0.0, 0.0, 1.0]).repeat(C, 1).cuda()
+    got = ops.seq_conv(rows, taps, None, torch.zeros(2, 2, C, device="cuda"), i32([0, 3]), i32([0]), i32([1]),
+                       (i32([0]), i32([0]), i32([0]), i32([3])), torch.bfloat16, act=True).double().cpu()
+    assert ((got - exact).abs() <= 2.0 ** -8 * exact.abs()).all()
+    y = (1.0 / exact.abs()).float()                               # (up to 1e37: the products with silu are near 1)
+    want = plain.group_norm(y.double() * exact, torch.ones(C, dtype=torch.float64), 1, 1e-6)
+    got = ops.gated_group_norm(y.cuda(), rows, torch.ones(C, device="cuda"), 1e-6, 1).double().cpu()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs()).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("E, T, top, tile, width", [(1, 3, 1, 8, 64), (40, 700, 3, 8, 2048), (1030, 900, 2, 64, 1032), (33, 5, 5, 16, 30)])
 def test_rows_sorted_by_expert_and_combined(E, T, top, tile, width):
     """Every pair has a row of its own in a tile of its expert, padding and unused tiles are marked, the experts' blocks end where

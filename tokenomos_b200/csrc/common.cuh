@@ -78,16 +78,11 @@ __device__ __forceinline__ float rcp_approx(float x) {
 }
 constexpr float TK_NEG_LOG2E = -1.4426950408889634f;
 
-// silu(g) before any rounding, in a kernel whose result is stored in T
-template <typename T>
-__device__ __forceinline__ float silu_for(float g) {
-    if constexpr (sizeof(T) == 2) return __fmul_rn(g, rcp_approx(__fadd_rn(1.0f, ex2_approx(__fmul_rn(g, TK_NEG_LOG2E)))));
-    return g / (1.0f + expf(-g));
-}
-
 template <typename T>
 __device__ __forceinline__ float silu_as(float g) {
-    return sizeof(T) == 2 ? round_as<T>(silu_for<T>(g)) : silu_for<T>(g);
+    if constexpr (sizeof(T) == 2)
+        return round_as<T>(__fmul_rn(g, rcp_approx(__fadd_rn(1.0f, ex2_approx(__fmul_rn(g, TK_NEG_LOG2E))))));
+    return g / (1.0f + expf(-g));
 }
 
 // The tanh form of gelu, z / 2 (1 + tanh(y)) = z sigmoid(2 y) with y = sqrt(2 / pi) (z + 0.044715 z^3); 16-bit

@@ -15,7 +15,7 @@
 // tile's tokens with the last K - 1 inputs in registers. Only the tile at offset 0 of a portion
 // reads the state, and it alone writes it, after reading: tiles are at least K - 1 tokens long,
 // so no later tile needs the state.
-#include "packed.cuh"
+#include "common.cuh"
 
 namespace {
 enum : int { TK_K_SEQ_CONV = 8 };
@@ -106,7 +106,7 @@ seq_conv_kernel(const TI* in, int64_t in_stride, const float* __restrict__ taps,
 #pragma unroll
             for (int d = 1; d < MAX_TAPS; ++d)
                 if (d < K) acc = fmaf(w[K - 1 - d], past[d - 1], acc);
-            if (act) acc = silu_for<TO>(acc);
+            if (act) acc = acc / (1.0f + expf(-acc));
             if (paged) {
                 const int pos = pos0 + i;
                 const int page = TK_PAGE(TK_K_SEQ_CONV, dest.block_table[(size_t)s * dest.bt_stride + pos / dest.P]);
@@ -138,8 +138,7 @@ seq_conv_kernel(const TI* in, int64_t in_stride, const float* __restrict__ taps,
 
 // The same for bfloat16 rows that all go to `out`, four neighbouring channels a thread (8 bytes a load and a store, K known so
 // that the taps and the past of all four stay in registers), the same sums in the same order. The form above moves two bytes
-// a thread and load: 2,048 tokens of 3,072 channels take it 28.1 us (25 MB), this one 13.0; 3,000 of 4,096 53 and 20 (17.6 and 31 with
-// the accurate exponential and divide, scalar multiply-adds, and the next inputs asked for when the last were used up). A quarter
+// a thread and load: 2,048 tokens of 3,072 channels take it 28.1 us (25 MB), this one 17.6; 3,000 of 4,096 53 and 31. A quarter
 // of the threads walk as long a tile: the caller says where they are enough (ops.seq_conv_plan).
 template <int K>
 __global__ void __launch_bounds__(128)
@@ -181,32 +180,25 @@ seq_conv_quad_kernel(const __nv_bfloat16* in, int64_t in_stride, const float* __
     for (int d = 1; d < K; ++d)
         past[d] = pos0 - d < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : off - d >= 0 ? wide(before[d]) : old[K - 1 - d];
     for (int i0 = 0; i0 < n; i0 += AHEAD) {
-        uint2 now[AHEAD];
+        if (i0 > 0) {
 #pragma unroll
-        for (int k = 0; k < AHEAD; ++k) now[k] = ahead[k];
-        if (i0 + AHEAD < n) {                         // the next inputs are in flight while these are used
-#pragma unroll
-            for (int k = 0; k < AHEAD; ++k) ahead[k] = row(tok0 + min(i0 + AHEAD + k, n - 1));
+            for (int k = 0; k < AHEAD; ++k) ahead[k] = row(tok0 + min(i0 + k, n - 1));
         }
 #pragma unroll
         for (int k = 0; k < AHEAD; ++k) {
             if (i0 + k >= n) break;
-            const float4 cur = wide(now[k]);
-            float2 lo = make_float2(b.x, b.y), hi = make_float2(b.z, b.w);
-            if (residual) lo.x += cur.x, lo.y += cur.y, hi.x += cur.z, hi.y += cur.w;
-            lo = fma2(make_float2(w[K - 1][0], w[K - 1][1]), make_float2(cur.x, cur.y), lo);
-            hi = fma2(make_float2(w[K - 1][2], w[K - 1][3]), make_float2(cur.z, cur.w), hi);
+            const float4 cur = wide(ahead[k]);
+            float y[4];
 #pragma unroll
-            for (int d = 1; d < K; ++d) {
-                lo = fma2(make_float2(w[K - 1 - d][0], w[K - 1 - d][1]), make_float2(past[d].x, past[d].y), lo);
-                hi = fma2(make_float2(w[K - 1 - d][2], w[K - 1 - d][3]), make_float2(past[d].z, past[d].w), hi);
-            }
-            float4 y = make_float4(lo.x, lo.y, hi.x, hi.y);
-            if (act) {
+            for (int i = 0; i < 4; ++i) {
+                const float u = (&cur.x)[i];
+                float acc = (residual ? u : 0.f) + (&b.x)[i];
+                acc = fmaf(w[K - 1][i], u, acc);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) (&y.x)[i] = silu_for<__nv_bfloat16>((&y.x)[i]);
+                for (int d = 1; d < K; ++d) acc = fmaf(w[K - 1 - d][i], (&past[d].x)[i], acc);
+                y[i] = act ? acc / (1.0f + expf(-acc)) : acc;
             }
-            Quad<__nv_bfloat16>::store(out + (size_t)(tok0 + i0 + k) * out_stride + c, y);
+            Quad<__nv_bfloat16>::store(out + (size_t)(tok0 + i0 + k) * out_stride + c, make_float4(y[0], y[1], y[2], y[3]));
 #pragma unroll
             for (int d = K - 1; d >= 2; --d) past[d] = past[d - 1];
             past[1] = cur;
