@@ -142,6 +142,8 @@ attn_prefill_tc_kernel(const __nv_bfloat16* q, const __nv_bfloat16* pool, __nv_b
                        const AtOptions opt) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     pdl_launch_dependents();
+    if (threadIdx.x == 0 && p_shift >= 3)            // (the map is the launch's own: fetched while the kernel before ends)
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&kv_map)) : "memory");
     pdl_wait();
     // (no static shared memory: the dynamic part begins on 1,024 bytes, as the swizzled tiles must)
     const uint32_t base = smem_u32(smem_raw);
@@ -398,8 +400,8 @@ attn_prefill_tc_kernel(const __nv_bfloat16* q, const __nv_bfloat16* pool, __nv_b
             tmem_ld32(s_addr + 32u, s_hi);
             // a tile every row of the CTA sees whole needs no comparisons
             const bool kept = X && split + j * nsplit < n_keep;
-            const bool masked = j0 + AT_KEYS - 1 > pos_first || j0 < lo_last ||
-                                rows < AT_ROWS || kept;
+            // (a row past the tile's rows is a query of zeros whose sums nobody reads)
+            const bool masked = j0 + AT_KEYS - 1 > pos_first || j0 < lo_last || kept;
             // what this row sees of the tile: [see_lo, see_hi], and below keep_first whatever the window
             const int see_hi = X ? min(pos_r, tile_hi(j)) : pos_r;
             const int see_lo = X ? tile_lo(j) : 0;
