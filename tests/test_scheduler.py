@@ -330,21 +330,25 @@ def test_one_kernel_decode_attention_split_rule():
 
 
 def test_prefill_attention_split_rule():
-    """How many CTAs may share one tile's keys in the tcgen05 prefill kernel: as many as fill the
-    GPU once, within the scratch memory's budget, 16 at most, one when the step has many tiles."""
+    """How many CTAs may share one tile's keys in the tcgen05 prefill kernel: powers of two to eight, eight key tiles a CTA, two CTAs an
+    SM at most, the second one only for long walks, one CTA when the step has many tiles or nothing behind it."""
     from tokenomos_b200.parts.attention import Attention
     from tokenomos_b200.parts.registry import Tuning
     f = Attention.prefill_splits
-    assert f(2048, 64, 32, 8) == 1 and f(8192, 256, 32, 8) == 1          # a step that fills the GPU by itself
-    assert f(512, 16, 32, 8) == 2 and f(128, 4, 32, 8) == 9 and f(32, 1, 32, 8) == 16
-    assert f(128, 69, 32, 8) == 3                                          # a captured step's long list: the memory budget
-    assert f(128, 4, 32, 8, Tuning(prefill_split_ctas_per_sm=0)) == 1      # switched off
+    assert f(2048, 64, 32, 8, 32000) == 1 and f(8192, 256, 32, 8, 32000) == 1      # a step that fills the GPU by itself
+    assert f(512, 16, 32, 8, 32000) == 2 and f(128, 4, 32, 8, 32000) == 8 and f(32, 1, 32, 8, 32000) == 8
+    assert f(128, 4, 32, 8, 4128) == 4 and f(256, 8, 32, 8, 2304) == 2 and f(512, 8, 64, 8, 8704) == 4
+    assert f(128, 4, 32, 8, 128) == 1 and f(128, 4, 32, 8, 959) == 1 and f(128, 4, 32, 8, 960) == 2
+    assert f(128, 69, 32, 8, 32000) == 2                                           # a captured step's long list
+    assert f(128, 4, 32, 8, 32000, Tuning(prefill_split_ctas_per_sm=0)) == 1       # switched off
+    assert f(64, 2, 32, 8, 32000, Tuning(sm_count=32)) == 4
     for tokens in (1, 2, 31, 32, 33, 500, 5000):
         for entries in (1, 5, 70, 300):
             for kv in (1, 2, 8):
-                n = f(tokens, entries, 32, kv)
-                assert 1 <= n <= 16
-                assert n == 1 or entries * kv * n * 128 * 66 * 4 <= 64 << 20
+                for longest in (1, 500, 2000, 5000, 100000):
+                    n, tiles = f(tokens, entries, 32, kv, longest), -(-tokens // 32)
+                    assert n in (1, 2, 4, 8)
+                    assert n == 1 or (entries * kv * n <= 2048 and tiles * kv * n <= 296 and longest >= 480 * n)
 
 
 @pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 200])

@@ -519,20 +519,25 @@ class Attention:
         return split
 
     @staticmethod
-    def prefill_splits(tokens: int, entries: int, per_tile: int, kv_heads: int,
+    def prefill_splits(tokens: int, entries: int, per_tile: int, kv_heads: int, longest: int,
                        tuning: Tuning = DEFAULT_TUNING) -> int:
-        """The most CTAs that may share one tile's keys in the tcgen05 prefill kernel, for a step
-        of ``tokens`` tokens whose tile list has ``entries`` entries (a captured step's list is
-        longer than what it uses). A tile is walked by one CTA, key tile after key tile; a step
-        with few tiles behind a long context would leave the GPU idle for hundreds of
-        microseconds (128 tokens behind 32,000 positions: 474 us a layer, 98 us shared 8 ways).
-        So: as many as fill the GPU once (``prefill_split_ctas_per_sm`` CTAs an SM), fewer where a long list of tiles leaves
-        most of a launch without work (``prefill_split_scratch_mb``, once the shares' memory); the kernel takes the next
-        power of two below, at most 8, and gives each tile as many of them as leave a CTA 8 key tiles."""
-        tiles = max(1, -(-tokens // per_tile))
-        by_ctas = tuning.prefill_split_ctas_per_sm * tuning.sm_count // (tiles * max(1, kv_heads))
-        by_memory = (tuning.prefill_split_scratch_mb << 20) // (max(1, entries) * max(1, kv_heads) * 128 * 66 * 4)
-        return max(1, min(16, by_ctas, by_memory))
+        """The most CTAs (1, 2, 4 or 8, a cluster) that may share one tile's keys in the tcgen05 prefill kernel, for a step
+        of ``tokens`` tokens whose tile list has ``entries`` entries (a captured step's list is longer than what it uses) and whose
+        sequences hold at most ``longest`` positions. A tile is walked by one CTA, key tile after key tile, so that a step with few tiles
+        behind a long context would leave most of the GPU idle. Doubled while a CTA keeps 8 key tiles (below that the kernel shares
+        nothing and the cluster costs 1 to 3 us), the CTAs are no more than ``prefill_split_ctas_per_sm`` an SM and, unused entries
+        included, than ``prefill_split_launch``; from two on, beyond one CTA an SM only where each keeps 32 key tiles: two CTAs
+        of an SM walk at 0.7 of one's pace, and of clusters of eight 15 find room at a time (us by 1, 2, 4 and 8; 32 heads over 8:
+        128 tokens behind 4,000 45.0, 30.3, 20.7, 26.9, behind 32,000 315, 180, 102, 73; 256 behind 2,048 27.4, 20.6, 22.2, 34.0; 512 behind
+        8,192 88, 70, 83, 118; 16 heads: 128 behind 32,000 312, 176, 96, 68; 512 behind 8,192 88, 53, 43, 62)."""
+        ctas = max(1, -(-tokens // per_tile)) * max(1, kv_heads)
+        launched = max(1, entries) * max(1, kv_heads)
+        split = 1
+        while (split < 8 and 2 * split * ctas <= tuning.prefill_split_ctas_per_sm * tuning.sm_count
+               and 2 * split * launched <= tuning.prefill_split_launch and longest >= 2 * split * 480
+               and (split == 1 or 2 * split * ctas <= tuning.sm_count or longest >= split * 2048)):
+            split *= 2
+        return split
 
     def _attend_mma(self, q, pool, table, ctx: StepContext, gate=None) -> torch.Tensor:
         """The tensor-core kernels: prompt portions in tiles of 64 rows, decoded tokens split
@@ -549,9 +554,8 @@ class Attention:
             self.heads, self.kv_heads)
         _, tok0, _, ntok = ctx.tiles(per_tile, "multi")
         if tok0.numel() and tc:
-            # (a cluster that no tile is long enough for costs 1 to 3 us)
             longest = min(ctx.host.longest, self.span) if self.span is not None else ctx.host.longest
-            nsplit = min(self.prefill_splits(ctx.n_tokens, tok0.numel(), per_tile, self.kv_heads, self.tuning), max(1, longest // 480))
+            nsplit = self.prefill_splits(ctx.n_tokens, tok0.numel(), per_tile, self.kv_heads, longest, self.tuning)
             ops.attention_prefill_tc(q, pool, out, ctx.positions, ctx.tok_seq, table, tok0, ntok, self.reach,
                                      self.scale, gate, nsplit, self.keep_first, self.sink, by_element)
         elif tok0.numel():

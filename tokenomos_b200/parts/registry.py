@@ -49,8 +49,9 @@ class Tuning:
     so a kernel that asks for another split than its neighbours cannot start under them, and the
     L1 it leaves is what their activation loads find; -1 leaves the choice to the driver, which
     it always is above ``skinny_rows`` rows.
-    ``prefill_split_ctas_per_sm`` / ``prefill_split_scratch_mb``: how far a prompt portion's
-    tiles may share their keys out over CTAs (``Attention.prefill_splits``).
+    ``prefill_split_ctas_per_sm`` / ``prefill_split_launch``: how far a prompt portion's
+    tiles may share their keys out over CTAs (``Attention.prefill_splits``): CTAs an SM, and CTAs a launch with those of a captured
+    step's unused tiles.
     ``grouped_library_rows``: from that many (token, expert) rows on, a mixture of experts' two
     grouped products are the library's (``torch._grouped_mm`` over the sorted layout, 149 us against
     435 us for the ``mma.sync`` kernel at 8,192 rows of 2,048 x 1,536); below, the framework's own
@@ -82,7 +83,7 @@ class Tuning:
     decode_fused_general_head: int = 64
     decode_fused_carveout: int = 62
     prefill_split_ctas_per_sm: int = 2
-    prefill_split_scratch_mb: int = 64
+    prefill_split_launch: int = 2048
     grouped_library_rows: int = 1024
     conv_tile: int = 16
     fuse_norms: bool = True
