@@ -1039,18 +1039,21 @@ def test_attention_tc_prefill(H, Hkv, P):
 @pytest.mark.parametrize("split, window", [(2, None), (3, None), (8, None), (4, 70), (5, 1)])
 def test_attention_tc_prefill_with_a_tiles_keys_shared_by_several_ctas(H, Hkv, P, split, window):
     """Portions behind long and short contexts with each tile's keys split over CTAs: sequences with
-    fewer key tiles than splits (some CTAs have nothing), a window, a gate; twice in a row (the
-    tickets of the first launch leave the second alone)."""
+    fewer key tiles than splits (some CTAs have nothing), a window, a gate; twice in a row with the same inputs: the same
+    bits, and no wait given up."""
     from tokenomos_b200 import ops
     seqs = [(0, 40), (1900, 130), (17, 3), (333, 64), (0, 2), (700, 33), (64, 64), (5000, 70), (2600, 40)]
     T = sum(n for _, n in seqs)
     gate = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    state, first = torch.random.get_rng_state(), None
     for _ in range(2):
+        torch.random.set_rng_state(state)
         got, want = attention_mma_case(H, Hkv, 64, P, seqs, window=window, tc=True, gate=gate, tc_split=split)
         close(got, want * torch.sigmoid(gate.double().cpu())[:, :, None], torch.bfloat16,
               f"tcgen05 prefill H{H} Hkv{Hkv} P{P} split {split} window {window}")
         assert ops.attention_prefill_tc_status() == 0
-        assert int(ops._tickets[got.device].abs().sum()) == 0
+        first = got if first is None else first
+        assert torch.equal(got.view(torch.int16), first.view(torch.int16))
 
 
 @pytest.mark.parametrize("P", [4, 8, 128])

@@ -33,7 +33,8 @@
 //
 // Masking, scale, rounding of P to bfloat16 and the unrounded row sum are those of the other
 // attention kernels (Tokenomos kernels/attention/paged.py:67-76,150,267;
-// models/blocks/attention.py:31-40,173). Keys past the tile's last position are never read.
+// models/blocks/attention.py:31-40,173). Rows of a page beside the positions a tile sees come with it and are
+// zeroed before a product reads them.
 //
 // Every mbarrier wait is bounded (about a second, or until another thread has recorded an
 // error); the kernel then leaves its loops, frees its tensor memory and returns, and
@@ -742,13 +743,4 @@ TK_API int tk_attn_prefill_tc_opt(const void* q, const void* kv_pool, void* out,
         return -2;
     }
     return 0;
-}
-
-TK_API int tk_attn_prefill_tc(const void* q, const void* kv_pool, void* out, const int* positions,
-                              const int* tok_seq, const int* block_table, int bt_stride,
-                              const int* tile_tok0, const int* tile_ntok, int n_tiles, int H, int Hkv, int D,
-                              int P, int window, float scale, const void* gate, int64_t ldg, int nsplit, cudaStream_t stream) {
-    return tk_attn_prefill_tc_opt(q, kv_pool, out, positions, tok_seq, block_table, bt_stride, tile_tok0, tile_ntok,
-                                  n_tiles, H, Hkv, D, P, window, scale, gate, ldg, nsplit, 0, 0,
-                                  gate != nullptr ? 1 : 0, stream);
 }

@@ -618,21 +618,16 @@ def attention_decode_fused_supported(heads: int, kv_heads: int, head_dim: int, r
 
 # per device: [n * kv_heads] zeros the fused decode kernel counts finished splits in and zeroes
 # again; a buffer that a captured step may point at is never freed, only outgrown
-class _Tickets(dict):
-    def __missing__(self, device: torch.device) -> torch.Tensor:
-        self[device] = made = torch.zeros(4096, dtype=torch.int32, device=device)
-        return made
-
-
-_tickets = _Tickets()
+_tickets: dict = {}
 _tickets_outgrown: list = []
 
 
 def _decode_tickets(n: int, device: torch.device) -> torch.Tensor:
-    have = _tickets[device]
-    if have.numel() < n:
-        _tickets_outgrown.append(have)
-        have = _tickets[device] = torch.zeros(n, dtype=torch.int32, device=device)
+    have = _tickets.get(device)
+    if have is None or have.numel() < n:
+        if have is not None:
+            _tickets_outgrown.append(have)
+        have = _tickets[device] = torch.zeros(max(n, 4096), dtype=torch.int32, device=device)
     return have
 
 

@@ -53,7 +53,6 @@ _SIGNATURES = {
     "tk_attn_prefill_tc_supported": [I, I, I],
     "tk_attn_prefill_tc_tokens": [I, I],
     "tk_attn_prefill_tc_status": [],
-    "tk_attn_prefill_tc": [P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, F, P, L, I, P],
     "tk_attn_prefill_tc_opt": [P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, F, P, L, I, I, I, I, P],
     "tk_attn_decode_mma": [P, P, P, P, P, P, I, P, I, I, I, I, I, I, F, I, P, P, L, P],
     "tk_attn_decode_fused_supported": [I, I, I, I],
