@@ -1006,8 +1006,9 @@ def test_scan_by_chunks(H, V, N, G, lens, ctx, dtype):
     (40, 64, 64, 8, (48, 50), (2, 0), 0), (32, 128, 128, 4, (150, 90), (0, 6), 0), (4, 64, 128, 2, (700,), (1,), 4)])
 def test_scan_by_chunks_of_16_bit_rows(H, V, N, G, lens, ctx, shift):
     """Chunks of 64 tokens on the tensor cores at the edges of a chunk, of 16 tokens within it and of the blocks' rows, one to eight
-    heads a group (rows that begin on 8 bytes instead of 16: by multiply-adds): against the recurrence in 64-bit, sums of up to 128 products in
-    32-bit; decays from 1 to 0. Numbers that are not finite reach their own row of x from their token on, b all rows, c its own output."""
+    heads a group (rows that begin on 8 bytes instead of 16: by multiply-adds): each head against the recurrence in 64-bit, sums of up to 128
+    products in 32-bit; decays from 1 to 0. Numbers that are not finite reach their own row of x and of the state from their token on, b all
+    rows, c its own output."""
     from tokenomos_b200 import ops
     g = torch.Generator().manual_seed(13)
     T, S = sum(lens), len(lens)
@@ -1015,9 +1016,9 @@ def test_scan_by_chunks_of_16_bit_rows(H, V, N, G, lens, ctx, shift):
     xbc = torch.randn(T, H * V + 2 * G * N, generator=g).to(torch.bfloat16)
     raw = torch.randn(T, H + 4, generator=g)
     raw[::17] += 8.0
-    raw[::47, 0] = 1e4                                            # a decay of 0
     raw[3::29] = -120.0                                           # dt of 0
     bias, a_log, skip = (torch.randn(H, generator=g) for _ in range(3))
+    a_log[0] = 6.0                                                # (a rate of 400: decays of 0 beside those of 1)
     state = torch.randn(S + 1, H, N, V, generator=g)
     cu = [0]
     for n in lens:
@@ -1045,26 +1046,32 @@ def test_scan_by_chunks_of_16_bit_rows(H, V, N, G, lens, ctx, shift):
             want[t] = torch.einsum("hn,hnv->hv", C[t], M) + skip.double()[:, None] * x[t]
         if lens[s]:
             after[slots[s]] = M
-    assert (got[0].double().cpu().view(T, H, V) - want).norm() <= 1e-6 * want.norm()
-    assert (st.double().cpu() - after).norm() <= 1e-6 * after.norm()
+    off = got[0].double().cpu().view(T, H, V) - want
+    assert (off.norm(dim=(0, 2)) <= 1e-6 * want.norm(dim=(0, 2))).all()
+    assert ((st.double().cpu() - after).norm(dim=(2, 3)) <= 1e-6 * after.norm(dim=(2, 3))).all()
 
     last = max(range(S), key=lambda s: lens[s])
     t = cu[last] + lens[last] // 2
     raw[t] = 0.0                                                  # (with a dt of 0 the walk keeps what is not finite too, as NaN)
-    got = run(xbc, state.cuda())
+    st = state.cuda()
+    got, kept = run(xbc, st), st.cpu()
     for value, column in ((float("nan"), V - 1), (float("inf"), 0), (float("nan"), H * V), (float("nan"), H * V + G * N)):
         rows = xbc.clone()
         rows[t, column] = value
-        again = run(rows, state.cuda())[0].view(T, H, V).cpu()
-        clean = torch.ones(T, H, V, dtype=torch.bool)
+        st = state.cuda()
+        again = run(rows, st)[0].view(T, H, V).cpu()
+        clean, untouched = torch.ones(T, H, V, dtype=torch.bool), torch.ones(S + 1, H, N, V, dtype=torch.bool)
         if column < H * V:                                        # x: its row of the state, from its token on
             clean[t:cu[last + 1], 0, column] = False
+            untouched[slots[last], 0, :, column] = False
         elif column < H * V + G * N:                              # b: the heads that read it, from its token on
             clean[t:cu[last + 1], :H // G] = False
+            untouched[slots[last], :H // G, 0] = False            # (its own column, every row of x)
         else:                                                     # c: its own output
             clean[t, :H // G] = False
         assert torch.equal(again[clean], got[0].view(T, H, V).cpu()[clean])
-        assert not torch.isfinite(again[t][~clean[t]]).any()
+        assert not torch.isfinite(again[~clean]).any()
+        assert torch.equal(st.cpu()[untouched], kept[untouched]) and not torch.isfinite(st.cpu()[~untouched]).any()
 
 
 @pytest.mark.gpu
