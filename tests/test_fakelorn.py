@@ -1003,10 +1003,11 @@ def test_scan_by_chunks(H, V, N, G, lens, ctx, dtype):
 @pytest.mark.gpu
 @pytest.mark.parametrize("H, V, N, G, lens, ctx, shift", [
     (1, 32, 64, 1, (64,), (0,), 0), (5, 32, 128, 1, (65, 127, 1), (4, 0, 7), 0), (6, 96, 128, 2, (63, 0, 129, 192), (0, 0, 9, 1), 0),
-    (40, 64, 64, 8, (48, 50), (2, 0), 0), (32, 128, 128, 4, (150, 90), (0, 6), 0), (4, 64, 128, 2, (700,), (1,), 4)])
+    (40, 64, 64, 8, (48, 50), (2, 0), 0), (32, 128, 128, 4, (150, 90), (0, 6), 0), (4, 64, 128, 2, (700,), (1,), 4),
+    (2, 64, 128, 1, (1500,), (1,), 0)])
 def test_scan_by_chunks_of_16_bit_rows(H, V, N, G, lens, ctx, shift):
     """Chunks of 64 tokens on the tensor cores at the edges of a chunk, of 16 tokens within it and of the blocks' rows, one to eight
-    heads a group (rows that begin on 8 bytes instead of 16: by multiply-adds): each head against the recurrence in 64-bit, sums of up to 128
+    heads a group (rows that begin on 8 bytes instead of 16, and a long sequence of few heads: by multiply-adds): each head against the recurrence in 64-bit, sums of up to 128
     products in 32-bit; decays from 1 to 0. Numbers that are not finite reach their own row of x and of the state from their token on, b all
     rows, c its own output."""
     from tokenomos_b200 import ops

@@ -444,3 +444,14 @@ def test_sequence_convolution_takes_four_channels_a_thread_where_they_fill_the_g
     assert f(1, 64, 4, single=True) == (16, True) and f(64, 4096, 4, single=True) == (16, True)
     assert f(2048, 6144, 5) == (32, False) and f(2048, 6144, 1) == (32, False)
     assert f(2048, 6144, 4, torch.float32) == (ops.seq_conv_tile(16, 2048, 6144), False)
+
+
+def test_side_by_side_rule_of_the_state_space_chunks():
+    """Chunks side by side instead of one after the other: long sequences of few heads, more so where short ones take their blocks' places;
+    recorded steps count as one portion."""
+    from tokenomos_b200 import ops
+    f = ops.ssd_chunks_side_by_side
+    assert not f(1000, 1, 64, 1, [1000]) and f(2048, 1, 64, 1, [2048]) and f(2048, 8, 64, 1, [2048]) and f(2048, 4, 128, 1)
+    assert not any(f(n, 16, 64, 1, [n]) for n in (64, 1000, 2048, 8192, 16000))
+    assert f(4096, 4, 64, 2, [2048, 2048]) and not f(4096, 8, 64, 2, [2048, 2048]) and f(4096, 8, 64, 4)
+    assert f(3200, 16, 64, 3, [3000, 100, 100]) and not f(3200, 24, 64, 3, [3000, 100, 100]) and not f(0, 8, 64, 1, [])

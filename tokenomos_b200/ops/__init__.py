@@ -1608,6 +1608,19 @@ def ssd_by_chunks(tokens: int, heads: int, v_dim: int, seq_lens: list[int] | Non
     return blocks * int(tokens) <= 240 * walk
 
 
+def ssd_chunks_side_by_side(tokens: int, heads: int, v_dim: int, n_seqs: int, seq_lens: list[int] | None = None, sm_count: int = 148) -> bool:
+    """Whether chunks in multiply-adds, all side by side, are the better way than chunks on the tensor cores, which a head walks one
+    after the other: long sequences of few heads. The walk's time is that of its longest sequence (1.6 times as much a token where blocks
+    of 16 columns outnumber the SMs and those of 32 are taken), the other's 1,000 of its tokens and a 32nd for every token and 32 columns
+    of the heads, whatever the state (us, tensor cores and side by side, 64 x 128: 1 head 1,000 tokens 33 and 35, 2,048 59 and 37, 16,000
+    415 and 68; 8 heads 1,000 34 and 48, 2,048 61 and 56, 8,192 223 and 143; 16 heads 2,048 62 and 81, 16,000 445 and 586, portions of 3,000,
+    100 and 100 122 and 115). ``seq_lens`` None: as if one portion had all tokens."""
+    longest = int(tokens) if seq_lens is None else max(seq_lens, default=0)
+    if -(-int(v_dim) // 16) * int(heads) * int(n_seqs) > int(sm_count):
+        longest = 8 * longest // 5
+    return longest > 1000 + int(tokens) * -(-int(v_dim) // 32) * int(heads) // 32
+
+
 def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, cu_seqlens: torch.Tensor, seq_ctx: torch.Tensor, seq_slot: torch.Tensor, n_seqs: int,
              heads: int, v_dim: int, n_state: int, groups: int, sm_count: int = 148,
@@ -1617,8 +1630,9 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
     n_state] (rows may be strided): x, then B, then C; ``dt_raw`` float32 [T, >= heads]; ``state`` float32 [slots,
     heads, n_state, v_dim]. Returns ``y`` float32 [parts, T, heads v_dim]: a step of few, long portions is walked
     by several blocks a head, each over a part of the state's rows, and their sums are still to be added
-    (``gated_group_norm`` does; ``y.sum(0)`` is the result). Portions of 48 tokens and more in 16-bit rows of whole 16-byte pieces, and few, long ones of any (``ssd_by_chunks``),
-    whose states the chunked kernels take are formed chunk by chunk instead (one part). ``seq_lens``: the portions' lengths, where the host knows them."""
+    (``gated_group_norm`` does; ``y.sum(0)`` is the result). Portions whose states the chunked kernels take are formed chunk by chunk instead
+    (one part): of 48 tokens and more in 16-bit rows of whole 16-byte pieces on the tensor cores, unless few heads make it the better
+    way, and few, long ones of any rows always (``ssd_by_chunks``), all chunks side by side (``ssd_chunks_side_by_side``). ``seq_lens``: the portions' lengths, where the host knows them."""
     _cuda(xbc, dt_raw, dt_bias, a_log, d_skip, state)
     T = xbc.shape[0]
     if xbc.stride(1) != 1 or xbc.shape[1] < heads * v_dim + 2 * groups * n_state:
@@ -1627,7 +1641,9 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
         raise KernelError(f"ssd_scan: dt is float32 [{T}, >= {heads}]")
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (heads, n_state, v_dim) or not state.is_contiguous():
         raise KernelError(f"ssd_scan: the state is float32 [slots, {heads}, {n_state}, {v_dim}]")
-    if xbc.dtype == torch.bfloat16 and xbc.stride(0) % 8 == 0 and xbc.data_ptr() % 16 == 0:
+    by_chunks = _lib.call("tk_ssd_chunked_scratch", T, int(n_seqs), heads, v_dim, n_state, groups)
+    if (xbc.dtype == torch.bfloat16 and xbc.stride(0) % 8 == 0 and xbc.data_ptr() % 16 == 0
+            and not (by_chunks and ssd_chunks_side_by_side(T, heads, v_dim, n_seqs, seq_lens, sm_count))):
         words = _lib.call("tk_ssd_tc_scratch", T, int(n_seqs), heads, v_dim, n_state, groups)
         if words:
             # portions of some length: chunk by chunk on the tensor cores
@@ -1638,11 +1654,10 @@ def ssd_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_l
                       _ptr(_i32(cu_seqlens, "cu_seqlens")), _ptr(_i32(seq_ctx, "seq_ctx")), _ptr(_i32(seq_slot, "seq_slot")),
                       int(n_seqs), T, _ptr(y), heads, v_dim, n_state, groups, _ptr(scratch), int(sm_count), _stream())
             return y
-    words = _lib.call("tk_ssd_chunked_scratch", T, int(n_seqs), heads, v_dim, n_state, groups)
-    if (words and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0
+    if (by_chunks and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0
             and ssd_by_chunks(T, heads, v_dim, seq_lens, sm_count)):
         # portions of some length: chunk by chunk, all side by side
-        scratch = torch.empty(words, dtype=torch.float32, device=xbc.device)
+        scratch = torch.empty(by_chunks, dtype=torch.float32, device=xbc.device)
         y = torch.empty(1, T, heads * v_dim, dtype=torch.float32, device=xbc.device)
         _lib.call("tk_ssd_chunked", _ptr(xbc), xbc.stride(0), _ptr(dt_raw), dt_raw.stride(0),
                   _ptr(_f32vec(dt_bias, "dt_bias", heads)), _ptr(_f32vec(a_log, "A_log", heads)),
