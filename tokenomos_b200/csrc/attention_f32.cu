@@ -213,6 +213,7 @@ attn32_prefill_kernel(const float* q, const float* kv_pool, float* out, const in
                     const int64_t at = rows_at[n * 8 + tok + (e & 1)];
                     float sum = 0.f;
                     if (at >= 0)
+#pragma unroll 1
                         for (int d = 0; d < F_D; ++d) sum = fmaf(q_row[e >> 1][d], kv_pool[at + d], sum);
                     s[n][e] = sum;
                 }
@@ -283,6 +284,7 @@ attn32_prefill_kernel(const float* q, const float* kv_pool, float* out, const in
             for (int e = 0; e < 4; ++e) o[n][e] *= alpha[e >> 1];
 #pragma unroll
         for (int n = 0; n < 8; ++n)
+#pragma unroll 1
             for (int k = 0; k < 8; ++k) {
                 const int from = (lane & ~3) | (k >> 1), key = j0 + n * 8 + k;
                 const float p0 = __shfl_sync(0xffffffffu, k & 1 ? s[n][1] : s[n][0], from);
