@@ -397,10 +397,10 @@ def kernel_case(name: str) -> None:
     ``conv_tile``: the tiled gated short conv over a 2,048-token portion of 2,048 channels (width 3,
     tiles of 16 tokens), 20 launches in a CUDA graph that is replayed five times;
     ``ssd_scan``: the state-space scan over a 2,048-token portion of one sequence, 4 launches;
-    ``linmem_scan``: the delta rule (a decay per head) over such a portion, 4 launches of its two kernels;
+    ``linmem_scan``: the delta rule (a decay per head) over such a portion, 4 launches of its two kernels (chunk by chunk, as the scan's);
     ``retention_scan``: the same for retention (16 heads, q and k rotated);
     ``attn_portions`` (a measurement, not a profiler case): the tcgen05 prefill attention on
-    portions behind cached contexts, with a tile's keys shared by 1 to 16 CTAs."""
+    portions behind cached contexts, with a tile's keys shared by 1 to 8 CTAs."""
     import torch
 
     from tokenomos_b200 import ops
@@ -410,10 +410,15 @@ def kernel_case(name: str) -> None:
     if name == "attn_portions":
         # the tcgen05 prefill attention on a portion of T tokens behind C cached positions (32
         # heads of 64 over 8 KV heads, one sequence), with up to `split` CTAs sharing a tile's
-        # keys: CUDA events around 10 launches, after 3
+        # keys: every form warmed up, then CUDA events around 10 launches of each, five times in
+        # another order each, the median; an asterisk marks the rule's choice
+        import random
+
+        from tokenomos_b200.parts.attention import Attention
         H, Hkv, D, P = 32, 8, 64, 16
         per = ops.attention_prefill_tc_tokens(H, Hkv)
-        for T, C in ((512, 0), (512, 3584), (512, 32256), (128, 4096), (128, 32640), (32, 32640), (2048, 0), (2048, 30720)):
+        order = random.Random(0)
+        for T, C in ((512, 0), (512, 3584), (512, 32256), (256, 2048), (128, 4096), (128, 32640), (32, 32640), (2048, 0), (2048, 30720)):
             q = torch.randn(T, H, D, device=dev, dtype=bf16)
             pages = (C + T) // P + 2
             pool = torch.randn(pages, 2, Hkv, P, D, device=dev, dtype=bf16)
@@ -425,20 +430,29 @@ def kernel_case(name: str) -> None:
             nt = torch.full((t0.numel(),), per, dtype=torch.int32, device=dev)
             flops = 4.0 * H * D * sum(C + i + 1 for i in range(T))
             line = f"portion {T:5d} behind {C:6d} ({t0.numel() * Hkv:4d} CTAs unsplit):"
-            for split in (1, 2, 4, 8, 16):
-                if split > 1 and t0.numel() * Hkv * split > 4 * 296:
-                    continue
-                for _ in range(3):
+            splits = [n for n in (1, 2, 4, 8) if n == 1 or t0.numel() * Hkv * n <= 4 * 296]
+            taken = {n: [] for n in splits}
+
+            def launches(n, split):
+                for _ in range(n):
                     ops.attention_prefill_tc(q, pool, out, pos, seq, table, t0, nt, None, D ** -0.5, None, split)
-                torch.cuda.synchronize()
-                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                a.record()
-                for _ in range(10):
-                    ops.attention_prefill_tc(q, pool, out, pos, seq, table, t0, nt, None, D ** -0.5, None, split)
-                b.record()
-                torch.cuda.synchronize()
-                us = a.elapsed_time(b) / 10 * 1e3
-                line += f"  x{split}: {us:7.1f} us ({flops / us / 1e6:5.0f} TFLOP/s)"
+
+            for split in splits:
+                launches(10, split)
+            for _ in range(5):
+                for split in order.sample(splits, len(splits)):
+                    launches(2, split)
+                    torch.cuda.synchronize()
+                    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                    a.record()
+                    launches(10, split)
+                    b.record()
+                    torch.cuda.synchronize()
+                    taken[split].append(a.elapsed_time(b) / 10 * 1e3)
+            rule = Attention.prefill_splits(T, t0.numel(), per, Hkv, C + T)
+            for split in splits:
+                us = sorted(taken[split])[2]
+                line += f"  x{split}{'*' if split == rule else ''}: {us:7.1f} us ({flops / us / 1e6:5.0f} TFLOP/s)"
             print(line, flush=True)
         if ops.attention_prefill_tc_status():
             raise RuntimeError("the tcgen05 attention reported an error")
