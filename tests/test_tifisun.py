@@ -1078,3 +1078,61 @@ def test_delta_rule_by_chunks_of_keys_that_share_a_direction(H, K, D, V, lens, s
         after[s + 1] = M
     assert ((got.double().cpu().view(T, H, V) - want).norm(dim=(0, 2)) <= 2e-6 * want.norm(dim=(0, 2))).all()
     assert ((st.double().cpu() - after).norm(dim=(2, 3)) <= 2e-6 * after.norm(dim=(2, 3)))[1:].all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", ["delta rule", "state space"])
+def test_recorded_step_of_chunks_replayed_for_other_lengths(which):
+    """A step recorded for four sequences (one portion, the rest empty) and replayed with a portion beside single tokens and an unused
+    sequence, then with none but short ones: the chunks' kernels take both, each sequence gives what it gives alone, rows past the last
+    token and states of unused sequences are left alone."""
+    from tokenomos_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(23)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    T, S = 512, 4
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    cu, ctx, slot = i32([0, T, T, T, T]), i32([0] * S), i32([1, 2, 3, 4])
+    if which == "delta rule":
+        H, K, D, V = 4, 2, 128, 64
+        u, zb, za = r(T, 2 * K * D + H * V).bfloat16(), r(T, H), r(T, H) - 2.0
+        A, bias, state0 = torch.rand(H, generator=g, device="cuda") * 3, r(H), r(S + 1, H, V, D) * 0.3
+        assert ops._lib.call("tk_delta_chunks_scratch", T, S, H, K, D, V) > 0
+
+        def run(rows, cu, ctx, slot, n, st):
+            return ops.linmem_scan(u[rows], (0, K * D, 2 * K * D), "delta", "head", A, st, cu, ctx, slot, n, H, K, D, V, D ** -0.5, unit=True,
+                                   beta=zb[rows], gates=za[rows], bias=bias)
+    else:
+        H, V, N, G = 32, 64, 128, 4
+        x, dt, (b, a, d), state0 = r(T, H * V + 2 * G * N).bfloat16(), r(T, H), r(3, H), r(S + 1, H, N, V)
+        assert ops._lib.call("tk_ssd_tc_scratch", T, S, H, V, N, G) > 0
+
+        def run(rows, cu, ctx, slot, n, st):
+            return ops.ssd_scan(x[rows], dt[rows], b, a, d, st, cu, ctx, slot, n, H, V, N, G).sum(0)
+    st = state0.clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        run(slice(0, T), cu, ctx, slot, S, st)
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = run(slice(0, T), cu, ctx, slot, S, st)
+    for lens, cached in (((400, 1, 1, 0), (0, 9, 3, 0)), ((3, 70, 65, 2), (5, 0, 1, 0))):
+        st.copy_(state0)
+        ends = [0]
+        for n in lens:
+            ends.append(ends[-1] + n)
+        cu.copy_(i32(ends))
+        ctx.copy_(i32(list(cached)))
+        y.fill_(7.0)
+        graph.replay()
+        assert which != "delta rule" or (y[ends[-1]:] == 7.0).all()
+        for s, n in enumerate(lens):
+            alone = state0.clone()
+            if n:
+                want = run(slice(ends[s], ends[s + 1]), i32([0, n]), i32([cached[s]]), i32([s + 1]), 1, alone)
+                got = y[ends[s]:ends[s + 1]]
+                assert (got - want).norm() <= 2e-6 * want.norm()
+            assert (st[s + 1] - alone[s + 1]).norm() <= 2e-6 * alone[s + 1].norm()
+        assert torch.equal(st[0], state0[0])

@@ -14,8 +14,8 @@
 // flight with their values, for all heads of the group; the keys of a token are shared out over `nsplit` blocks and their
 // eight half-warps, each with a softmax of its own, merged in a fixed order in the block, then by a second kernel.
 //
-// The prompt kernel (us; by multiply-adds, 4 x 4 of them a thread, in brackets): 16 heads over 8 on 1,000 tokens 74 (146), on 300 28 (34),
-// 33 behind 2,500 positions 37 (226), 3 x 700 behind 2,500 586 (890); against 64 bits 1e-7 to 2.5e-7 off (2e-7 to 8e-7).
+// The prompt kernel (us; by multiply-adds, 4 x 4 of them a thread, in brackets): 16 heads over 8 on 1,000 tokens 74 (153), on 300 29 (40), on
+// 64 8.3 (9.7), 33 behind 2,500 positions 37 (226), 3 x 700 behind 2,500 586 (890); against 64 bits 1e-7 to 2.5e-7 off (2e-7 to 8e-7).
 #include <cooperative_groups.h>
 #include <math.h>
 

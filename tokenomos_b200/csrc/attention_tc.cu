@@ -27,9 +27,9 @@
 // Bound by each group's chain: 2,500 cycles a tile alone on an SM (scores there 100, maximum 330, exponentials 850, the
 // products' issue and the barriers around them 1,200), 3,000 beside a second CTA, where four chains keep the special-function
 // unit (512 cycles a tile) at two thirds. One group of 128 threads a CTA, with V turned by ldmatrix and stmatrix, took
-// 2,700 a tile and CTA: 512 tokens of 32 heads over 8 behind 8,192 positions 87 us, now 71; a prompt of 2,048 48.7 and 39.9, of 77
-// 8.2 and 7.1; 3 x 700 behind 2,500 134 and 107; 128 tokens of 16 heads behind 32,000, whose keys 16 CTAs shared and now 8, 60
-// and 70.
+// 2,700 a tile and CTA: 512 tokens of 32 heads over 8 behind 8,192 positions 89 us, now 70; a prompt of 2,048 48.3 and 39.8; 3 x 700
+// behind 2,500 (the layer) 190 and 141; 128 tokens of 16 heads behind 32,000, whose keys 16 CTAs shared and now 8, 60
+// and 68. At 80 registers a thread the compiler spills 140 bytes of a thread (3 % of the instructions it runs).
 //
 // Masking, scale, rounding of P to bfloat16 and the unrounded row sum are those of the other
 // attention kernels (Tokenomos kernels/attention/paged.py:67-76,150,267;

@@ -26,11 +26,15 @@
 //
 // A number that is not finite reaches its own row of V from its token on, as in the walk, and nothing before: such elements of
 // R and U are taken out of the products and every output of the row from the first one on, and the row of S, are set to NaN.
-// (Products with k come before its length is divided out: values and states beyond 2^128 / |k| overflow.)
+// (Products with k come before its length is divided out: values and states beyond 2^128 / |k| overflow, and k of 2^64 and more in two
+// tokens of a chunk.)
 //
 // Measured (both kernels, us; token by token in brackets): 16 heads of 128 x 128 over 8 on 750 and 2,250 tokens 138 (462), on 2,048
-// 112 (324); heads of 64 x 64 88 (314) and 78 (280); 16 x 16 heads of 128, sixteen sequences of 512, 251 (614). Against 64 bits y
-// is 1.7e-7 off and S 1.3e-7, the walk 2.1e-7 to 6.8e-7 and 2.1e-7 to 3.7e-7 (growing with the tokens). A chunk takes 4,800 cycles of
+// 112 (324); heads of 64 x 64 88 (314) and 78 (280); 16 x 16 heads of 128, sixteen sequences of 512, 251 (614). Against 64 bits, on
+// what projections and convolutions of random weights give (fourteen cases of 72 to 3,000 tokens), y is 1.4e-7 to 1.7e-7 off and S 1.1e-7 to
+// 1.4e-7, the walk 1.7e-7 to 9.5e-7 and 1.8e-7 to 1.2e-6 (growing with the tokens). Keys that share a direction (0.9 to all of it, or with
+// alternating signs): 1.8e-7 to 2.4e-7 where gates forget within some ten tokens (the walk 1.4e-7 to 2.9e-7), 4.0e-7 to 6.0e-7 where
+// they hardly do (3.6e-7 to 1.9e-6). A chunk takes 4,800 cycles of
 // a state warp (P 1,050, R 450, U 900, its parts 600, the update of S 1,200 with its sums), of which 2,000 are its 252 products.
 #include "chunk_tc.cuh"
 
